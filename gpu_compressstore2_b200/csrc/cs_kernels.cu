@@ -685,73 +685,140 @@ cudaError_t launch_writeout_naive(const void* in, const uint32_t* mask, void* ou
 
 // ---------------------------------------------------------------------------------
 // Pass 3, sparse units (3-pass hybrid, chunk length <= 4096). Units of the TMA kernel whose
-// selected count is at most sparse_max are compacted here instead. A warp takes groups of 4
-// blocks of 1024 elements (one mask word per lane per block), each starting on a chunk
-// boundary, derives each block's output offset from the pass-2 chunk offset plus in-warp
-// block popcounts, and lanes gather only their selected elements — DRAM traffic is the mask
-// plus the sectors holding selected elements. The work is whole 16K-element items (4
-// groups) when there are more items than resident warps, quarter items (one group) when
-// there are fewer: a column with few sparse units then gets four times the warps, each with
-// a quarter of the dependent steps (batch256 +3.5%, 2^24 u32 p = 0.01 40.0 -> 27.6 us), while
-// many items keep the cheaper whole-item work (2^28 f32 p = 0.001: 56.6 us whole, 60.9
-// quartered). A dense unit is rejected with two loads, and the whole kernel returns at once
-// when pass 1 saw no sparse block. The TMA kernel skips exactly these units (same count test).
+// selected count is at most sparse_max are compacted here instead: DRAM traffic is the mask
+// plus the sectors holding selected elements.
+// What bounds it is latency (per item a flag, then the mask, then the payload) and, at 1% and
+// above, DRAM sectors. A warp therefore loads the masks of a whole work item at once (128
+// consecutive elements per lane and 4096-element group), writes the indices of its selected
+// elements to a list in shared memory at their ranks (one packed scan per two groups), and
+// gathers from the list with SPARSE_INFLIGHT loads per lane in flight before the first store;
+// the stores of a warp are consecutive, and a load fetches 64 bytes instead of a line
+// (ldg_gather). Walking a mask word's bits lane by lane, as before, every load waited for the
+// store before it. Per 3-pass call on B200, before -> now: 2^28 f32 p = 0.01 95.6 -> 66.4 us,
+// p = 0.001 49.6 -> 31.7, p = 0.03 194 -> 146, 2^29 u8 p = 0.01 127 -> 90, 2^27 u64 p = 0.01
+// 74.7 -> 48.2, 2^24 u32 p = 0.01 15.4 -> 14.0.
+// 4 CTAs per SM (64 registers) with 4 loads in flight: 8 loads spill at that bound (86.4 us at
+// 2^28 f32 p = 0.01) and cost a CTA per SM without it (70.0); 5 CTAs spill (97.5).
+// A work item is a 16K-element item (4 groups) when there are more items than resident warps
+// and a quarter of one (one group) when there are fewer, so that a column with few sparse units
+// still spreads over many warps. A dense unit is rejected with two loads, and the whole kernel
+// returns at once when pass 1 saw no sparse block. The TMA kernel skips exactly these units
+// (same count test).
 // ---------------------------------------------------------------------------------
+constexpr uint32_t SPARSE_LIST = 1024;   // indices a warp's list holds: twice what a 16K-element item of a
+                                         // unit at exactly 1/32 holds on average; clustered ones take several rounds
+constexpr uint32_t SPARSE_INFLIGHT = 4;  // payload loads per lane in flight (8 spill, see above)
+
+// The elements listed (indices from `in`), `len` of them, to consecutive outputs.
 template <typename T>
-__device__ __forceinline__ void sparse_groups(const ColumnDesc& c, uint64_t item, uint32_t g_begin, uint32_t g_end,
-                                              uint32_t chunk_log2, uint32_t lane)
+__device__ __forceinline__ void sparse_gather(const uint8_t* in_bytes, uint8_t* out_bytes, const uint16_t* list,
+                                              uint32_t len, uint32_t lane)
 {
-    const T* __restrict__ in = reinterpret_cast<const T*>(c.in);
-    T* __restrict__ out = reinterpret_cast<T*>(c.out);
-    const uint32_t* __restrict__ mask = c.mask;
+    constexpr uint32_t F = sizeof(T) == 8 ? SPARSE_INFLIGHT / 2 : SPARSE_INFLIGHT; // 4 of 8 bytes spill
+    const T* __restrict__ in = reinterpret_cast<const T*>(in_bytes);
+    T* __restrict__ out = reinterpret_cast<T*>(out_bytes) + lane;
+    list += lane;
+    for (uint32_t j0 = 0; j0 < len; j0 += 32 * F) {
+        T x[F];
+        const uint32_t left = len - j0;
+#pragma unroll
+        for (uint32_t i = 0; i < F; ++i)
+            if (lane + 32 * i < left) x[i] = ldg_gather(in + list[j0 + 32 * i]);
+#pragma unroll
+        for (uint32_t i = 0; i < F; ++i)
+            if (lane + 32 * i < left) out[j0 + 32 * i] = x[i];
+    }
+}
+
+template <int GROUPS>
+__device__ __forceinline__ void sparse_groups(const ColumnDesc& c, uint64_t item, uint32_t g_begin,
+                                              uint32_t chunk_log2, uint32_t lane, uint16_t* list)
+{
     const uint64_t n = c.n;
+    const uint64_t e0 = item * 16384 + g_begin * 4096ull; // first element of the work item
+    if (e0 >= n) return;
     const uint64_t nw = (n + 31) / 32;
-    const uint64_t nblocks = (n + 1023) / 1024;
-    const uint64_t unit_elems = unit_elems_for(sizeof(T));
-    const uint64_t sparse_max = unit_elems / 32;
-    const uint64_t unit = (item * 16 * 1024) / unit_elems; // an item never straddles units
+    const uint32_t* __restrict__ mask = c.mask;
+    uint32_t m[GROUPS][4];
+#pragma unroll
+    for (int g = 0; g < GROUPS; ++g) {
+        const uint64_t w0 = e0 / 32 + g * 128ull + lane * 4u; // a multiple of 4
+        if (w0 + 4 <= nw) {
+            const uint4 q = __ldg(reinterpret_cast<const uint4*>(mask + w0));
+            m[g][0] = q.x, m[g][1] = q.y, m[g][2] = q.z, m[g][3] = q.w;
+        } else {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) m[g][k] = w0 + k < nw ? __ldg(mask + w0 + k) : 0u;
+        }
+        if (w0 + 4 >= nw && (n & 31u)) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (w0 + k == nw - 1) m[g][k] &= (1u << (n & 31u)) - 1u;
+        }
+    }
+    const uint64_t pos0 = chunk_offset(c, e0 >> chunk_log2, chunk_log2); // groups start on chunk boundaries
+    const uint32_t wl = 31 - __clz(c.elem_bytes); // log2 of the element width
+    const uint64_t unit_elems = unit_elems_for(1) >> wl;
+    const uint64_t unit = e0 / unit_elems; // an item never straddles units
     const uint64_t u_end_elem = (unit + 1) * unit_elems;
     const uint64_t off_b = chunk_offset(c, (unit * unit_elems) >> chunk_log2, chunk_log2);
     const uint64_t off_e = u_end_elem >= n ? *c.d_count : chunk_offset(c, u_end_elem >> chunk_log2, chunk_log2);
-    if (off_e - off_b > sparse_max) return; // dense unit: the TMA kernel owns it
-    // groups of 4 blocks = 4096 elements start on chunk boundaries (chunk length <= 4096)
-    for (uint64_t b0 = item * 16 + g_begin * 4; b0 < item * 16 + g_end * 4 && b0 < nblocks; b0 += 4) {
-        uint32_t m[4];
+    if (off_e - off_b > unit_elems / 32) return; // dense unit: the TMA kernel owns it
+
+    uint32_t rank[GROUPS]; // of the lane's first selected element of each group, within the work item
+    uint32_t total = 0;
+    uint32_t cnt[GROUPS];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const uint64_t wi = (b0 + k) * 32 + lane;
-            m[k] = 0;
-            if (wi < nw) {
-                m[k] = __ldg(mask + wi);
-                if (wi == nw - 1 && (n & 31u)) m[k] &= (1u << (n & 31u)) - 1u;
-            }
+    for (int g = 0; g < GROUPS; ++g)
+        cnt[g] = __popc(m[g][0]) + __popc(m[g][1]) + __popc(m[g][2]) + __popc(m[g][3]);
+#pragma unroll
+    for (int g = 0; g < GROUPS; g += 2) { // two groups (at most 4096 each) per scan
+        const uint32_t second = g + 1 < GROUPS ? cnt[(g + 1) % GROUPS] : 0u;
+        const uint32_t own = cnt[g] | (second << 16);
+        const uint32_t incl = warp_incl_scan(own, lane);
+        const uint32_t all = __shfl_sync(0xffffffffu, incl, 31);
+        rank[g] = total + ((incl - own) & 0xffffu);
+        total += all & 0xffffu;
+        if (g + 1 < GROUPS) {
+            rank[(g + 1) % GROUPS] = total + ((incl - own) >> 16);
+            total += all >> 16;
         }
-        uint64_t pos0 = chunk_offset(c, (b0 * 1024) >> chunk_log2, chunk_log2);
+    }
+    const uint8_t* const in = c.in + (e0 << wl);
+    uint8_t* out = c.out + (pos0 << wl);
+    for (uint32_t r0 = 0; r0 < total; r0 += SPARSE_LIST) {
+        // indices of ranks [r0, r0 + SPARSE_LIST)
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            // chunks shorter than a group: take the offset where a later chunk starts
-            const uint64_t e0 = (b0 + k) * 1024;
-            if (k > 0 && (e0 & ((1ull << chunk_log2) - 1)) == 0 && e0 < n) pos0 = chunk_offset(c, e0 >> chunk_log2, chunk_log2);
-            const uint32_t cnt = __popc(m[k]);
-            const uint32_t incl = warp_incl_scan(cnt, lane);
-            if (__ballot_sync(0xffffffffu, m[k] != 0u) != 0u) {
-                uint64_t pos = pos0 + incl - cnt;
-                uint32_t mm = m[k];
-                const uint64_t e_word = ((b0 + k) * 32 + lane) * 32;
+        for (int g = 0; g < GROUPS; ++g) {
+            uint32_t at = rank[g] - r0;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                uint32_t mm = m[g][k];
                 while (mm) {
-                    const uint32_t b = __ffs(mm) - 1;
+                    if (at < SPARSE_LIST) list[at] = static_cast<uint16_t>(g * 4096 + lane * 128 + k * 32 + __ffs(mm) - 1);
                     mm &= mm - 1;
-                    out[pos++] = in[e_word + b];
+                    ++at;
                 }
             }
-            pos0 += __shfl_sync(0xffffffffu, incl, 31);
         }
+        __syncwarp();
+        const uint32_t len = total - r0 < SPARSE_LIST ? total - r0 : SPARSE_LIST;
+        switch (wl) {
+            case 0: sparse_gather<uint8_t>(in, out, list, len, lane); break;
+            case 1: sparse_gather<uint16_t>(in, out, list, len, lane); break;
+            case 2: sparse_gather<uint32_t>(in, out, list, len, lane); break;
+            default: sparse_gather<uint64_t>(in, out, list, len, lane); break;
+        }
+        out += static_cast<uint64_t>(SPARSE_LIST) << wl;
+        __syncwarp(); // the list is rewritten by the next round or work item
     }
 }
 
 template <int SPLIT> // work items per 16K-element item: 1 (whole items) or 4 (quarters)
-__global__ void __launch_bounds__(256) k_writeout_sparse(const SparseParams p)
+__global__ void __launch_bounds__(256, 4) k_writeout_sparse(const SparseParams p)
 {
+    __shared__ uint16_t s_list[8][SPARSE_LIST];
+    uint16_t* const list = s_list[threadIdx.x >> 5];
     grid_dependency_wait(); // offsets and counts of pass 2
     __shared__ uint32_t s_hflags;
     const uint32_t hflags = cta_header_flags(p.hdr, &s_hflags);
@@ -765,7 +832,7 @@ __global__ void __launch_bounds__(256) k_writeout_sparse(const SparseParams p)
     // a warp tests 32 work items per round, taken round robin over all warps so that marked
     // items spread evenly whether few or all are marked
     static_assert(SPLIT == 1 || SPLIT == 4, "whole or quarter items");
-    constexpr uint32_t gpw = 4u / SPLIT; // groups per work item
+    constexpr int gpw = 4 / SPLIT; // groups per work item
     const uint64_t num_work = p.num_items * SPLIT;
     for (uint64_t r0 = 0; warp_global + r0 * total_warps < num_work; r0 += 32) {
         const uint64_t mine = warp_global + (r0 + lane) * total_warps;
@@ -778,12 +845,7 @@ __global__ void __launch_bounds__(256) k_writeout_sparse(const SparseParams p)
             const uint32_t g0 = static_cast<uint32_t>(work % SPLIT) * gpw;
             const ColumnDesc& c = column_of(p.col0, p.cols, p.item_col, item);
             const uint64_t il = item - c.item_base;
-            switch (c.elem_bytes) {
-                case 1: sparse_groups<uint8_t>(c, il, g0, g0 + gpw, p.chunk_log2, lane); break;
-                case 2: sparse_groups<uint16_t>(c, il, g0, g0 + gpw, p.chunk_log2, lane); break;
-                case 4: sparse_groups<uint32_t>(c, il, g0, g0 + gpw, p.chunk_log2, lane); break;
-                default: sparse_groups<uint64_t>(c, il, g0, g0 + gpw, p.chunk_log2, lane); break;
-            }
+            sparse_groups<gpw>(c, il, g0, p.chunk_log2, lane, list);
         }
     }
 }
