@@ -688,7 +688,7 @@ def kernel_roofline(cs, torch, args, n, w, d_in, d_mask, d_out, d_count, B, step
     """Roofline of the dominant kernel, timed alone with CUDA events on its stream.
 
     1-pass: the step is the single k_compact_tma launch, so the step time is its time.
-    3-pass: k_compact_tma (writeout) is launched alone through cs_writeout, over the same
+    3-pass: k_writeout_warp is launched alone through cs_writeout, over the same
     inputs with the chunk offsets of the same chunk length, and timed; its algorithmic bytes
     are the call's (every payload byte read once, mask read, selected written; the counts and
     offsets it also reads are under 0.3% of that)."""
@@ -716,7 +716,7 @@ def kernel_roofline(cs, torch, args, n, w, d_in, d_mask, d_out, d_count, B, step
                          args.steps, 3, stream)
         torch.cuda.synchronize()
         verify(torch, d_in, d_mask, d_out, int(total.item()), n)
-        kernel = f"k_compact_tma (3-pass writeout, chunk length {chunk}), launched alone through cs_writeout"
+        kernel = f"k_writeout_warp (3-pass writeout, chunk length {chunk}), launched alone through cs_writeout"
         launches_timed = args.steps
         del counts, offsets, total
     achieved = B / (kms * 1e-3) / 1e9

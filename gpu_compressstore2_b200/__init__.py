@@ -571,13 +571,13 @@ def bench_1pass(id: IntermediateData, d_input, d_mask, d_output, element_count: 
 def bench_auto(id: IntermediateData, d_input, d_mask, d_output, element_count: int, chunk_length: int = 1024,
                grid_size: int = 0) -> Timings:
     """The library's plain call as it runs in production (the tuned form: reduce-then-scan
-    pass 1+2, sparse gather and TMA writeout, or the 1-pass kernel), timed as a whole."""
+    pass 1+2 and the writeout, or the 1-pass kernel), timed as a whole."""
     return id._run(ALGO_AUTO, d_input, d_mask, d_output, element_count, chunk_length, grid_size)
 
 
 def bench_3pass(id: IntermediateData, d_input, d_mask, d_output, element_count: int, chunk_length: int = 1024,
                 grid_size: int = 0) -> Timings:
-    """popcount -> chunk prefix sum -> TMA-staged writeout as three separate calls with
+    """popcount -> chunk prefix sum -> writeout as three separate calls with
     per-phase times; the counterpart of bench10 (src/benchmarks.cuh:418-440). grid_size is
     accepted for the reference's signature; the writeout's persistent grid is fixed."""
     return id._run_phases(ALGO_3PASS, d_input, d_mask, d_output, element_count, chunk_length)

@@ -13,7 +13,7 @@ selectivity is unknown: the plain call cannot measure it before it runs without 
 own. The fastest candidate at each selectivity becomes that selectivity bucket's entry
 (``sel`` lines), which a call takes when its caller states the fraction it expects
 (``cs_config.selectivity``). Within the 3-pass
-hybrid the per-unit choice between the TMA writeout and the sparse gather is made at run time
+hybrid the per-unit choice between the dense writeout and the sparse gather is made at run time
 from the pass-1 counts, so the dense / sparse split needs no table entry.
 
 The batched form has a table of its own, keyed by (element width, size bucket, selectivity
@@ -39,6 +39,7 @@ DEFAULT_TABLE = _lib.TUNE_TABLE
 # candidates: (algo, chunk_length)
 CANDIDATES = [
     (_lib.ALGO_1PASS, 1024),
+    (_lib.ALGO_3PASS, 512),
     (_lib.ALGO_3PASS, 1024),
     (_lib.ALGO_3PASS, 2048),
     (_lib.ALGO_3PASS, 4096),

@@ -216,29 +216,28 @@ ColumnDesc make_column(const void* d_in, const void* d_mask, void* d_out, uint64
     return c;
 }
 
-// Pass 3 of the 3-pass form over chunk offsets already in the workspace: the sparse gather
-// (hybrid only: units with at most 1/32 selected) and the TMA-staged writeout of the rest.
+// Pass 3 of the 3-pass form over chunk offsets already in the workspace: independent warps for
+// chunk lengths up to 4096 (hybrid: units with at most 1/32 selected are gathered), the
+// TMA-staged writeout for longer ones.
 int launch_writeout_3pass(const ColumnDesc& col, const Layout& l, ws_header* hdr, const Resolved& r, bool hybrid,
                           const uint32_t* item_flags, const DeviceInfo& di, cudaStream_t stream)
 {
     const uint32_t elem_bytes = col.elem_bytes;
-    const uint64_t ue = unit_elems_for(elem_bytes);
-    const uint64_t sparse_max = hybrid ? ue / 32 : 0;
-    if (hybrid) {
-        SparseParams spp{};
-        spp.col0 = col;
-        spp.num_items = sparse_items_for(col.n);
-        spp.hdr = hdr;
-        spp.chunk_log2 = r.chunk_log2;
-        spp.item_flags = item_flags;
-        const cudaError_t e = launch_writeout_sparse(spp, di.sms, stream);
-        if (e != cudaSuccess) return cuda_status(e);
+    if (r.chunk_log2 <= 12) {
+        WriteoutParams p{};
+        p.col0 = col;
+        p.num_units = l.num_tiles;
+        p.num_sparse_items = sparse_items_for(col.n);
+        p.sparse_max = hybrid ? unit_elems_for(elem_bytes) / 32 : 0;
+        p.item_flags = item_flags;
+        p.hdr = hdr;
+        p.chunk_log2 = r.chunk_log2;
+        return cuda_status(launch_writeout_warp(p, elem_bytes, r.grid, di.sms, stream));
     }
     CompactParams p{};
     p.col0 = col;
     p.num_tiles = l.num_tiles;
     p.hdr = hdr;
-    p.sparse_max = sparse_max;
     p.chunk_log2 = r.chunk_log2;
     p.skip = r.skip;
     p.timeout_ns = r.timeout_ns;
@@ -262,7 +261,8 @@ int run_compaction(const void* d_in, const void* d_mask, void* d_out, uint64_t n
     const bool tma_ok = aligned(d_in, 16) && aligned(d_out, 16) && aligned(d_mask, 16);
     if ((algo == CS_ALGO_1PASS || algo == CS_ALGO_3PASS) && !tma_ok) {
         if (!auto_route) return CS_ERR_MISALIGNED;
-        algo = CS_ALGO_NAIVE;
+        // the warp writeout takes any element-aligned pointers; it needs the block pass's offsets
+        algo = r.chunk_log2 >= 7 && r.chunk_log2 <= 12 ? CS_ALGO_3PASS : CS_ALGO_NAIVE;
     }
 
     if (algo == CS_ALGO_1PASS) {
@@ -292,7 +292,7 @@ int run_compaction(const void* d_in, const void* d_mask, void* d_out, uint64_t n
     const uint64_t ue = unit_elems_for(elem_bytes);
     const bool tma_writeout = algo == CS_ALGO_3PASS && (1ull << r.chunk_log2) <= ue;
     // passes 1 + 2 in one reduce-then-scan launch (block-relative offsets + block prefixes)
-    const bool blocks = tma_writeout && r.chunk_log2 >= 7 && r.chunk_log2 <= 12 && aligned(d_mask, 16);
+    const bool blocks = tma_writeout && r.chunk_log2 >= 7 && r.chunk_log2 <= 12;
     const bool hybrid = algo == CS_ALGO_3PASS && r.chunk_log2 <= 12 && r.skip;
     uint64_t* blk_base = blocks ? reinterpret_cast<uint64_t*>(ws + l.off_blk_base) : nullptr;
     // with the block pass, pass 1 marks the sparse units' items and the gather visits only those
@@ -554,7 +554,7 @@ int compressstore_if(const void* d_in, void* d_out, uint64_t n, const cs_predica
     if (st) return st;
     Resolved r{};
     r.algo = CS_ALGO_3PASS;
-    r.chunk_log2 = 12; // one chunk per 4096-element row of the predicate pass
+    r.chunk_log2 = 12 - ilog2(w); // a chunk per item of the writeout (4 KB of payload)
     r.grid = 0;
     r.skip = 1;
     r.timeout_ns = DEFAULT_TIMEOUT_NS;
@@ -677,10 +677,19 @@ int cs_writeout(const void* d_in, const uint32_t* d_mask, void* d_out, uint64_t 
     if (algo == CS_ALGO_3PASS) {
         if (!(aligned(d_in, 16) && aligned(d_out, 16) && aligned(d_mask, 16))) return CS_ERR_MISALIGNED;
         if (chunk_length > ue) return CS_ERR_NOT_SUPPORTED;
+        // no workspace: errors are not recorded, inconsistent offsets still never write
+        const ColumnDesc col =
+            make_column(d_in, d_mask, d_out, n, elem_bytes, nullptr, const_cast<uint64_t*>(d_chunk_offsets));
+        if (log2L <= 12) {
+            WriteoutParams p{};
+            p.col0 = col;
+            p.num_units = (n + ue - 1) / ue;
+            p.chunk_log2 = log2L;
+            return cuda_status(launch_writeout_warp(p, elem_bytes, 0, di.sms, s));
+        }
         CompactParams p{};
-        p.col0 = make_column(d_in, d_mask, d_out, n, elem_bytes, nullptr, const_cast<uint64_t*>(d_chunk_offsets));
+        p.col0 = col;
         p.num_tiles = (n + ue - 1) / ue;
-        p.hdr = nullptr; // no workspace: errors are not recorded, inconsistent offsets still never write
         p.chunk_log2 = log2L;
         p.skip = 1;
         p.timeout_ns = DEFAULT_TIMEOUT_NS;

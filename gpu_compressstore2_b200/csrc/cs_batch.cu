@@ -1,12 +1,11 @@
 // cs_batch.cu — the batched form: a plan over many columns of uneven length and width.
 //
-// Each column takes the 3-pass hybrid (4096-element chunks) or the 1-pass form, as the
+// Each column takes the 3-pass hybrid or the 1-pass form, as the
 // batch table of the autotuner says for its (width, size, selectivity) bucket; each pass is
 // ONE launch for all the columns that take it: the reduce-then-scan popcount + prefix kernel
-// walks a flat list of the 3-pass columns' 2^18-element blocks, the sparse-gather kernel walks
-// their 16K-element items, one persistent TMA-staged writeout per element width walks that
-// width's 128 KB units over every SM, and one 1-pass kernel per width walks the 1-pass
-// columns' units (decoupled look-back confined to each column). Work-to-column maps and column
+// walks a flat list of the 3-pass columns' 2^18-element blocks, one writeout per element width
+// walks that width's 128 KB units and sparse 16K-element items over every SM, and one 1-pass
+// kernel per width walks the 1-pass columns' units (decoupled look-back confined to each column). Work-to-column maps and column
 // descriptors are built on the host once (cs_plan.cu) and uploaded with the plan, so a unit
 // finds its column with one load. The launches can be captured in a CUDA graph.
 //
@@ -32,7 +31,6 @@ struct cs_batch {
     PlanLayout layout;
     PlanDevice dev;
     PlanCounts counts;
-    uint32_t grid[4] = {0, 0, 0, 0};
     uint32_t grid1[4] = {0, 0, 0, 0};
     uint32_t one_pass_cols = 0;
     std::vector<cs_column> cols; // for the per-call loop
@@ -61,7 +59,7 @@ int run_direct(cs_batch* b, cudaStream_t s)
         cudaError_t e = cudaMemsetAsync(c, 0, sizeof(uint64_t), s);
         if (e != cudaSuccess) return to_status(e);
     }
-    return plan_launch(b->dev, b->counts, b->grid, b->sms, b->timeout_ns, s, b->grid1);
+    return plan_launch(b->dev, b->counts, b->sms, b->timeout_ns, s, b->grid1);
 }
 
 // Selected fraction of every column, from one reduce-then-scan popcount pass over the masks
@@ -72,7 +70,8 @@ int measure_selectivity(const cs_column* cols, uint32_t ncols, int sms, cudaStre
     std::vector<ColumnDesc> desc;
     std::vector<uint64_t> chunk_base;
     PlanCounts c;
-    int st = plan_columns(cols, ncols, desc, chunk_base, c, nullptr);
+    constexpr uint32_t ROW_LOG2 = 12; // whole 4096-element rows: only the counts are wanted
+    int st = plan_columns(cols, ncols, desc, chunk_base, c, nullptr, nullptr, ROW_LOG2);
     if (st != CS_SUCCESS) return st;
     if (!c.tiles) return CS_SUCCESS;
     const PlanLayout L = plan_layout(c, true);
@@ -97,7 +96,7 @@ int measure_selectivity(const cs_column* cols, uint32_t ncols, int sms, cudaStre
         bp.blk_sum = d.blk_sum;
         bp.blk_base = d.blk_base;
         bp.hdr = d.hdr;
-        bp.chunk_log2 = 12;
+        bp.chunk_log2 = ROW_LOG2;
         bp.keep_begin = d.keep_begin;
         bp.keep_end = d.keep_end;
         e = launch_popc_blocks(bp, sms, s);
@@ -189,8 +188,7 @@ int cs_batch_create(cs_batch** out, const cs_column* cols, uint32_t ncols, const
     }
     // persistent grids (also applies the kernels' shared-memory attribute outside any capture)
     for (int wi = 0; wi < 4; ++wi) {
-        b->grid[wi] = plan_grid(1u << wi, b->counts.units[wi], b->sms, 1);
-        b->grid1[wi] = plan_grid(1u << wi, b->counts.units1[wi], b->sms, 0);
+        b->grid1[wi] = plan_grid(1u << wi, b->counts.units1[wi], b->sms);
     }
     b->kernels_per_run = plan_kernels(b->counts);
     *out = b;

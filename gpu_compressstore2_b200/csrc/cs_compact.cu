@@ -1,4 +1,6 @@
-// cs_compact.cu — the TMA-staged, warp-specialised persistent compaction kernel.
+// cs_compact.cu — the TMA-staged, warp-specialised persistent compaction kernel: the 1-pass
+// form, and the 3-pass writeout for chunks longer than 4096 elements (cs_writeout.cu has the
+// others).
 //
 // Work is split into UNITS of U consecutive tiles; a tile is TILE_BYTES of payload
 // (TILE_BYTES/w elements). One CTA per SM takes units one after another (an atomic ticket
@@ -269,19 +271,12 @@ __global__ void __launch_bounds__(Roles<MODE>::NTHREADS, 1) k_compact_tma(const 
     if (MODE == 0) __syncthreads();
     const uint32_t epoch = (MODE == 0) ? p.hdr->epoch : 0u;
     const bool scan_ok = (hflags & 1u) != 0u; // 3-pass: pass 2 completed cleanly
-    // 3-pass hybrid: some units may belong to the sparse gather kernel
-    const bool hybrid = MODE == 1 && p.sparse_max != 0 && scan_ok && (hflags & 2u) != 0u;
 
     if (warp == 0) {
         // ------------------------------------------------------------- producer
         const uint64_t policy = l2_policy_evict_first();
         bool failed = false;
         // take the next unit id (warp-uniform)
-        // 3-pass hybrid: window of 32 candidates from this CTA's round-robin unit list; bit k
-        // of cand_bits set = candidate cand_base + k is a unit this kernel must process
-        uint64_t cand_base = 0;
-        uint32_t cand_bits = 0;
-        bool cand_loaded = false;
         // 1-pass: lane 0 requests the NEXT ticket right after using the current one, so the
         // atomic's round trip overlaps a unit of streaming. A CTA's tickets still increase,
         // and the one left over at the end lies past the last unit, so no unit is dropped.
@@ -297,27 +292,7 @@ __global__ void __launch_bounds__(Roles<MODE>::NTHREADS, 1) k_compact_tma(const 
                 ticket_pending = true;
                 return __shfl_sync(0xffffffffu, t, 0);
             } else {
-            if (!hybrid) return static_cast<uint64_t>(blockIdx.x) + static_cast<uint64_t>(j) * gridDim.x;
-            while (cand_bits == 0u) {
-                if (cand_loaded) cand_base += 32;
-                cand_loaded = true;
-                const uint64_t u = static_cast<uint64_t>(blockIdx.x) + (cand_base + lane) * gridDim.x;
-                bool take = u >= p.num_tiles; // past the end: sentinel
-                if (!take) {
-                    const ColumnDesc& C = col_of_unit(u);
-                    const uint64_t ul = u - C.unit_base;
-                    const uint64_t e_b = ul * UE, e_e = (ul + 1) * UE;
-                    const uint64_t off_b = chunk_offset(C, e_b >> p.chunk_log2, p.chunk_log2);
-                    const uint64_t off_e =
-                        e_e >= C.n ? *C.d_count : chunk_offset(C, e_e >> p.chunk_log2, p.chunk_log2);
-                    take = off_e - off_b > p.sparse_max;
-                }
-                cand_bits = __ballot_sync(0xffffffffu, take);
-            }
-            const uint32_t k = __ffs(cand_bits) - 1;
-            cand_bits &= cand_bits - 1;
-            const uint64_t pick = static_cast<uint64_t>(blockIdx.x) + (cand_base + k) * gridDim.x;
-            return pick < p.num_tiles ? pick : p.num_tiles;
+                return static_cast<uint64_t>(blockIdx.x) + static_cast<uint64_t>(j) * gridDim.x;
             }
         };
         // arm mask slot j % MSLOTS with unit `unit` (or the end-of-work sentinel)

@@ -488,8 +488,6 @@ struct CompactParams {
     uint64_t num_tiles;            // number of look-back units (UNIT_TILES tiles each) of this launch
     ws_header* hdr;
     uint64_t* status;              // 1-pass: one status per unit
-    uint64_t sparse_max;           // 3-pass hybrid: units with at most this many selected
-                                   // elements belong to the sparse kernel (0: none)
     uint32_t chunk_log2;           // 3-pass: log2(chunk length)
     uint32_t skip;                 // 1: skip payload loads of empty segments
     uint64_t timeout_ns;
@@ -621,15 +619,18 @@ __device__ __forceinline__ void blocks_last_cta(const BlockScanParams& p, uint64
     }
 }
 
-struct SparseParams {
-    ColumnDesc col0;          // single column (cols null)
-    const ColumnDesc* cols;   // batch: item t belongs to cols[item_col[t]]
+// Pass 3 by independent warps (cs_writeout.cu).
+struct WriteoutParams {
+    ColumnDesc col0;          // the column (cols null); unit_base and item_base 0
+    const ColumnDesc* cols;   // batch: unit u belongs to cols[unit_col[u]], sparse item t to
+    const uint32_t* unit_col; // cols[item_col[t]]; items of other widths are another launch's
     const uint32_t* item_col;
-    uint64_t num_items;       // 16-block items over all columns
-    const ws_header* hdr;
-    uint32_t chunk_log2;
-    const uint32_t* item_flags; // items pass 1 marked with its epoch (the sparse ones); null:
-                                // test every item
+    uint64_t num_units;       // 128 KB units of this launch's width over all columns
+    uint64_t num_sparse_items; // 16K-element items over all columns
+    uint64_t sparse_max;      // hybrid: units with at most this many selected are gathered (0: none)
+    const uint32_t* item_flags; // items pass 1 marked with its epoch (the sparse ones); null: test every item
+    ws_header* hdr;
+    uint32_t chunk_log2;      // at most 12
 };
 
 // ---------------------------------------------------------------------------------
@@ -661,7 +662,6 @@ constexpr uint32_t FUSED_TILE_CHUNKS = 64; // 4096-element chunks per reduce-the
 static_assert(FUSED_TILE_CHUNKS * 4096u == (1u << SCAN_BLOCK_LOG2), "a plan tile is one scan block");
 cudaError_t launch_popc_blocks(const BlockScanParams& p, int num_sms, cudaStream_t stream);
 cudaError_t launch_pred_mask(const PredParams& p, int type, int op, int num_sms, cudaStream_t stream);
-cudaError_t launch_writeout_sparse(const SparseParams& p, int num_sms, cudaStream_t stream);
 __host__ __device__ constexpr uint64_t sparse_items_for(uint64_t n)
 {
     return ((n + 1023) / 1024 + 15) / 16; // items of 16 blocks of 1024 elements
@@ -674,6 +674,10 @@ cudaError_t launch_writeout_naive(const void* in, const uint32_t* mask, void* ou
 // unit_tiles: tiles per look-back unit, UNIT_TILES or (mode 0 only) 1 for short columns.
 cudaError_t launch_compact_tma(const CompactParams& p, uint32_t elem_bytes, int mode, uint32_t grid,
                                cudaStream_t stream, uint32_t unit_tiles = UNIT_TILES);
+// 3-pass writeout by independent warps (cs_writeout.cu): pointers aligned to the element width
+// and 4 bytes (mask). `requested`: CTAs, 0 for one resident wave.
+cudaError_t launch_writeout_warp(const WriteoutParams& p, uint32_t elem_bytes, uint32_t requested, int num_sms,
+                                 cudaStream_t stream);
 // Occupancy-derived resident CTAs per SM of the TMA kernel (after its smem attribute is set).
 int compact_tma_blocks_per_sm(uint32_t elem_bytes, int mode, uint32_t unit_tiles = UNIT_TILES);
 // Dynamic shared memory of one TMA-kernel CTA (its Layout TOTAL); 0 for bad arguments.

@@ -279,8 +279,7 @@ __device__ __forceinline__ void mark_sparse_units(const BlockScanParams& p, cons
 }
 
 // ---------------------------------------------------------------------------------
-// Pass 1 + 2 as one reduce-then-scan kernel (3-pass form, chunk length L = 128 .. 4096,
-// 16-byte-aligned masks). A column is cut into blocks of 2^18 elements (32 KB of mask). A
+// Pass 1 + 2 as one reduce-then-scan kernel (3-pass form, chunk length L = 128 .. 4096). A column is cut into blocks of 2^18 elements (32 KB of mask). A
 // CTA takes whole blocks by static assignment and never waits on another CTA: its 8 warps
 // each load 8 rows of 32 uint4 (4096 elements per row) in one round, each lane's share of a
 // chunk is summed over the LPC = L/128 lanes holding the chunk, and warp and block scans
@@ -296,7 +295,8 @@ __device__ __forceinline__ void mark_sparse_units(const BlockScanParams& p, cons
 // ---------------------------------------------------------------------------------
 
 // This warp's 8 rows (32 uint4 each) of block `bl` of `col`, read from global memory: the
-// last word of the column has its bits past n cleared, and words past the column read 0.
+// last word of the column has its bits past n cleared, and words past the column read 0. A mask
+// that starts inside a 16-byte group (4-byte aligned) is read word by word.
 __device__ __forceinline__ void popc_block_load(const ColumnDesc& col, uint64_t bl, uint32_t warp, uint32_t lane,
                                                 uint4 (&q)[8])
 {
@@ -305,10 +305,11 @@ __device__ __forceinline__ void popc_block_load(const ColumnDesc& col, uint64_t 
     const uint32_t* __restrict__ mask = col.mask;
     const uint4* mv = reinterpret_cast<const uint4*>(mask);
     const uint64_t row0 = bl * 64 + warp * 8; // this warp's first row (4096 elements each)
+    const bool vec = (reinterpret_cast<uintptr_t>(mask) & 15u) == 0;
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
         const uint64_t vi = (row0 + r) * 32 + lane;
-        if (vi * 4 + 3 < nw) {
+        if (vec && vi * 4 + 3 < nw) {
             q[r] = __ldg(mv + vi);
             if (vi * 4 + 3 == nw - 1 && (n & 31u)) q[r].w &= (1u << (n & 31u)) - 1u;
         } else {
@@ -487,8 +488,10 @@ __global__ void __launch_bounds__(256, POPC_STREAM_CTAS) k_popc_stream(const Blo
         s_fail = 0u;
     }
     grid_dependency_wait(); // the mask may come from the previous kernel, the workspace too
-    // a block is copied in bulk when all its bits lie inside its column
-    auto whole = [&](const ColumnDesc& c, uint64_t bl) -> bool { return ((bl + 1) << SCAN_BLOCK_LOG2) <= c.n; };
+    // a block is copied in bulk when all its bits lie inside its column and its mask is 16-byte aligned
+    auto whole = [&](const ColumnDesc& c, uint64_t bl) -> bool {
+        return ((bl + 1) << SCAN_BLOCK_LOG2) <= c.n && (reinterpret_cast<uintptr_t>(c.mask) & 15u) == 0;
+    };
     uint32_t pending = 0; // thread 0: stages with a copy in flight
     auto issue = [&](uint64_t blk, uint32_t s) {
         const ColumnDesc& c = column_of(p.col0, p.cols, p.blk_col, blk);
@@ -681,205 +684,6 @@ cudaError_t launch_writeout_naive(const void* in, const uint32_t* mask, void* ou
     }
     note_launch();
     return cudaGetLastError();
-}
-
-// ---------------------------------------------------------------------------------
-// Pass 3, sparse units (3-pass hybrid, chunk length <= 4096). Units of the TMA kernel whose
-// selected count is at most sparse_max are compacted here instead: DRAM traffic is the mask
-// plus the sectors holding selected elements.
-// What bounds it is latency (per item a flag, then the mask, then the payload) and, at 1% and
-// above, DRAM sectors. A warp therefore loads the masks of a whole work item at once (128
-// consecutive elements per lane and 4096-element group), writes the indices of its selected
-// elements to a list in shared memory at their ranks (one packed scan per two groups), and
-// gathers from the list with SPARSE_INFLIGHT loads per lane in flight before the first store;
-// the stores of a warp are consecutive, and a load fetches 64 bytes instead of a line
-// (ldg_gather). Walking a mask word's bits lane by lane, as before, every load waited for the
-// store before it. Per 3-pass call on B200, before -> now: 2^28 f32 p = 0.01 95.6 -> 66.4 us,
-// p = 0.001 49.6 -> 31.7, p = 0.03 194 -> 146, 2^29 u8 p = 0.01 127 -> 90, 2^27 u64 p = 0.01
-// 74.7 -> 48.2, 2^24 u32 p = 0.01 15.4 -> 14.0.
-// 4 CTAs per SM (64 registers) with 4 loads in flight: 8 loads spill at that bound (86.4 us at
-// 2^28 f32 p = 0.01) and cost a CTA per SM without it (70.0); 5 CTAs spill (97.5).
-// A work item is a 16K-element item (4 groups) when there are more items than resident warps
-// and a quarter of one (one group) when there are fewer, so that a column with few sparse units
-// still spreads over many warps. A dense unit is rejected with two loads, and the whole kernel
-// returns at once when pass 1 saw no sparse block. The TMA kernel skips exactly these units
-// (same count test).
-// ---------------------------------------------------------------------------------
-constexpr uint32_t SPARSE_LIST = 1024;   // indices a warp's list holds: twice what a 16K-element item of a
-                                         // unit at exactly 1/32 holds on average; clustered ones take several rounds
-constexpr uint32_t SPARSE_INFLIGHT = 4;  // payload loads per lane in flight (8 spill, see above)
-
-// The elements listed (indices from `in`), `len` of them, to consecutive outputs.
-template <typename T>
-__device__ __forceinline__ void sparse_gather(const uint8_t* in_bytes, uint8_t* out_bytes, const uint16_t* list,
-                                              uint32_t len, uint32_t lane)
-{
-    constexpr uint32_t F = sizeof(T) == 8 ? SPARSE_INFLIGHT / 2 : SPARSE_INFLIGHT; // 4 of 8 bytes spill
-    const T* __restrict__ in = reinterpret_cast<const T*>(in_bytes);
-    T* __restrict__ out = reinterpret_cast<T*>(out_bytes) + lane;
-    list += lane;
-    for (uint32_t j0 = 0; j0 < len; j0 += 32 * F) {
-        T x[F];
-        const uint32_t left = len - j0;
-#pragma unroll
-        for (uint32_t i = 0; i < F; ++i)
-            if (lane + 32 * i < left) x[i] = ldg_gather(in + list[j0 + 32 * i]);
-#pragma unroll
-        for (uint32_t i = 0; i < F; ++i)
-            if (lane + 32 * i < left) out[j0 + 32 * i] = x[i];
-    }
-}
-
-template <int GROUPS>
-__device__ __forceinline__ void sparse_groups(const ColumnDesc& c, uint64_t item, uint32_t g_begin,
-                                              uint32_t chunk_log2, uint32_t lane, uint16_t* list)
-{
-    const uint64_t n = c.n;
-    const uint64_t e0 = item * 16384 + g_begin * 4096ull; // first element of the work item
-    if (e0 >= n) return;
-    const uint64_t nw = (n + 31) / 32;
-    const uint32_t* __restrict__ mask = c.mask;
-    uint32_t m[GROUPS][4];
-#pragma unroll
-    for (int g = 0; g < GROUPS; ++g) {
-        const uint64_t w0 = e0 / 32 + g * 128ull + lane * 4u; // a multiple of 4
-        if (w0 + 4 <= nw) {
-            const uint4 q = __ldg(reinterpret_cast<const uint4*>(mask + w0));
-            m[g][0] = q.x, m[g][1] = q.y, m[g][2] = q.z, m[g][3] = q.w;
-        } else {
-#pragma unroll
-            for (int k = 0; k < 4; ++k) m[g][k] = w0 + k < nw ? __ldg(mask + w0 + k) : 0u;
-        }
-        if (w0 + 4 >= nw && (n & 31u)) {
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-                if (w0 + k == nw - 1) m[g][k] &= (1u << (n & 31u)) - 1u;
-        }
-    }
-    const uint64_t pos0 = chunk_offset(c, e0 >> chunk_log2, chunk_log2); // groups start on chunk boundaries
-    const uint32_t wl = 31 - __clz(c.elem_bytes); // log2 of the element width
-    const uint64_t unit_elems = unit_elems_for(1) >> wl;
-    const uint64_t unit = e0 / unit_elems; // an item never straddles units
-    const uint64_t u_end_elem = (unit + 1) * unit_elems;
-    const uint64_t off_b = chunk_offset(c, (unit * unit_elems) >> chunk_log2, chunk_log2);
-    const uint64_t off_e = u_end_elem >= n ? *c.d_count : chunk_offset(c, u_end_elem >> chunk_log2, chunk_log2);
-    if (off_e - off_b > unit_elems / 32) return; // dense unit: the TMA kernel owns it
-
-    uint32_t rank[GROUPS]; // of the lane's first selected element of each group, within the work item
-    uint32_t total = 0;
-    uint32_t cnt[GROUPS];
-#pragma unroll
-    for (int g = 0; g < GROUPS; ++g)
-        cnt[g] = __popc(m[g][0]) + __popc(m[g][1]) + __popc(m[g][2]) + __popc(m[g][3]);
-#pragma unroll
-    for (int g = 0; g < GROUPS; g += 2) { // two groups (at most 4096 each) per scan
-        const uint32_t second = g + 1 < GROUPS ? cnt[(g + 1) % GROUPS] : 0u;
-        const uint32_t own = cnt[g] | (second << 16);
-        const uint32_t incl = warp_incl_scan(own, lane);
-        const uint32_t all = __shfl_sync(0xffffffffu, incl, 31);
-        rank[g] = total + ((incl - own) & 0xffffu);
-        total += all & 0xffffu;
-        if (g + 1 < GROUPS) {
-            rank[(g + 1) % GROUPS] = total + ((incl - own) >> 16);
-            total += all >> 16;
-        }
-    }
-    const uint8_t* const in = c.in + (e0 << wl);
-    uint8_t* out = c.out + (pos0 << wl);
-    for (uint32_t r0 = 0; r0 < total; r0 += SPARSE_LIST) {
-        // indices of ranks [r0, r0 + SPARSE_LIST)
-#pragma unroll
-        for (int g = 0; g < GROUPS; ++g) {
-            uint32_t at = rank[g] - r0;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                uint32_t mm = m[g][k];
-                while (mm) {
-                    if (at < SPARSE_LIST) list[at] = static_cast<uint16_t>(g * 4096 + lane * 128 + k * 32 + __ffs(mm) - 1);
-                    mm &= mm - 1;
-                    ++at;
-                }
-            }
-        }
-        __syncwarp();
-        const uint32_t len = total - r0 < SPARSE_LIST ? total - r0 : SPARSE_LIST;
-        switch (wl) {
-            case 0: sparse_gather<uint8_t>(in, out, list, len, lane); break;
-            case 1: sparse_gather<uint16_t>(in, out, list, len, lane); break;
-            case 2: sparse_gather<uint32_t>(in, out, list, len, lane); break;
-            default: sparse_gather<uint64_t>(in, out, list, len, lane); break;
-        }
-        out += static_cast<uint64_t>(SPARSE_LIST) << wl;
-        __syncwarp(); // the list is rewritten by the next round or work item
-    }
-}
-
-template <int SPLIT> // work items per 16K-element item: 1 (whole items) or 4 (quarters)
-__global__ void __launch_bounds__(256, 4) k_writeout_sparse(const SparseParams p)
-{
-    __shared__ uint16_t s_list[8][SPARSE_LIST];
-    uint16_t* const list = s_list[threadIdx.x >> 5];
-    grid_dependency_wait(); // offsets and counts of pass 2
-    __shared__ uint32_t s_hflags;
-    const uint32_t hflags = cta_header_flags(p.hdr, &s_hflags);
-    if (!(hflags & 1u)) return; // pass 2 offsets not trustworthy: write nothing
-    if (!(hflags & 2u)) return; // no 16K block with <= 1/32 selected: no sparse unit
-    // items pass 1 marked carry the epoch of that pass, the one before the current
-    const uint32_t mark = p.item_flags ? prev_epoch(*reinterpret_cast<const volatile uint32_t*>(&p.hdr->epoch)) : 0u;
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint64_t warp_global = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    const uint64_t total_warps = (static_cast<uint64_t>(gridDim.x) * blockDim.x) >> 5;
-    // a warp tests 32 work items per round, taken round robin over all warps so that marked
-    // items spread evenly whether few or all are marked
-    static_assert(SPLIT == 1 || SPLIT == 4, "whole or quarter items");
-    constexpr int gpw = 4 / SPLIT; // groups per work item
-    const uint64_t num_work = p.num_items * SPLIT;
-    for (uint64_t r0 = 0; warp_global + r0 * total_warps < num_work; r0 += 32) {
-        const uint64_t mine = warp_global + (r0 + lane) * total_warps;
-        const bool flagged = mine < num_work && (!p.item_flags || __ldg(p.item_flags + mine / SPLIT) == mark);
-        uint32_t todo = __ballot_sync(0xffffffffu, flagged);
-        while (todo) {
-            const uint64_t work = warp_global + (r0 + (__ffs(todo) - 1)) * total_warps;
-            todo &= todo - 1;
-            const uint64_t item = work / SPLIT;
-            const uint32_t g0 = static_cast<uint32_t>(work % SPLIT) * gpw;
-            const ColumnDesc& c = column_of(p.col0, p.cols, p.item_col, item);
-            const uint64_t il = item - c.item_base;
-            sparse_groups<gpw>(c, il, g0, p.chunk_log2, lane, list);
-        }
-    }
-}
-
-// CTAs of 256 threads of KERNEL resident on one SM at once (taken once). Grid-stride passes
-// launch one wave of them: CTAs past the first wave would run their whole round-robin share
-// after it.
-template <auto KERNEL>
-int resident_per_sm_256()
-{
-    static std::atomic<int> cached{0};
-    int v = cached.load(std::memory_order_relaxed);
-    if (v > 0) return v;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, KERNEL, 256, 0) != cudaSuccess || v < 1) {
-        cudaGetLastError();
-        v = 4;
-    }
-    cached.store(v, std::memory_order_relaxed);
-    return v;
-}
-
-cudaError_t launch_writeout_sparse(const SparseParams& p, int num_sms, cudaStream_t stream)
-{
-    const bool quarters = p.num_items * 4 <= static_cast<uint64_t>(num_sms) * 64; // while there are warps for them
-    const uint64_t per_sm = quarters ? resident_per_sm_256<k_writeout_sparse<4>>() : resident_per_sm_256<k_writeout_sparse<1>>();
-    const uint64_t cap = static_cast<uint64_t>(num_sms) * per_sm; // CTAs of 8 warps
-    uint64_t blocks = (p.num_items * (quarters ? 4 : 1) + 7) / 8;
-    if (blocks > cap) blocks = cap;
-    if (blocks == 0) blocks = 1;
-    const cudaError_t e = quarters
-        ? launch_pdl(k_writeout_sparse<4>, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, stream, p)
-        : launch_pdl(k_writeout_sparse<1>, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, stream, p);
-    note_launch();
-    return e;
 }
 
 // ---------------------------------------------------------------------------------

@@ -42,12 +42,13 @@ constexpr uint64_t SPARSE_ITEM_ELEMS = 16384ull;
 
 } // namespace
 
-void plan_column_work(uint64_t n, uint32_t w, uint64_t* tiles, uint64_t* items, uint64_t* units, uint64_t* chunks)
+void plan_column_work(uint64_t n, uint32_t w, uint64_t* tiles, uint64_t* items, uint64_t* units, uint64_t* chunks,
+                      uint32_t chunk_log2)
 {
-    const uint64_t ch = (n + 4095) / 4096;
+    const uint64_t ch = (n + (1ull << chunk_log2) - 1) >> chunk_log2;
     const uint64_t ue = unit_elems_for(w);
     *chunks = ch;
-    *tiles = (ch + FUSED_TILE_CHUNKS - 1) / FUSED_TILE_CHUNKS;
+    *tiles = (n + FUSED_TILE_ELEMS - 1) / FUSED_TILE_ELEMS;
     *items = sparse_items_for(n);
     *units = (n + ue - 1) / ue;
 }
@@ -60,7 +61,7 @@ PlanCounts plan_capacity(uint64_t max_elems, uint32_t max_cols)
     c.tiles = max_elems / FUSED_TILE_ELEMS + max_cols;
     c.items = max_elems / SPARSE_ITEM_ELEMS + max_cols;
     for (int wi = 0; wi < 4; ++wi) c.units[wi] = max_elems / unit_elems_for(1u << wi) + max_cols;
-    c.chunks = max_elems / 4096 + max_cols;
+    c.chunks = (max_elems >> PLAN_CHUNK_LOG2) + max_cols;
     return c;
 }
 
@@ -143,7 +144,7 @@ PlanDevice plan_device(uint8_t* base, const PlanLayout& L, const PlanMaps& m)
 
 int plan_columns(const cs_column* cols, uint32_t ncols, std::vector<ColumnDesc>& desc,
                  std::vector<uint64_t>& chunk_base, PlanCounts& tot, std::vector<uint64_t*>* empty,
-                 const std::vector<uint8_t>* one_pass)
+                 const std::vector<uint8_t>* one_pass, uint32_t chunk_log2)
 {
     desc.assign(ncols, ColumnDesc{});
     chunk_base.assign(ncols, 0);
@@ -171,7 +172,7 @@ int plan_columns(const cs_column* cols, uint32_t ncols, std::vector<ColumnDesc>&
         d.out = static_cast<uint8_t*>(col.d_out);
         d.n = col.n;
         uint64_t tiles, items, units, chunks;
-        plan_column_work(col.n, w, &tiles, &items, &units, &chunks);
+        plan_column_work(col.n, w, &tiles, &items, &units, &chunks, chunk_log2);
         const int wi = plan_width_index(w);
         if (one_pass && (*one_pass)[c]) {
             d.one_pass = 1;
@@ -222,10 +223,10 @@ void plan_write_image(uint8_t* img, const PlanMaps& m, const PlanDevice& dev, co
     }
 }
 
-uint32_t plan_grid(uint32_t w, uint64_t units, int sms, int mode)
+uint32_t plan_grid(uint32_t w, uint64_t units, int sms)
 {
     if (!units) return 0;
-    int bps = compact_tma_blocks_per_sm(w, mode);
+    int bps = compact_tma_blocks_per_sm(w, 0);
     if (bps < 1) bps = 1;
     uint64_t g = static_cast<uint64_t>(bps) * sms;
     if (g > units) g = units;
@@ -234,13 +235,13 @@ uint32_t plan_grid(uint32_t w, uint64_t units, int sms, int mode)
 
 uint32_t plan_kernels(const PlanCounts& c)
 {
-    uint32_t k = (c.tiles ? 1u : 0u) + (c.items ? 1u : 0u);
+    uint32_t k = c.tiles ? 1u : 0u;
     for (int wi = 0; wi < 4; ++wi) k += (c.units[wi] ? 1u : 0u) + (c.units1[wi] ? 1u : 0u);
     return k;
 }
 
-int plan_launch(const PlanDevice& d, const PlanCounts& c, const uint32_t grid[4], int sms, uint64_t timeout_ns,
-                cudaStream_t s, const uint32_t* grid1)
+int plan_launch(const PlanDevice& d, const PlanCounts& c, int sms, uint64_t timeout_ns, cudaStream_t s,
+                const uint32_t* grid1)
 {
     if (c.tiles) {
         BlockScanParams bp{};
@@ -251,36 +252,26 @@ int plan_launch(const PlanDevice& d, const PlanCounts& c, const uint32_t grid[4]
         bp.blk_base = d.blk_base;
         bp.hdr = d.hdr;
         bp.item_flags = d.item_flags;
-        bp.chunk_log2 = 12;
+        bp.chunk_log2 = PLAN_CHUNK_LOG2;
         bp.keep_begin = d.keep_begin;
         bp.keep_end = d.keep_end;
         cudaError_t e = launch_popc_blocks(bp, sms, s);
         if (e != cudaSuccess) return to_status(e);
     }
-    if (c.items) {
-        SparseParams spp{};
-        spp.cols = d.cols;
-        spp.item_col = d.item_col;
-        spp.num_items = c.items;
-        spp.hdr = d.hdr;
-        spp.chunk_log2 = 12;
-        spp.item_flags = d.item_flags;
-        cudaError_t e = launch_writeout_sparse(spp, sms, s);
-        if (e != cudaSuccess) return to_status(e);
-    }
     for (int wi = 0; wi < 4; ++wi) {
         if (!c.units[wi]) continue;
         const uint32_t w = 1u << wi;
-        CompactParams p{};
-        p.num_tiles = c.units[wi];
-        p.hdr = d.hdr;
-        p.sparse_max = unit_elems_for(w) / 32;
-        p.chunk_log2 = 12;
-        p.skip = 1;
-        p.timeout_ns = timeout_ns;
+        WriteoutParams p{};
         p.cols = d.cols;
         p.unit_col = d.unit_col[wi];
-        cudaError_t e = launch_compact_tma(p, w, 1, grid[wi], s);
+        p.item_col = d.item_col;
+        p.num_units = c.units[wi];
+        p.num_sparse_items = c.items;
+        p.sparse_max = unit_elems_for(w) / 32;
+        p.item_flags = d.item_flags;
+        p.hdr = d.hdr;
+        p.chunk_log2 = PLAN_CHUNK_LOG2;
+        cudaError_t e = launch_writeout_warp(p, w, 0, sms, s);
         if (e != cudaSuccess) return to_status(e);
     }
     for (int wi = 0; wi < 4; ++wi) {

@@ -26,12 +26,18 @@
 
 namespace cs {
 
+// Chunk length of a plan's 3-pass columns: the smallest item of the writeout (4 KB of 8-byte
+// elements), so that no item starts inside a chunk. (With 4096-element chunks a warp popcounts
+// the chunk before its item: the plain call at 2^28 f32 takes 297 us instead of 268, at 2^27 u64
+// 288 instead of 255.)
+constexpr uint32_t PLAN_CHUNK_LOG2 = 9;
+
 struct PlanCounts {
-    uint64_t tiles = 0;               // 2^18-element blocks (64 chunks of 4096) over the 3-pass columns
-    uint64_t items = 0;               // sparse-kernel items (16K elements) over the 3-pass columns
-    uint64_t units[4] = {0, 0, 0, 0}; // TMA units of the 3-pass columns per width index (1, 2, 4, 8 bytes)
+    uint64_t tiles = 0;               // 2^18-element blocks over the 3-pass columns
+    uint64_t items = 0;               // sparse items (16K elements) over the 3-pass columns
+    uint64_t units[4] = {0, 0, 0, 0}; // 128 KB units of the 3-pass columns per width index (1, 2, 4, 8 bytes)
     uint64_t units1[4] = {0, 0, 0, 0}; // TMA units of the 1-pass columns per width index
-    uint64_t chunks = 0;              // 4096-element chunks over the 3-pass columns (offsets array)
+    uint64_t chunks = 0;              // PLAN_CHUNK-element chunks over the 3-pass columns (offsets array)
     uint64_t cols = 0;
 };
 
@@ -73,7 +79,8 @@ inline int plan_width_index(uint32_t w)
 }
 
 // Work of one column of n elements of width w.
-void plan_column_work(uint64_t n, uint32_t w, uint64_t* tiles, uint64_t* items, uint64_t* units, uint64_t* chunks);
+void plan_column_work(uint64_t n, uint32_t w, uint64_t* tiles, uint64_t* items, uint64_t* units, uint64_t* chunks,
+                      uint32_t chunk_log2 = PLAN_CHUNK_LOG2);
 
 // Upper bound on the work of any set of at most `max_cols` columns holding at most
 // `max_elems` elements in total, of any widths.
@@ -93,25 +100,26 @@ PlanDevice plan_device(uint8_t* dbase, const PlanLayout& L, const PlanMaps& m);
 // no blocks, items or chunks. Returns a cs_status.
 int plan_columns(const cs_column* cols, uint32_t ncols, std::vector<ColumnDesc>& desc,
                  std::vector<uint64_t>& chunk_base, PlanCounts& tot, std::vector<uint64_t*>* empty,
-                 const std::vector<uint8_t>* one_pass = nullptr);
+                 const std::vector<uint8_t>* one_pass = nullptr, uint32_t chunk_log2 = PLAN_CHUNK_LOG2);
 
 // Write the descriptors and maps as the host image (m.bytes) of the maps region; each
 // descriptor's offsets and block-prefix pointers refer to dev.offsets and dev.blk_base.
 void plan_write_image(uint8_t* img, const PlanMaps& m, const PlanDevice& dev, const std::vector<ColumnDesc>& desc,
                       const std::vector<uint64_t>& chunk_base);
 
-// Persistent grid of the TMA kernel (mode 1: 3-pass writeout, 0: 1-pass) for `units` units of width w.
-uint32_t plan_grid(uint32_t w, uint64_t units, int sms, int mode = 1);
+// Persistent grid of the 1-pass TMA kernel for `units` units of width w.
+uint32_t plan_grid(uint32_t w, uint64_t units, int sms);
 
 // Kernels one run of the plan launches.
 uint32_t plan_kernels(const PlanCounts& c);
 
 // Enqueue the plan's kernels on the stream: for the 3-pass columns the reduce-then-scan
-// popcount + prefix pass, the sparse gather and one TMA writeout per width present; then one
+// popcount + prefix pass and one writeout per width present (which also gathers that width's
+// sparse units); then one
 // 1-pass TMA kernel per width with 1-pass columns (grid1, may be null when there are none).
 // The 1-pass kernels come last: each advances the workspace epoch, which the 3-pass writeouts
 // read to validate the pass-2 results. Returns a cs_status.
-int plan_launch(const PlanDevice& d, const PlanCounts& c, const uint32_t grid[4], int sms, uint64_t timeout_ns,
-                cudaStream_t s, const uint32_t* grid1 = nullptr);
+int plan_launch(const PlanDevice& d, const PlanCounts& c, int sms, uint64_t timeout_ns, cudaStream_t s,
+                const uint32_t* grid1 = nullptr);
 
 } // namespace cs

@@ -1,7 +1,6 @@
 // cs_predicate.cu — pass 0 of predicate compaction: the selection mask is computed from
 // the payload on the device instead of being read (k_pred_mask). The 3-pass form then runs
-// on that mask: k_popc_blocks (chunk counts and prefixes), the sparse gather and the
-// TMA-staged writeout.
+// on that mask: k_popc_blocks (chunk counts and prefixes) and the writeout.
 // Reference: the reference evaluates the predicate on the host while packing the mask
 // (gen_predicate, src/utils.cuh:102-122, with predicate_function x > threshold,
 // src/main.cu:24-28,92) and copies mask and payload to the device before compacting.

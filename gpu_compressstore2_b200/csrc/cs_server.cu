@@ -323,12 +323,7 @@ int launch_slot(cs_server* s, Slot& sl, const std::vector<Req*>& rs)
         plan_write_image(sl.himg, m, d, desc, chunk_base);
         e = cudaMemcpyAsync(d.maps, sl.himg, m.bytes, cudaMemcpyHostToDevice, st);
         if (e != cudaSuccess) return to_status(e);
-        uint32_t grid[4];
-        for (int wi = 0; wi < 4; ++wi) {
-            const uint64_t g = static_cast<uint64_t>(s->bps[wi]) * s->sms;
-            grid[wi] = static_cast<uint32_t>(std::min<uint64_t>(g, c.units[wi]));
-        }
-        rc = plan_launch(d, c, grid, s->sms, s->cfg.timeout_ns, st);
+        rc = plan_launch(d, c, s->sms, s->cfg.timeout_ns, st);
         if (rc != CS_SUCCESS) return rc;
         kernels = plan_kernels(c);
         result_bytes = s->layout.off_counts + 8 * rs.size(); // header and counts are contiguous

@@ -66,7 +66,7 @@ typedef enum cs_status {
 typedef enum cs_algo {
     CS_ALGO_AUTO = 0,   /* autotuner table (size x width bucket) */
     CS_ALGO_1PASS = 1,  /* single-pass decoupled look-back, TMA-staged persistent kernel */
-    CS_ALGO_3PASS = 2,  /* chunk popcount -> chunk prefix sum -> TMA-staged writeout */
+    CS_ALGO_3PASS = 2,  /* chunk popcount -> chunk prefix sum -> writeout */
     CS_ALGO_NAIVE = 3   /* chunk popcount -> prefix sum -> warp-per-word writeout, no
                            alignment requirement beyond elem_bytes */
 } cs_algo;
@@ -201,7 +201,7 @@ CS_API int cs_chunk_prefix_sum(const uint32_t* d_chunk_counts, uint64_t chunk_co
  * skip empty chunks). chunk_length must equal the one used in pass 1.
  * Replaces launch_3pass_proc_true<T, true> / kernel_3pass_proc_true_striding_optimized_
  * writeout (src/kernels/kernel_3pass.cuh:329-576) and launch_3pass_proc_none
- * (src/kernels/kernel_3pass.cuh:578-693). algo CS_ALGO_3PASS (TMA-staged, 16-byte
+ * (src/kernels/kernel_3pass.cuh:578-693). algo CS_ALGO_3PASS (16-byte
  * aligned pointers, chunk_length <= 4 * cs_tile_elems(elem_bytes)) or CS_ALGO_NAIVE (any
  * element-aligned pointers, any chunk length). */
 CS_API int cs_writeout(const void* d_in, const uint32_t* d_mask, void* d_out, uint64_t n,
@@ -301,11 +301,10 @@ CS_API int cs_gen_mask_pattern(uint32_t* d_mask, uint64_t n, uint32_t pattern, u
 
 /* ------------------------------------------------------------------------------------
  * Batched form: many columns of uneven length and element width compacted by one plan.
- * Each column takes the 3-pass hybrid (4096-element chunks) or the 1-pass form, and each
+ * Each column takes the 3-pass hybrid or the 1-pass form, and each
  * pass runs ONCE for all the columns that take it: one reduce-then-scan popcount + prefix
- * launch over the 3-pass columns' blocks, one sparse-gather launch over their items, one
- * persistent TMA-staged writeout launch per element width over their units (a work list
- * spread over every SM), and one 1-pass launch per element width over the 1-pass columns'
+ * launch over the 3-pass columns' blocks, one writeout launch per element width over their
+ * units and sparse items (a work list spread over every SM), and one 1-pass launch per element width over the 1-pass columns'
  * units (decoupled look-back confined to each column). The plan is built once
  * (descriptors, work-to-column maps and scratch live in one device allocation made by
  * cs_batch_create); cs_batch_graph captures the launches in a CUDA graph that later
