@@ -3,12 +3,19 @@
 // Element i is selected when bit (i % L) of `pattern` is set (LSB-first, 1 <= L <= 32). With
 // P = popcount of the pattern's L bits, output j is input (j / P) * L + pos[j % P], pos[r]
 // being the r-th set bit: every output has a closed-form source, so there is no popcount
-// pass, no scan and no mask read. Each thread produces 16-byte output vectors (16 / w
-// consecutive outputs, streaming stores) and gathers their sources with read-only loads;
-// neighbouring lanes read neighbouring periods, so the loads of a warp fall on few lines
-// and DRAM reads each touched sector once. A thread keeps the loads of 16 outputs in flight
-// before it stores, and the (quotient, remainder) of the output index advances
-// incrementally, so a thread divides once.
+// pass, no scan and no mask read. Two kernels:
+//
+// k_pattern gathers. A warp produces runs of 128 output bytes (256 for 8-byte elements): each
+// lane 4 consecutive bytes of them (1, 2 or 4 elements) or one 8-byte element, so that one load
+// instruction of the warp falls on the few lines that its outputs come from and one store
+// instruction writes whole lines. The offsets of a lane's sources repeat every P such runs: they
+// come from a table in shared memory, and a thread divides once. A thread keeps the loads of
+// PATTERN_RUNS runs in flight before it stores. Where the selected elements lie 64 bytes and more
+// apart a load fetches 64 bytes instead of a line (2^28 u32, 1 of 32: 163 -> 91 us).
+//
+// k_pattern_dense streams the input through registers and a stage per warp as the 3-pass
+// writeout does (cs_writeout.cu), with mask bits and positions from the pattern; it runs at the HBM
+// rate from about a third selected on (2^28 u32, 31 of 32: 2.11 GB in 322 us).
 // Reference: bench9_pattern (src/benchmarks.cuh:397-416) over launch_pattern_proc /
 // kernel_pattern_proc (src/kernels/kernel_pattern.cuh:13-131), whose pattern is read from
 // the most significant bit (element i <-> bit 31 - i % L); pass __brev of such a pattern.
@@ -18,93 +25,247 @@
 
 #include "compressstore.h"
 #include "cs_internal.cuh"
+#include "cs_place.cuh"
 
 namespace cs {
 
 namespace {
 
-template <typename T, bool VEC_OUT>
+constexpr uint32_t PATTERN_RUNS = 8;
+constexpr uint32_t PATTERN_CTAS = 8; // per SM
+
+// VEC_OUT: the output is aligned to a lane's bytes. APART: the selected elements lie 64 bytes and
+// more apart on average, so a load fetches 64 bytes rather than a line.
+template <typename T, bool VEC_OUT, bool APART>
 __global__ void __launch_bounds__(256) k_pattern(const T* __restrict__ in, T* __restrict__ out, uint32_t pattern,
                                                  uint32_t L, uint32_t P, uint64_t count, uint64_t* d_count)
 {
-    constexpr uint32_t VEC = 16 / sizeof(T);
+    constexpr uint32_t G = sizeof(T) < 4 ? 4 / sizeof(T) : 1; // elements per lane and run
+    constexpr uint32_t RUN = 32 * G;                          // outputs per run
+    constexpr uint32_t U = PATTERN_RUNS;
     __shared__ uint32_t s_pos[32];
+    // source offset of output i of P consecutive runs, from the period the first one starts
+    __shared__ __align__(8) uint16_t s_off[RUN * 32];
     if (threadIdx.x < 32) {
         const uint32_t b = threadIdx.x;
         if (b < L && ((pattern >> b) & 1u)) s_pos[__popc(pattern & ((1u << b) - 1u))] = b;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) *d_count = count;
     __syncthreads();
-    const uint64_t nvec = (count + VEC - 1) / VEC;
-    const uint64_t tid = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
-    // a thread takes UNR vectors stride apart per iteration, all their loads before any store;
-    constexpr uint32_t UNR = sizeof(T); // 16 elements per iteration at every width
-    const uint64_t dq1 = (stride * VEC) / P; // output-index step between a thread's vectors
-    const uint32_t dr1 = static_cast<uint32_t>((stride * VEC) % P);
-    uint64_t q = (tid * VEC) / P;
-    uint32_t r = static_cast<uint32_t>((tid * VEC) % P);
-    for (uint64_t v0 = tid; v0 < nvec; v0 += UNR * stride) {
-        union {
-            uint4 u;
-            T e[VEC];
-        } x[UNR];
-        uint64_t qk = q;
+    for (uint32_t i = threadIdx.x; i < RUN * P; i += 256) s_off[i] = static_cast<uint16_t>(i / P * L + s_pos[i % P]);
+    __syncthreads();
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint64_t warp_global = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    const uint64_t step = ((static_cast<uint64_t>(gridDim.x) * blockDim.x) >> 5) * U; // runs between a warp's groups
+    const uint64_t runs = (count + RUN - 1) / RUN;
+    const uint64_t dq = step / P;
+    const uint32_t dr = static_cast<uint32_t>(step % P);
+    const uint32_t period = RUN * L; // inputs of P runs
+    uint64_t q = warp_global * U / P;
+    uint32_t r = static_cast<uint32_t>(warp_global * U % P);
+    for (uint64_t s0 = warp_global * U; s0 < runs; s0 += step) {
+        T x[U][G];
+        const T* src = in + q * period;
         uint32_t rk = r;
+        const uint64_t j0 = s0 * RUN + lane * G; // this lane's first output
+        const bool whole = (s0 + U) * RUN <= count;
 #pragma unroll
-        for (uint32_t k = 0; k < UNR; ++k) {
-            const uint64_t j0 = (v0 + k * stride) * VEC;
-            uint64_t qq = qk;
-            uint32_t rr = rk;
+        for (uint32_t u = 0; u < U; ++u) {
+            uint16_t off[G];
+            if constexpr (G == 4) *reinterpret_cast<uint2*>(off) = *reinterpret_cast<const uint2*>(&s_off[rk * RUN + lane * G]);
+            else if constexpr (G == 2) *reinterpret_cast<uint32_t*>(off) = *reinterpret_cast<const uint32_t*>(&s_off[rk * RUN + lane * G]);
+            else off[0] = s_off[rk * RUN + lane];
 #pragma unroll
-            for (uint32_t e = 0; e < VEC; ++e) {
-                x[k].e[e] = j0 + e < count ? __ldg(in + qq * L + s_pos[rr]) : T(0);
-                if (++rr == P) {
-                    rr = 0;
-                    ++qq;
-                }
-            }
-            qk += dq1;
-            rk += dr1;
-            if (rk >= P) {
-                rk -= P;
-                ++qk;
+            for (uint32_t e = 0; e < G; ++e)
+                if (whole || j0 + u * RUN + e < count) x[u][e] = APART ? ldg_gather(src + off[e]) : __ldg(src + off[e]);
+            if (++rk == P) {
+                rk = 0;
+                src += period;
             }
         }
 #pragma unroll
-        for (uint32_t k = 0; k < UNR; ++k) {
-            const uint64_t j0 = (v0 + k * stride) * VEC;
-            if (j0 >= count) break;
-            if (VEC_OUT && j0 + VEC <= count) {
-                stg128_cs(out + j0, x[k].u);
+        for (uint32_t u = 0; u < U; ++u) {
+            T* dst = out + j0 + u * RUN;
+            if (VEC_OUT && G > 1 && (whole || j0 + u * RUN + G <= count)) {
+                uint32_t v;
+                if constexpr (G == 4) v = x[u][0] | x[u][1 % G] << 8 | x[u][2 % G] << 16 | static_cast<uint32_t>(x[u][3 % G]) << 24;
+                else v = static_cast<uint32_t>(x[u][0]) | static_cast<uint32_t>(x[u][1 % G]) << 16;
+                __stcs(reinterpret_cast<uint32_t*>(dst), v);
             } else {
 #pragma unroll
-                for (uint32_t e = 0; e < VEC; ++e)
-                    if (j0 + e < count) out[j0 + e] = x[k].e[e];
+                for (uint32_t e = 0; e < G; ++e)
+                    if (whole || j0 + u * RUN + e < count) __stcs(dst + e, x[u][e]);
             }
         }
-        q = qk; // the next iteration's first vector is UNR strides on
-        r = rk;
+        q += dq;
+        r += dr;
+        if (r >= P) {
+            r -= P;
+            ++q;
+        }
     }
 }
 
+// Dense patterns: items of 4 KB of payload per warp as in the 3-pass writeout (cs_writeout.cu),
+// with the mask bits and the positions from the pattern instead of a mask and a scan: element e
+// has rank (e / L) * P + the pattern's set bits below e % L. `rep`: the pattern repeated over 64
+// bits. The input 16-byte aligned.
+constexpr uint32_t DENSE_WARPS = 8;
+constexpr uint32_t DENSE_CTAS = 3;
+
+template <typename T, bool SWZ>
+__global__ void __launch_bounds__(DENSE_WARPS * 32, DENSE_CTAS)
+    k_pattern_dense(const uint8_t* __restrict__ in, uint8_t* __restrict__ out, uint64_t n, uint32_t pattern, uint64_t rep,
+                    uint32_t L, uint32_t P, uint64_t count, uint64_t* d_count)
+{
+    constexpr uint32_t EPL = LANE_BYTES / sizeof(T);
+    constexpr uint32_t ROW = 32 * EPL;
+    constexpr uint32_t ITEM = ROWS * ROW;
+    constexpr uint32_t VEC = 16 / sizeof(T);
+    constexpr uint32_t BITS = EPL == 32 ? 0xffffffffu : (1u << (EPL & 31u)) - 1u;
+    __shared__ __align__(128) uint8_t s_stage[DENSE_WARPS][STAGE_BYTES];
+    __shared__ uint32_t s_lut[sizeof(T) == 1 ? PACK_TABLE_WORDS : 1];
+    if constexpr (sizeof(T) == 1) {
+        fill_pack_table(s_lut, DENSE_WARPS * 32);
+        __syncthreads();
+    }
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t warp = threadIdx.x >> 5;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *d_count = count;
+    uint8_t* const stage = s_stage[warp];
+    const uint32_t stage_a = smem_u32(stage);
+    const uint32_t lut = sizeof(T) == 1 ? smem_u32(s_lut) + lane * 4 : 0u;
+    const bool in32 = (reinterpret_cast<uintptr_t>(in) & 31u) == 0;
+    const uint64_t total_warps = static_cast<uint64_t>(gridDim.x) * DENSE_WARPS;
+    const uint64_t step = total_warps * ITEM;
+    uint64_t e0 = (static_cast<uint64_t>(blockIdx.x) * DENSE_WARPS + warp) * ITEM;
+    // the period and the place within it of this lane's first element; both advance without
+    // further divisions
+    const uint64_t dq = step / L;
+    const uint32_t dr = static_cast<uint32_t>(step % L);
+    uint64_t q = (e0 + lane * EPL) / L;
+    uint32_t r = static_cast<uint32_t>((e0 + lane * EPL) % L);
+    const uint32_t row_q = ROW / L, row_r = ROW % L;
+    for (; e0 < n; e0 += step) {
+        const bool whole = e0 + ITEM <= n;
+        const uint8_t* src = in + e0 * sizeof(T) + lane * LANE_BYTES;
+        uint32_t bits[ROWS], rank[ROWS], x[ROWS][8];
+        uint32_t rk = r, qk = static_cast<uint32_t>(q); // ranks within an item fit 32 bits
+#pragma unroll
+        for (uint32_t k = 0; k < ROWS; ++k) {
+            uint32_t b = __funnelshift_r(static_cast<uint32_t>(rep), static_cast<uint32_t>(rep >> 32), rk) & BITS;
+            const uint64_t e = e0 + k * ROW + lane * EPL;
+            if (!whole && e + EPL > n) b &= e < n ? (1u << (n - e)) - 1u : 0u;
+            bits[k] = b;
+            rank[k] = qk * P + __popc(pattern & ((1u << rk) - 1u));
+            if (b) {
+                if (whole || e + EPL <= n) {
+                    if (in32) ldg256(src + k * ROW_BYTES, x[k]);
+                    else ldg128x2(src + k * ROW_BYTES, x[k]);
+                } else {
+                    // the lane in which the column ends: element by element, through the idle stage
+                    const T* last = reinterpret_cast<const T*>(in) + e;
+                    T* tmp = reinterpret_cast<T*>(stage + lane * LANE_BYTES);
+                    for (uint32_t i = 0; e + i < n; ++i) tmp[i] = __ldg(last + i);
+#pragma unroll
+                    for (uint32_t w = 0; w < 8; ++w) x[k][w] = lds32(stage_a + lane * LANE_BYTES + 4 * w);
+                }
+            }
+            qk += row_q;
+            rk += row_r;
+            if (rk >= L) {
+                rk -= L;
+                ++qk;
+            }
+        }
+        const uint64_t off = __shfl_sync(0xffffffffu, q * P + __popc(pattern & ((1u << r) - 1u)), 0); // rank of e0
+        const uint32_t a = static_cast<uint32_t>((reinterpret_cast<uintptr_t>(out) / sizeof(T) + off) % VEC);
+        const uint32_t end = __shfl_sync(0xffffffffu, rank[ROWS - 1] + __popc(bits[ROWS - 1]), 31);
+        const uint32_t run = a + (whole ? end - static_cast<uint32_t>(off) : static_cast<uint32_t>(count - off));
+        __syncwarp(); // the ragged lane has read its place in the stage
+        Tail tail[ROWS];
+#pragma unroll
+        for (uint32_t k = 0; k < ROWS; ++k)
+            tail[k] = place_row<T, SWZ>(x[k], bits[k],
+                                        stage_a + (rank[k] - static_cast<uint32_t>(off) + a) * static_cast<uint32_t>(sizeof(T)), lut);
+        if constexpr (sizeof(T) == 1) {
+            __syncwarp(); // every whole word is in the stage before the partial ones
+#pragma unroll
+            for (uint32_t k = 0; k < ROWS; ++k) place_tail(tail[k]);
+        }
+        __syncwarp();
+        emit_stage<T>(out + (static_cast<int64_t>(off) - static_cast<int64_t>(a)) * static_cast<int64_t>(sizeof(T)), stage, a,
+                      run, lane, SWZ ? 0x70u : 0u);
+        __syncwarp(); // the stage is rewritten by the next item
+        q += dq;
+        r += dr;
+        if (r >= L) {
+            r -= L;
+            ++q;
+        }
+    }
+}
+
+// Which kernel a pattern takes. The gather's time follows the outputs, the dense kernel's the inputs.
+// Per call on B200, n = 2^28 (2^27 for 8 bytes), gather / dense, us, by selected share P / L:
+//           0.25       0.33       0.375      0.43       0.5        0.75       0.97
+//   1 byte  67 / 75    - / 78     108 / 76   119 / 80   136 / 78   - / 80     257 / 88
+//   2       105 / 110  120 / 147  147 / 118  162 / 131  175 / 145  - / 159    333 / 172
+//   4       201 / 202  214 / 230  233 / 217  250 / 230  266 / 245  318 / 288  371 / 322
+//   8       196 / 196  209 / 214  230 / 215  241 / 230  252 / 242  306 / 282  349 / 325
+// (dense at the better of 2 and 3 CTAs per SM; one thread per 16 output bytes, which both replace:
+// 1 byte 131 .. 156 .. 297, 2 bytes 158 .. 164 .. 318, 4 bytes 213 .. 256 .. 438).
+bool dense_pattern(uint32_t w, uint32_t L, uint32_t P)
+{
+    return P * 100 >= L * (w == 1 || w == 8 ? 30u : 36u);
+}
+
+// CTAs of the dense kernel per SM. 3 keep enough loads in flight for what is mostly read; where as
+// much is written, 2 disturb the memory less: 4 bytes 0.375 217 (3) / 249 (2), 0.5 272 / 245, 0.97
+// 364 / 322; 8 bytes 0.375 215 / 239, 0.5 273 / 250, 0.97 369 / 325. The 1- and 2-byte forms are
+// held back by their instructions: 1 byte 0.97 88 / 100, 2 bytes 0.67 151 / 170, 0.97 188 / 172.
+uint32_t dense_ctas_per_sm(uint32_t w, uint32_t L, uint32_t P)
+{
+    if (w == 1) return DENSE_CTAS;
+    return P * 100 >= L * (w == 2 ? 85u : 45u) ? 2u : DENSE_CTAS;
+}
+
 template <typename T>
-cudaError_t launch_t(const void* in, void* out, uint32_t pattern, uint32_t L, uint32_t P, uint64_t count,
+cudaError_t launch_t(const void* in, void* out, uint64_t n, uint32_t pattern, uint32_t L, uint32_t P, uint64_t count,
                      uint64_t* d_count, int sms, cudaStream_t s)
 {
-    constexpr uint64_t VEC = 16 / sizeof(T);
-    const uint64_t nvec = (count + VEC - 1) / VEC;
-    uint64_t blocks = (nvec + 255) / 256;
-    const uint64_t cap = static_cast<uint64_t>(sms) * 8;
+    constexpr uint64_t GROUP = 8 * PATTERN_RUNS * 32 * (sizeof(T) < 4 ? 4 / sizeof(T) : 1); // outputs per CTA and iteration
+    uint64_t blocks = (count + GROUP - 1) / GROUP;
+    const uint64_t cap = static_cast<uint64_t>(sms) * PATTERN_CTAS;
     if (blocks > cap) blocks = cap;
     if (blocks == 0) blocks = 1;
-    const bool vec = (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
+    const bool vec = (reinterpret_cast<uintptr_t>(out) & 3u) == 0;
+    const bool apart = sizeof(T) * L >= 64 * P;
+    if (dense_pattern(sizeof(T), L, P) && (reinterpret_cast<uintptr_t>(in) & 15u) == 0) {
+        uint64_t rep = 0;
+        for (uint32_t i = 0; i < 64; ++i) rep |= static_cast<uint64_t>((pattern >> (i % L)) & 1u) << i;
+        const uint64_t items = (n * sizeof(T) + ITEM_BYTES - 1) / ITEM_BYTES;
+        uint64_t ctas = (items + DENSE_WARPS - 1) / DENSE_WARPS;
+        const uint64_t most = static_cast<uint64_t>(sms) * dense_ctas_per_sm(sizeof(T), L, P);
+        if (ctas > most) ctas = most;
+        // With an even number per period the lanes' elements fall into step on few banks, unless the
+        // period divides a lane's elements (us, plain / swizzled stage: 2 bytes, 2 of 3 237 / 142, 2 of 5
+        // 169 / 135, 3 of 7 131 / 139; 4 bytes, 2 of 5 249 / 226, 4 of 8 256 / 270)
+        constexpr bool CAN = sizeof(T) == 2 || sizeof(T) == 4;
+        const auto kernel = CAN && P % 2 == 0 && (L & (L - 1)) != 0 ? k_pattern_dense<T, CAN> : k_pattern_dense<T, false>;
+        kernel<<<static_cast<unsigned>(ctas), DENSE_WARPS * 32, 0, s>>>(static_cast<const uint8_t*>(in),
+                                                                        static_cast<uint8_t*>(out), n, pattern, rep, L, P,
+                                                                        count, d_count);
+        note_launch();
+        return cudaGetLastError();
+    }
     const T* ti = static_cast<const T*>(in);
     T* to = static_cast<T*>(out);
-    if (vec)
-        k_pattern<T, true><<<static_cast<unsigned>(blocks), 256, 0, s>>>(ti, to, pattern, L, P, count, d_count);
-    else
-        k_pattern<T, false><<<static_cast<unsigned>(blocks), 256, 0, s>>>(ti, to, pattern, L, P, count, d_count);
+    const unsigned g = static_cast<unsigned>(blocks);
+    if (vec && apart) k_pattern<T, true, true><<<g, 256, 0, s>>>(ti, to, pattern, L, P, count, d_count);
+    else if (vec) k_pattern<T, true, false><<<g, 256, 0, s>>>(ti, to, pattern, L, P, count, d_count);
+    else if (apart) k_pattern<T, false, true><<<g, 256, 0, s>>>(ti, to, pattern, L, P, count, d_count);
+    else k_pattern<T, false, false><<<g, 256, 0, s>>>(ti, to, pattern, L, P, count, d_count);
     note_launch();
     return cudaGetLastError();
 }
@@ -149,10 +310,10 @@ int compressstore_pattern(const void* d_in, void* d_out, uint64_t n, uint32_t el
     const uint32_t P = static_cast<uint32_t>(__builtin_popcount(pm));
     cudaError_t e;
     switch (elem_bytes) {
-        case 1: e = launch_t<uint8_t>(d_in, d_out, pm, pattern_length, P, count, d_count, sms, s); break;
-        case 2: e = launch_t<uint16_t>(d_in, d_out, pm, pattern_length, P, count, d_count, sms, s); break;
-        case 4: e = launch_t<uint32_t>(d_in, d_out, pm, pattern_length, P, count, d_count, sms, s); break;
-        default: e = launch_t<uint64_t>(d_in, d_out, pm, pattern_length, P, count, d_count, sms, s); break;
+        case 1: e = launch_t<uint8_t>(d_in, d_out, n, pm, pattern_length, P, count, d_count, sms, s); break;
+        case 2: e = launch_t<uint16_t>(d_in, d_out, n, pm, pattern_length, P, count, d_count, sms, s); break;
+        case 4: e = launch_t<uint32_t>(d_in, d_out, n, pm, pattern_length, P, count, d_count, sms, s); break;
+        default: e = launch_t<uint64_t>(d_in, d_out, n, pm, pattern_length, P, count, d_count, sms, s); break;
     }
     return e == cudaSuccess ? CS_SUCCESS : (e == cudaErrorMemoryAllocation ? CS_ERR_OUT_OF_MEMORY : CS_ERR_CUDA);
 }

@@ -47,16 +47,12 @@
 #include <cuda_runtime.h>
 
 #include "cs_internal.cuh"
+#include "cs_place.cuh"
 
 namespace cs {
 
 namespace {
 
-constexpr uint32_t ROWS = 4;                              // 32-byte loads per lane and item
-constexpr uint32_t LANE_BYTES = 32;                       // payload bytes per lane and row
-constexpr uint32_t ROW_BYTES = 32 * LANE_BYTES;
-constexpr uint32_t ITEM_BYTES = ROWS * ROW_BYTES;         // 4 KB
-constexpr uint32_t STAGE_BYTES = ITEM_BYTES + 32;         // selected elements from any 16-byte phase
 constexpr uint32_t SPARSE_LIST = 1024;                    // indices of one gather round (in the stage)
 constexpr uint32_t SPARSE_INFLIGHT = 4;                   // payload loads per lane in flight
 static_assert(SPARSE_LIST * 2 <= STAGE_BYTES, "the list lies in the stage");
@@ -69,20 +65,6 @@ static_assert(SPARSE_LIST * 2 <= STAGE_BYTES, "the list lies in the stage");
 constexpr uint32_t WARPS = 8;
 template <bool SHIFT>
 constexpr uint32_t CTAS = SHIFT ? 2 : 3;
-
-__device__ __forceinline__ void ldg256(const void* p, uint32_t (&x)[8])
-{
-    asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]), "=r"(x[4]), "=r"(x[5]), "=r"(x[6]), "=r"(x[7])
-                 : "l"(p));
-}
-
-__device__ __forceinline__ void ldg128x2(const void* p, uint32_t (&x)[8])
-{
-    const uint4 a = __ldg(static_cast<const uint4*>(p)), b = __ldg(static_cast<const uint4*>(p) + 1);
-    x[0] = a.x, x[1] = a.y, x[2] = a.z, x[3] = a.w;
-    x[4] = b.x, x[5] = b.y, x[6] = b.z, x[7] = b.w;
-}
 
 // 32 bytes from an address `d` bytes (1 .. 15, the same for the whole column) past a 16-byte
 // boundary, out of the three 16-byte vectors that hold them.
@@ -100,102 +82,6 @@ __device__ __forceinline__ void ldg_shifted(const uint8_t* p, uint32_t d, uint32
         else if (d >= 4u) lo = w[i + 1], hi = w[i + 2];
         x[i] = __funnelshift_r(lo, hi, s);
     }
-}
-
-__device__ __forceinline__ void sts32(uint32_t a, uint32_t v)
-{
-    asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
-}
-__device__ __forceinline__ void sts64(uint32_t a, uint32_t lo, uint32_t hi)
-{
-    asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(a), "r"(lo), "r"(hi) : "memory");
-}
-__device__ __forceinline__ void sts8(uint32_t a, uint32_t v)
-{
-    asm volatile("st.shared.u8 [%0], %1;" ::"r"(a), "r"(v) : "memory");
-}
-__device__ __forceinline__ void sts16(uint32_t a, uint32_t v)
-{
-    asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "h"(static_cast<uint16_t>(v)) : "memory");
-}
-__device__ __forceinline__ uint32_t lds32(uint32_t a)
-{
-    uint32_t v;
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
-    return v;
-}
-
-// What a lane's run of 1-byte elements leaves past its last whole word: `f8` bits of acc, of
-// which the lowest lo8 are earlier lanes'.
-struct Tail {
-    uint32_t acc, at, f8, lo8;
-};
-
-// One lane's row (32 payload bytes in x, `bits` selecting from them) to the stage address `at`.
-template <typename T>
-__device__ __forceinline__ Tail place_row(const uint32_t (&x)[8], uint32_t bits, uint32_t at, uint32_t lut)
-{
-    Tail t{0u, at, 0u, 0u};
-    if constexpr (sizeof(T) == 8) {
-#pragma unroll
-        for (uint32_t e = 0; e < 4; ++e)
-            if ((bits >> e) & 1u) {
-                sts64(at, x[2 * e], x[2 * e + 1]);
-                at += 8;
-            }
-    } else if constexpr (sizeof(T) == 4) {
-#pragma unroll
-        for (uint32_t e = 0; e < 8; ++e)
-            if ((bits >> e) & 1u) {
-                sts32(at, x[e]);
-                at += 4;
-            }
-    } else if constexpr (sizeof(T) == 2) {
-#pragma unroll
-        for (uint32_t e = 0; e < 16; ++e)
-            if ((bits >> e) & 1u) {
-                sts16(at, e & 1u ? x[e / 2] >> 16 : x[e / 2]);
-                at += 2;
-            }
-    } else {
-        // `fill`: bits placed so far, from the start of the run's first word; a word is complete
-        // when bit 5 of it changes (shifts take it modulo 32)
-        uint32_t fill = at * 8u;
-        const uint32_t word0 = fill >> 5;
-        t.lo8 = fill & 31u;
-        at &= ~3u;
-        uint32_t acc = 0;
-#pragma unroll
-        for (uint32_t k = 0; k < 8; ++k) {
-            // the table's entry of 4 mask bits: byte selectors that pack the selected bytes (low
-            // 16 bits; 4 selects a zero), 8 x their number (high 16 bits)
-            const uint32_t ent = lds32(lut + ((k < 2 ? bits << (7 - 4 * k) : bits >> (4 * k - 7)) & 0x780u));
-            const uint32_t pk = __byte_perm(x[k], 0u, ent);
-            const uint32_t next = fill + (ent >> 16);
-            const uint32_t w0 = acc | __funnelshift_l(0u, pk, fill);
-            const uint32_t w1 = __funnelshift_l(pk, 0u, fill);
-            if ((next ^ fill) & 32u) {
-                sts32(at, w0);
-                at += 4;
-                acc = w1;
-            } else {
-                acc = w0;
-            }
-            fill = next;
-        }
-        if ((fill >> 5) != word0) t.lo8 = 0;
-        t.acc = acc;
-        t.at = at;
-        t.f8 = fill & 31u;
-    }
-    return t;
-}
-
-__device__ __forceinline__ void place_tail(const Tail& t)
-{
-#pragma unroll
-    for (uint32_t b = 0; b < 3; ++b)
-        if (b * 8 >= t.lo8 && b * 8 < t.f8) sts8(t.at + b, t.acc >> (8 * b));
 }
 
 // GROUPS 4096-element groups of a sparse unit of column c, from element e0.
@@ -296,23 +182,12 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS<SHIFT>) k_writeout_warp(const
     constexpr uint32_t IPU = UE / ITEM; // items per unit
     constexpr uint32_t VEC = 16 / sizeof(T);
     constexpr uint32_t NONE = 0xffffffffu;
-    __shared__ __align__(16) uint8_t s_stage[WARPS][STAGE_BYTES];
-    __shared__ uint32_t s_lut[sizeof(T) == 1 ? 16 * 32 : 1];
+    __shared__ __align__(128) uint8_t s_stage[WARPS][STAGE_BYTES];
+    __shared__ uint32_t s_lut[sizeof(T) == 1 ? PACK_TABLE_WORDS : 1];
     __shared__ uint32_t s_hflags;
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t warp = threadIdx.x >> 5;
-    if constexpr (sizeof(T) == 1) {
-        for (uint32_t i = threadIdx.x; i < 16 * 32; i += WARPS * 32) {
-            const uint32_t nib = i >> 5;
-            uint32_t sel = 0x4444u, k = 0;
-            for (uint32_t b = 0; b < 4; ++b)
-                if ((nib >> b) & 1u) {
-                    sel = (sel & ~(0xfu << (4 * k))) | (b << (4 * k));
-                    ++k;
-                }
-            s_lut[i] = sel | (k << 19);
-        }
-    }
+    if constexpr (sizeof(T) == 1) fill_pack_table(s_lut, WARPS * 32);
     grid_dependency_wait(); // offsets and counts of pass 2
     const uint32_t hflags = cta_header_flags(p.hdr, &s_hflags); // a barrier: the table is filled
     if (!(hflags & 1u)) return; // pass 2 offsets not trustworthy: write nothing
@@ -461,24 +336,15 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS<SHIFT>) k_writeout_warp(const
         Tail tail[ROWS];
 #pragma unroll
         for (uint32_t r = 0; r < ROWS; ++r)
-            tail[r] = place_row<T>(x[r], bits[r], stage_a + pos[r] * static_cast<uint32_t>(sizeof(T)), lut);
+            tail[r] = place_row<T, false>(x[r], bits[r], stage_a + pos[r] * static_cast<uint32_t>(sizeof(T)), lut);
         if constexpr (sizeof(T) == 1) {
             __syncwarp(); // every whole word is in the stage before the partial ones
 #pragma unroll
             for (uint32_t r = 0; r < ROWS; ++r) place_tail(tail[r]);
         }
         __syncwarp();
-        // the stage leaves as whole 16-byte vectors, and its ragged ends element by element
-        // (lanes 0-15 the head, lanes 16-31 the tail)
-        uint8_t* gdst = C.out + (static_cast<int64_t>(off) - static_cast<int64_t>(a)) * static_cast<int64_t>(sizeof(T));
-        const uint32_t v0 = a ? 1u : 0u, v1 = run / VEC;
-        for (uint32_t v = v0 + lane; v < v1; v += 32) stg128_cs(gdst + v * 16u, lds128(stage + v * 16u));
-        const uint32_t i = lane & 15u;
-        if (i < VEC) {
-            const uint32_t e = lane & 16u ? v1 * VEC + i : i;
-            const bool st = lane & 16u ? v1 >= v0 && e < run : a != 0u && e >= a && e < run;
-            if (st) reinterpret_cast<T*>(gdst)[e] = reinterpret_cast<const T*>(stage)[e];
-        }
+        emit_stage<T>(C.out + (static_cast<int64_t>(off) - static_cast<int64_t>(a)) * static_cast<int64_t>(sizeof(T)), stage,
+                      a, run, lane, 0u);
         __syncwarp(); // the stage is rewritten by the next item
     }
 
