@@ -68,6 +68,17 @@ constexpr uint32_t CTAS = SHIFT ? 2 : 3;
 
 // 32 bytes from an address `d` bytes (1 .. 15, the same for the whole column) past a 16-byte
 // boundary, out of the three 16-byte vectors that hold them.
+// Warps of a CTA that stay idle for a long column of which most, but not nearly all, is selected:
+// there the loads in flight of 24 warps per SM hold up the writes. 3-pass call on B200, us, 24 / 21 /
+// 18 warps: 2^27 u64 p = 0.7 298 / 295 / 309, 0.8 348 / 333 / 314, 0.9 360 / 345 / 335, 0.99 354 / 351 /
+// 354; 2^28 u32 p = 0.7 303 / 310 / 331, 0.8 339 / 326 / 334, 0.9 357 / 340 / 355, 0.99 374 / 373 / 381;
+// 2^26 u32 p = 0.9 102 / 94 / 94, but 2^24 29.6 / 30.6 / 31.7 (few items per warp). Narrower elements
+// are held back by their instructions: 2^28 u16 p = 0.9 185 / 198 / 200.
+template <typename T>
+constexpr uint32_t throttle_warps = sizeof(T) == 8 ? 2 : sizeof(T) == 4 ? 1 : 0;
+template <typename T>
+constexpr uint32_t throttle_percent = sizeof(T) == 8 ? 75 : 85; // from this share selected on, up to 97%
+
 __device__ __forceinline__ void ldg_shifted(const uint8_t* p, uint32_t d, uint32_t (&x)[8])
 {
     const uint4* q = reinterpret_cast<const uint4*>(p - d);
@@ -196,8 +207,15 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS<SHIFT>) k_writeout_warp(const
     const uint32_t stage_a = smem_u32(stage);
     const uint32_t lut = sizeof(T) == 1 ? smem_u32(s_lut) + lane * 4 : 0u;
     const uint32_t num_items = static_cast<uint32_t>(p.num_units) * IPU; // below 2^32 for every column the library takes
-    const uint32_t warp_global = blockIdx.x * WARPS + warp;
-    const uint32_t total_warps = gridDim.x * WARPS;
+    // a long column of mostly selected elements runs better with fewer warps (throttle_warps)
+    uint32_t active = WARPS;
+    const uint64_t percent = p.throttle != 0u ? *p.col0.d_count * 100 / p.col0.n : 0u;
+    if (percent >= throttle_percent<T> && percent < 97u) {
+        active = WARPS - p.throttle;
+        if (warp >= active) return;
+    }
+    const uint32_t warp_global = blockIdx.x * active + warp;
+    const uint32_t total_warps = gridDim.x * active;
 
     auto column = [&](uint32_t it) -> const ColumnDesc& {
         return MULTI ? p.cols[__ldg(p.unit_col + it / IPU)] : p.col0;
@@ -333,10 +351,21 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS<SHIFT>) k_writeout_warp(const
             continue;
         }
         __syncwarp(); // the ragged lanes have read their places in the stage
+        uint32_t swz = 0u;
         Tail tail[ROWS];
+        if ((sizeof(T) == 2 || sizeof(T) == 4) && run - a > ITEM / 16 * 15) {
+            // nearly all of the item is selected: the lanes' elements lie 8 words apart (2^28 u32 runs of
+            // 4096 262 -> 239 us, 2^28 u16 205 -> 170, p = 0.99 247 -> 204; with every item 2^28 u16
+            // p = 0.5 151 -> 162)
+            swz = 0x70u;
 #pragma unroll
-        for (uint32_t r = 0; r < ROWS; ++r)
-            tail[r] = place_row<T, false>(x[r], bits[r], stage_a + pos[r] * static_cast<uint32_t>(sizeof(T)), lut);
+            for (uint32_t r = 0; r < ROWS; ++r)
+                place_row<T, (sizeof(T) > 1)>(x[r], bits[r], stage_a + pos[r] * static_cast<uint32_t>(sizeof(T)), lut);
+        } else {
+#pragma unroll
+            for (uint32_t r = 0; r < ROWS; ++r)
+                tail[r] = place_row<T, false>(x[r], bits[r], stage_a + pos[r] * static_cast<uint32_t>(sizeof(T)), lut);
+        }
         if constexpr (sizeof(T) == 1) {
             __syncwarp(); // every whole word is in the stage before the partial ones
 #pragma unroll
@@ -344,7 +373,7 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS<SHIFT>) k_writeout_warp(const
         }
         __syncwarp();
         emit_stage<T>(C.out + (static_cast<int64_t>(off) - static_cast<int64_t>(a)) * static_cast<int64_t>(sizeof(T)), stage,
-                      a, run, lane, 0u);
+                      a, run, lane, swz);
         __syncwarp(); // the stage is rewritten by the next item
     }
 
@@ -381,11 +410,13 @@ cudaError_t launch_t(const WriteoutParams& p, uint32_t requested, int num_sms, c
     const uint64_t cap = requested ? requested : static_cast<uint64_t>(num_sms) * CTAS<SHIFT>; // one resident wave
     if (blocks > cap) blocks = cap;
     if (blocks == 0) blocks = 1;
+    WriteoutParams pp = p;
+    pp.throttle = !p.cols && p.col0.d_count && items >= 8 * blocks * WARPS ? throttle_warps<T> : 0u;
     const dim3 g(static_cast<unsigned>(blocks)), b(WARPS * 32);
     cudaError_t e;
-    if constexpr (SHIFT) e = launch_pdl(k_writeout_warp<T, false, true>, g, b, 0, stream, p);
-    else e = p.cols ? launch_pdl(k_writeout_warp<T, true, false>, g, b, 0, stream, p)
-                    : launch_pdl(k_writeout_warp<T, false, false>, g, b, 0, stream, p);
+    if constexpr (SHIFT) e = launch_pdl(k_writeout_warp<T, false, true>, g, b, 0, stream, pp);
+    else e = p.cols ? launch_pdl(k_writeout_warp<T, true, false>, g, b, 0, stream, pp)
+                    : launch_pdl(k_writeout_warp<T, false, false>, g, b, 0, stream, pp);
     note_launch();
     return e;
 }

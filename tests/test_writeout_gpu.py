@@ -69,3 +69,19 @@ def test_unaligned_pointers(cuda, oracle, w):
             assert np.array_equal(out[out_off:out_off + k], exp), what
             rest = np.concatenate([out[:out_off], out[out_off + k:]]).view(np.uint8)
             assert np.all(rest == 0xAB), what
+
+
+@pytest.mark.parametrize("w", [1, 2, 4, 8])
+def test_long_dense_column(cuda, oracle, w):
+    """Many items per warp with 7 of 8 elements selected (the throttled grid of 4 and 8 bytes), a
+    stretch of full words (the swizzled stage) and an empty one."""
+    n = (8 * 148 * 3 * 8 * ITEM + 3 * UNIT) // w + 77
+    rng = np.random.default_rng(w)
+    words = (n + 31) // 32
+    mask = np.zeros(words, np.uint32)
+    for _ in range(3):
+        mask |= rng.integers(0, 1 << 32, size=words, dtype=np.uint64).astype(np.uint32)
+    mask[words // 3:words // 3 + words // 20] = 0xFFFFFFFF
+    mask[words // 2:words // 2 + 3000] = 0
+    payload = rng.integers(0, 256, size=n * w, dtype=np.uint8).view(UNSIGNED[w])
+    check_against_oracle(oracle, payload, mask, n, "3pass", chunk_length=4096 // w)
