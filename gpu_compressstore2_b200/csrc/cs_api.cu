@@ -3,10 +3,12 @@
 // generator / pass entry points.
 #include <atomic>
 #include <cstdint>
-#include <limits>
+#include <cmath>
 #include <cstring>
+#include <limits>
 #include <map>
 #include <mutex>
+#include <type_traits>
 #include <utility>
 
 #include <cuda_runtime.h>
@@ -96,14 +98,13 @@ struct Layout {
     size_t off_counts = 0;
     size_t off_offsets = 0;
     size_t off_blk_base = 0;  // per-2^18-element block prefixes of the reduce-then-scan pass
-    size_t off_mask = 0;      // predicate compaction: the selection mask it writes (0: none)
     size_t off_item_flags = 0; // sparse items of the hybrid writeout, marked by pass 1
     size_t off_flags = 0;     // pass 1's per-CTA sparse flags
     size_t total = 0;
 };
 
 // All regions every algorithm may need, so AUTO may switch algorithm freely.
-Layout plan_layout(uint64_t n, uint32_t elem_bytes, uint32_t chunk_log2, bool with_mask = false)
+Layout plan_layout(uint64_t n, uint32_t elem_bytes, uint32_t chunk_log2)
 {
     Layout l;
     const uint64_t ue = unit_elems_for(elem_bytes);
@@ -129,10 +130,6 @@ Layout plan_layout(uint64_t n, uint32_t elem_bytes, uint32_t chunk_log2, bool wi
     // inside the range the epoch-wrap clear keeps: later kernels of the call read these
     l.off_item_flags = off;
     off += align256(4 * sparse_items_for(n));
-    if (with_mask) {
-        l.off_mask = off;
-        off += align256(4 * ((n + 31) / 32));
-    }
     l.off_flags = off;
     off += align256(4 * POPC_FLAG_SLOTS);
     l.total = align256(off);
@@ -423,50 +420,76 @@ int check_workspace_error(void* d_ws, cudaStream_t stream)
     return err == DEVERR_RANGE ? CS_ERR_INVALID_VALUE : CS_ERR_TIMEOUT;
 }
 
-// The predicate as lo (<|<=) x (<|<=) hi, negated for NE; bounds as bit patterns of T.
+// The predicate as lo <= x <= hi, negated for NE (and for a selection of nothing): inclusive bounds
+// of whole numbers, hi as the distance from lo; of floating numbers the neighbouring values.
 template <typename T>
-void predicate_bounds_t(const cs_predicate& pr, PredParams& pp)
+void predicate_bounds_t(const cs_predicate& pr, IfParams& p)
 {
+    constexpr bool REAL = std::numeric_limits<T>::has_infinity;
     T a, b;
     std::memcpy(&a, &pr.a, sizeof(T));
     std::memcpy(&b, &pr.b, sizeof(T));
-    const T lowest = std::numeric_limits<T>::has_infinity ? -std::numeric_limits<T>::infinity()
-                                                          : std::numeric_limits<T>::lowest();
-    const T highest = std::numeric_limits<T>::has_infinity ? std::numeric_limits<T>::infinity()
-                                                           : std::numeric_limits<T>::max();
+    const T lowest = REAL ? -std::numeric_limits<T>::infinity() : std::numeric_limits<T>::lowest();
+    const T highest = REAL ? std::numeric_limits<T>::infinity() : std::numeric_limits<T>::max();
     T lo = lowest, hi = highest;
-    bool li = true, hi_i = true, neg = false;
+    bool none = false, neg = false;
+    // the largest value below a, the smallest above it
+    auto below = [&]() -> T {
+        if constexpr (REAL) return std::nextafter(a, lowest);
+        else return static_cast<T>(a - 1);
+    };
+    auto above = [&]() -> T {
+        if constexpr (REAL) return std::nextafter(a, highest);
+        else return static_cast<T>(a + 1);
+    };
     switch (pr.op) {
-        case CS_PRED_LT: hi = a; hi_i = false; break;
-        case CS_PRED_LE: hi = a; break;
-        case CS_PRED_GT: lo = a; li = false; break;
+        case CS_PRED_LT:
+            none = !(a > lowest); // a NaN too
+            if (!none) hi = below();
+            break;
+        case CS_PRED_LE: hi = a; break; // a NaN compares false
+        case CS_PRED_GT:
+            none = !(a < highest);
+            if (!none) lo = above();
+            break;
         case CS_PRED_GE: lo = a; break;
         case CS_PRED_EQ: lo = hi = a; break;
         case CS_PRED_NE: lo = hi = a; neg = true; break;
-        default: lo = a; hi = b; break; // CS_PRED_BETWEEN
+        default: // CS_PRED_BETWEEN
+            lo = a;
+            hi = b;
+            none = !(lo <= hi);
+            break;
     }
-    pp.lo = pp.hi = 0;
-    std::memcpy(&pp.lo, &lo, sizeof(T));
-    std::memcpy(&pp.hi, &hi, sizeof(T));
-    pp.lo_incl = li;
-    pp.hi_incl = hi_i;
-    pp.negate = neg;
+    if constexpr (REAL) {
+        if (none) lo = highest, hi = lowest;
+    } else {
+        if (none) lo = lowest, hi = highest, neg = true;
+        using U = typename std::make_unsigned<T>::type;
+        const U rng = static_cast<U>(static_cast<U>(hi) - static_cast<U>(lo));
+        std::memcpy(&hi, &rng, sizeof(T));
+    }
+    p.lo = p.hi = 0;
+    std::memcpy(&p.lo, &lo, sizeof(T));
+    std::memcpy(&p.hi, &hi, sizeof(T));
+    p.negate = neg;
+    p.sides = none ? 3u : pr.op == CS_PRED_GT || pr.op == CS_PRED_GE ? 1u : pr.op == CS_PRED_LT || pr.op == CS_PRED_LE ? 2u : 3u;
 }
 
 // Element width of a cs_elem_type and its bounds; 0 for an unknown type.
-uint32_t predicate_bounds(const cs_predicate& pr, PredParams& pp)
+uint32_t predicate_bounds(const cs_predicate& pr, IfParams& p)
 {
     switch (pr.type) {
-        case CS_U8: predicate_bounds_t<uint8_t>(pr, pp); return 1;
-        case CS_U16: predicate_bounds_t<uint16_t>(pr, pp); return 2;
-        case CS_U32: predicate_bounds_t<uint32_t>(pr, pp); return 4;
-        case CS_U64: predicate_bounds_t<uint64_t>(pr, pp); return 8;
-        case CS_I8: predicate_bounds_t<int8_t>(pr, pp); return 1;
-        case CS_I16: predicate_bounds_t<int16_t>(pr, pp); return 2;
-        case CS_I32: predicate_bounds_t<int32_t>(pr, pp); return 4;
-        case CS_I64: predicate_bounds_t<int64_t>(pr, pp); return 8;
-        case CS_F32: predicate_bounds_t<float>(pr, pp); return 4;
-        case CS_F64: predicate_bounds_t<double>(pr, pp); return 8;
+        case CS_U8: predicate_bounds_t<uint8_t>(pr, p); return 1;
+        case CS_U16: predicate_bounds_t<uint16_t>(pr, p); return 2;
+        case CS_U32: predicate_bounds_t<uint32_t>(pr, p); return 4;
+        case CS_U64: predicate_bounds_t<uint64_t>(pr, p); return 8;
+        case CS_I8: predicate_bounds_t<int8_t>(pr, p); return 1;
+        case CS_I16: predicate_bounds_t<int16_t>(pr, p); return 2;
+        case CS_I32: predicate_bounds_t<int32_t>(pr, p); return 4;
+        case CS_I64: predicate_bounds_t<int64_t>(pr, p); return 8;
+        case CS_F32: predicate_bounds_t<float>(pr, p); return 4;
+        case CS_F64: predicate_bounds_t<double>(pr, p); return 8;
         default: return 0;
     }
 }
@@ -540,8 +563,8 @@ int compressstore_if(const void* d_in, void* d_out, uint64_t n, const cs_predica
 {
     if (!pred || !d_count) return CS_ERR_INVALID_VALUE;
     if (pred->op < CS_PRED_LT || pred->op > CS_PRED_BETWEEN) return CS_ERR_INVALID_VALUE;
-    PredParams pp{};
-    const uint32_t w = predicate_bounds(*pred, pp);
+    IfParams p{};
+    const uint32_t w = predicate_bounds(*pred, p);
     if (w == 0) return CS_ERR_INVALID_VALUE;
     if (n > MAX_N) return CS_ERR_NOT_SUPPORTED;
     if (!aligned(d_count, 8)) return CS_ERR_MISALIGNED;
@@ -552,40 +575,20 @@ int compressstore_if(const void* d_in, void* d_out, uint64_t n, const cs_predica
     DeviceInfo di;
     int st = current_device_info(&di);
     if (st) return st;
-    Resolved r{};
-    r.algo = CS_ALGO_3PASS;
-    r.chunk_log2 = 12 - ilog2(w); // a chunk per item of the writeout (4 KB of payload)
-    r.grid = 0;
-    r.skip = 1;
-    r.timeout_ns = DEFAULT_TIMEOUT_NS;
-    const Layout l = plan_layout(n, w, r.chunk_log2, d_mask_out == nullptr);
+    const size_t need = align256(sizeof(ws_header) + 8 * if_max_slices(n, w));
     void* ws = nullptr;
     size_t ws_bytes = 0;
-    st = cached_workspace(l.total, s, &ws, &ws_bytes);
+    st = cached_workspace(need, s, &ws, &ws_bytes);
     if (st) return st;
-    uint8_t* wsb = static_cast<uint8_t*>(ws);
-    ws_header* hdr = reinterpret_cast<ws_header*>(wsb);
-    uint32_t* mask = d_mask_out ? d_mask_out : reinterpret_cast<uint32_t*>(wsb + l.off_mask);
-    uint64_t* offsets = reinterpret_cast<uint64_t*>(wsb + l.off_offsets);
-    uint64_t* blk_base = reinterpret_cast<uint64_t*>(wsb + l.off_blk_base);
-    ColumnDesc col = make_column(d_in, mask, d_out, n, w, d_count, offsets);
-    col.blk_base = blk_base;
-    pp.bs.col0 = col;
-    pp.bs.num_blocks = (n + (1ull << SCAN_BLOCK_LOG2) - 1) >> SCAN_BLOCK_LOG2;
-    pp.bs.blk_sum = reinterpret_cast<uint64_t*>(wsb + l.off_scan_status);
-    pp.bs.blk_base = blk_base;
-    pp.bs.hdr = hdr;
-    pp.bs.item_flags = reinterpret_cast<uint32_t*>(wsb + l.off_item_flags);
-    pp.bs.chunk_log2 = r.chunk_log2;
-    pp.bs.keep_begin = l.off_counts;
-    pp.bs.keep_end = l.off_flags + 4 * POPC_FLAG_SLOTS;
-    pp.in = static_cast<const uint8_t*>(d_in);
-    pp.mask = mask;
-    cudaError_t e = launch_pred_mask(pp, pred->type, pred->op, di.sms, s);
-    if (e != cudaSuccess) return cuda_status(e);
-    e = launch_popc_blocks(pp.bs, di.sms, s);
-    if (e != cudaSuccess) return cuda_status(e);
-    return launch_writeout_3pass(col, l, hdr, r, true, pp.bs.item_flags, di, s);
+    p.in = static_cast<const uint8_t*>(d_in);
+    p.out = static_cast<uint8_t*>(d_out);
+    p.mask = d_mask_out;
+    p.n = n;
+    p.d_count = d_count;
+    p.hdr = static_cast<ws_header*>(ws);
+    p.status = reinterpret_cast<uint64_t*>(static_cast<uint8_t*>(ws) + sizeof(ws_header));
+    p.timeout_ns = DEFAULT_TIMEOUT_NS;
+    return cuda_status(launch_if(p, pred->type, di.sms, s));
 }
 
 int cs_workspace_check(void* d_ws, cs_stream_t stream)

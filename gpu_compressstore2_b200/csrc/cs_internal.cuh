@@ -306,6 +306,45 @@ __device__ __forceinline__ uint64_t lookback_cta(uint64_t* status, uint64_t tile
     return excl;
 }
 
+// Sum of the totals published for slices [from, to), read by a whole CTA of NT threads: a thread
+// polls its slices' statuses (any flag but POISON of this epoch), each warp leaves its part of the
+// sum in red[0 .. NT / 32). Returns, per thread, whether all of them appeared in time; the caller
+// adds up `red` after a barrier. For to - from <= 2 * NT and slices of less than 2^22 elements.
+template <int NT>
+__device__ __forceinline__ bool poll_totals(const uint64_t* status, uint32_t from, uint32_t to, uint32_t epoch,
+                                            uint64_t timeout_ns, uint32_t* red)
+{
+    uint32_t sum = 0;
+    bool ok = true;
+    uint64_t s[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const uint32_t at = from + threadIdx.x + i * NT;
+        s[i] = at < to ? ld_relaxed_gpu(status + at) : pack_status(epoch, FLAG_AGG, 0);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const uint32_t at = from + threadIdx.x + i * NT;
+        if (status_epoch(s[i]) != epoch) {
+            const uint64_t t0 = globaltimer_ns();
+            uint32_t spins = 0;
+            do {
+                __nanosleep(spins < 16 ? 20 : 100);
+                s[i] = ld_relaxed_gpu(status + at);
+                if ((++spins & 63u) == 0u && globaltimer_ns() - t0 > timeout_ns) {
+                    ok = false;
+                    s[i] = pack_status(epoch, FLAG_AGG, 0);
+                }
+            } while (status_epoch(s[i]) != epoch);
+        }
+        sum += static_cast<uint32_t>(status_value(s[i]));
+    }
+    __syncwarp();
+    sum = __reduce_add_sync(0xffffffffu, sum);
+    if ((threadIdx.x & 31u) == 0u) red[threadIdx.x >> 5] = sum;
+    return ok;
+}
+
 __host__ __device__ __forceinline__ uint32_t prev_epoch(uint32_t e)
 {
     return e == EPOCH_MIN ? EPOCH_MAX : e - 1u;
@@ -535,16 +574,21 @@ struct BlockScanParams {
     uint64_t keep_end;        // preserved by the epoch-wrap clear
 };
 
-// Predicate compaction, mask pass (cs_predicate.cu): bs.col0 is the column (its mask is
-// `mask`, written by the kernel); lo and hi hold the comparison's bounds as bit patterns of
-// the element type in their low bytes (lo_incl, hi_incl and negate describe the same
-// selection in bounds form).
-struct PredParams {
-    BlockScanParams bs;
+// Predicate compaction (cs_predicate.cu). lo, hi: bit patterns of the element type in their low
+// bytes; whole numbers: the lower bound and the distance to the upper one, modulo the width.
+struct IfParams {
     const uint8_t* in;
-    uint32_t* mask;
+    uint8_t* out;
+    uint32_t* mask;      // null, or where the selection's words go
+    uint64_t n;
+    uint64_t* d_count;
+    ws_header* hdr;
+    uint64_t* status;    // if_max_slices words
     uint64_t lo, hi;
-    uint32_t lo_incl, hi_incl, negate, pad;
+    uint64_t timeout_ns;
+    uint32_t negate;
+    uint32_t sides;      // floating numbers: 1 only a lower bound, 2 only an upper one, 3 both
+    uint32_t num_slices; // set by the launcher
 };
 
 // Last CTA of a reduce-then-scan pass (all 256 threads): turns the block sums into the
@@ -662,7 +706,9 @@ cudaError_t launch_scan(const ScanParams& p, int num_sms, cudaStream_t stream);
 constexpr uint32_t FUSED_TILE_CHUNKS = 64; // 4096-element chunks per reduce-then-scan block
 static_assert(FUSED_TILE_CHUNKS * 4096u == (1u << SCAN_BLOCK_LOG2), "a plan tile is one scan block");
 cudaError_t launch_popc_blocks(const BlockScanParams& p, int num_sms, cudaStream_t stream);
-cudaError_t launch_pred_mask(const PredParams& p, int type, int op, int num_sms, cudaStream_t stream);
+// Predicate compaction; 16-byte aligned pointers.
+cudaError_t launch_if(const IfParams& p, int type, int num_sms, cudaStream_t stream);
+uint64_t if_max_slices(uint64_t n, uint32_t elem_bytes); // look-back statuses it may use
 __host__ __device__ constexpr uint64_t sparse_items_for(uint64_t n)
 {
     return ((n + 1023) / 1024 + 15) / 16; // items of 16 blocks of 1024 elements

@@ -180,4 +180,57 @@ __device__ __forceinline__ void emit_stage(uint8_t* gdst, const uint8_t* stage, 
     }
 }
 
+// Stage positions of a lane's four runs, from the lanes' counts: two rows (at most 1024 elements
+// each) per packed scan. `a`: position of the item's first selected element; returns the end.
+__device__ __forceinline__ uint32_t scan_item(const uint32_t (&bits)[ROWS], uint32_t a, uint32_t (&pos)[ROWS], uint32_t lane)
+{
+    uint32_t run = a;
+#pragma unroll
+    for (uint32_t r = 0; r < ROWS; r += 2) {
+        const uint32_t own = __popc(bits[r]) | (__popc(bits[r + 1]) << 16);
+        const uint32_t incl = warp_incl_scan(own, lane);
+        const uint32_t all = __shfl_sync(0xffffffffu, incl, 31);
+        pos[r] = run + ((incl - own) & 0xffffu);
+        run += all & 0xffffu;
+        pos[r + 1] = run + ((incl - own) >> 16);
+        run += all >> 16;
+    }
+    return run;
+}
+
+// The selected elements of an item (bits of x) through the stage to gdst + [a, run): the positions
+// are scan_item's, gdst is 16-byte aligned.
+template <typename T>
+__device__ __forceinline__ void write_item(const uint32_t (&x)[ROWS][8], const uint32_t (&bits)[ROWS],
+                                           const uint32_t (&pos)[ROWS], uint32_t a, uint32_t run, uint8_t* gdst,
+                                           uint8_t* stage, uint32_t lut, uint32_t lane)
+{
+    constexpr uint32_t ITEM = ITEM_BYTES / sizeof(T);
+    const uint32_t base = smem_u32(stage);
+    uint32_t swz = 0u;
+    Tail tail[ROWS];
+    __syncwarp(); // lanes that passed their payload through the stage have read it
+    if ((sizeof(T) == 2 || sizeof(T) == 4) && run - a > ITEM / 16 * 15) {
+        // nearly all of the item is selected: the lanes' elements lie 8 words apart (2^28 u32 runs of
+        // 4096 262 -> 239 us, 2^28 u16 205 -> 170, p = 0.99 247 -> 204; with every item 2^28 u16
+        // p = 0.5 151 -> 162)
+        swz = 0x70u;
+#pragma unroll
+        for (uint32_t r = 0; r < ROWS; ++r)
+            place_row<T, (sizeof(T) > 1)>(x[r], bits[r], base + pos[r] * static_cast<uint32_t>(sizeof(T)), lut);
+    } else {
+#pragma unroll
+        for (uint32_t r = 0; r < ROWS; ++r)
+            tail[r] = place_row<T, false>(x[r], bits[r], base + pos[r] * static_cast<uint32_t>(sizeof(T)), lut);
+    }
+    if constexpr (sizeof(T) == 1) {
+        __syncwarp(); // every whole word is in the stage before the partial ones
+#pragma unroll
+        for (uint32_t r = 0; r < ROWS; ++r) place_tail(tail[r]);
+    }
+    __syncwarp();
+    emit_stage<T>(gdst, stage, a, run, lane, swz);
+    __syncwarp(); // the stage is rewritten by the next item
+}
+
 } // namespace cs

@@ -1,22 +1,56 @@
-// cs_predicate.cu — pass 0 of predicate compaction: the selection mask is computed from
-// the payload on the device instead of being read (k_pred_mask). The 3-pass form then runs
-// on that mask: k_popc_blocks (chunk counts and prefixes) and the writeout.
+// cs_predicate.cu — predicate compaction (compressstore_if): the selection is a comparison
+// evaluated on the payload, in one kernel that reads the payload from HBM once.
+//
+// The column is cut into slices of 32 KB: 8 warps x an item of 4 KB (cs_place.cuh). CTAs take slices
+// in order from a device counter and work two slices ahead of themselves. In each turn a CTA
+//   evaluates the slice two turns ahead: loads its payload, keeps its mask bits in registers and
+//             publishes its count; the payload itself is dropped and stays in L2;
+//   sums      the counts of the slices between its last one and the present one (about one per
+//             CTA; published two turns ago, so it rarely waits): with the selected elements
+//             before its last slice, which it carries along, that is the present slice's offset;
+//   writes    the present slice: loads the payload again, now from L2, places and stores the
+//             selected elements (an item with few is listed and gathered instead).
+// The warps of a CTA meet at one barrier per turn. A CTA only ever waits for slices that running
+// CTAs already hold, in order. Waits are bounded; one that gives up records an error, the CTA
+// writes nothing more and the count reads CS_COUNT_ERROR.
+//
+// What bounds it is instructions: the evaluation and the placing together take about as long as
+// 16 warps' issue of an SM allows while the payload streams at 4 to 5 TB/s. Per call on B200
+// against a mask pass, pass 1 + 2 and the writeout, which read the payload from HBM twice, before ->
+// now: 2^28 f32 x > c with 0.5 selected 459 -> 328 us, 0.01 259 -> 227, 0.1 414 -> 274, 0.9 556 -> 410;
+// 2^27 f64 463 -> 313, 2^28 i16 289 -> 217, 2^28 u8 225 -> 179, 2^24 f32 41 -> 25, 2^20 18 -> 7.
+// Tried: a look-back over slices instead of the carried sum (it grows with the number of slices: 494
+// us at the best slice size), evaluating one slice ahead (365), slices of two items per warp
+// (374 .. 384), 2 and 4 CTAs per SM (408, 378), the evaluated payload through shared memory by bulk
+// copies (377).
+//
+// A comparison of whole numbers is (x - lo) <= (hi - lo) in unsigned arithmetic, whatever the sign
+// (the host turns each operator into bounds), one of floating numbers lo <= x && x <= hi; != is the
+// negation of ==. Every ordered comparison with a NaN is false, != is true (C++ semantics).
+//
 // Reference: the reference evaluates the predicate on the host while packing the mask
 // (gen_predicate, src/utils.cuh:102-122, with predicate_function x > threshold,
 // src/main.cu:24-28,92) and copies mask and payload to the device before compacting.
 #include <cstdint>
 #include <cstring>
-
-#include <atomic>
+#include <type_traits>
 
 #include <cuda_runtime.h>
 
 #include "compressstore.h"
 #include "cs_internal.cuh"
+#include "cs_place.cuh"
 
 namespace cs {
 
 namespace {
+
+constexpr uint32_t WARPS = 8;
+constexpr uint32_t CTAS = 3; // per SM
+// Selected elements of an item up to which they are listed and gathered (2^28 f32 with 0.01 selected
+// 256 -> 227 us). Their ranks within a row take 8 bits.
+constexpr uint32_t FEW = 64;
+static_assert(FEW < 256, "ranks in 8 bits");
 
 template <typename T>
 __device__ __forceinline__ T from_bits(uint64_t b)
@@ -26,174 +60,331 @@ __device__ __forceinline__ T from_bits(uint64_t b)
     return v;
 }
 
-// The comparison of each cs_pred_op as one instruction where it can be; lo/hi are the
-// host-prepared bounds (LT/LE: hi = a; GT/GE/EQ/NE: lo = a; BETWEEN: lo = a, hi = b). Every
-// ordered comparison with a NaN is false, != is true (C++ semantics).
-template <int OP, typename T>
-__device__ __forceinline__ bool pred_eval(T x, T lo, T hi)
+// Which bounds a comparison of floating numbers has (whole numbers take both in one).
+enum Sides { FROM = 1, TO = 2, BOTH = 3 };
+
+// Selected elements of a lane's 32 bytes, as bits.
+template <typename T, int SIDES>
+__device__ __forceinline__ uint32_t select_row(const uint32_t (&x)[8], T lo, T hi)
 {
-    if constexpr (OP == CS_PRED_LT) return x < hi;
-    else if constexpr (OP == CS_PRED_LE) return x <= hi;
-    else if constexpr (OP == CS_PRED_GT) return x > lo;
-    else if constexpr (OP == CS_PRED_GE) return x >= lo;
-    else if constexpr (OP == CS_PRED_EQ) return x == lo;
-    else if constexpr (OP == CS_PRED_NE) return x != lo;
-    else return lo <= x && x <= hi;
+    constexpr uint32_t EPL = LANE_BYTES / sizeof(T);
+    constexpr bool REAL = T(0.5) != T(0);
+    uint32_t b = 0;
+#pragma unroll
+    for (uint32_t e = 0; e < EPL; ++e) {
+        bool s;
+        if constexpr (REAL) {
+            T v;
+            if constexpr (sizeof(T) == 8)
+                v = __longlong_as_double(static_cast<long long>(static_cast<uint64_t>(x[2 * e]) | (static_cast<uint64_t>(x[2 * e + 1]) << 32)));
+            else
+                v = __uint_as_float(x[e]);
+            s = SIDES == FROM ? lo <= v : SIDES == TO ? v <= hi : lo <= v && v <= hi;
+        } else if constexpr (sizeof(T) == 8) {
+            s = (static_cast<uint64_t>(x[2 * e]) | (static_cast<uint64_t>(x[2 * e + 1]) << 32)) - lo <= hi;
+        } else {
+            constexpr uint32_t PER = 4 / sizeof(T);
+            s = static_cast<T>(static_cast<T>(x[e / PER] >> ((e % PER) * 8 * sizeof(T))) - lo) <= hi;
+        }
+        if (s) b |= 1u << e;
+    }
+    return b;
 }
 
-// Mask words from the payload: a grid-stride pass in which every thread takes UNR 16-byte
-// vectors (16 / w elements each) per iteration, all loads before the evaluation; the
-// G = 32 / (16 / w) lanes that share a mask word OR their shifted bits with xor shuffles and
-// one of them stores the word. Bits at positions >= n are zero.
-// 16-byte vectors per thread per iteration, and whether the grid is one resident wave.
-// Measured on B200 (us per compressstore_if call, one wave vs a grid of 8 CTAs per SM, of
-// which only the resident ones run at first): 2^28 f32 497 -> 468 (UNR 4; 8: 467), 2^28 u64
-// 1170 -> 938 (UNR 8; 4: 1073), but 2^29 u8 463 -> 467 and u16 585 -> 594, whose per-element
-// evaluation keeps the old grid busy. With the bounds-free path, UNR 8 on the old grid:
-// u8 428.5 -> 425.7, u16 579.0 -> 553.9 (one wave with UNR 8: 431.0 / 560.8).
-template <typename T>
-struct PredShape {
-    static constexpr uint32_t UNR = sizeof(T) == 4 ? 4u : 8u;
-    static constexpr bool ONE_WAVE = sizeof(T) >= 4;
-};
-
-template <typename T, int OP>
-__global__ void __launch_bounds__(256) k_pred_mask(const PredParams pp)
+// T: uint8_t .. uint64_t (bounds lo and hi - lo), float, double (bounds lo, hi).
+template <typename T, int SIDES>
+__global__ void __launch_bounds__(WARPS * 32, CTAS) k_if(const IfParams p)
 {
-    constexpr uint32_t VEC = 16 / sizeof(T); // elements per lane load
-    constexpr uint32_t G = 32 / VEC;         // lanes per mask word
-    constexpr uint32_t UNR = PredShape<T>::UNR;
+    constexpr uint32_t EPL = LANE_BYTES / sizeof(T);
+    constexpr uint32_t ROW = 32 * EPL;
+    constexpr uint32_t ITEM = ROWS * ROW;
+    constexpr uint32_t VEC = 16 / sizeof(T);
+    constexpr int PK = EPL * ROWS > 32 ? EPL * ROWS / 32 : 1; // words that hold a lane's bits of an item
+    constexpr uint32_t ROW_BITS = EPL == 32 ? 0xffffffffu : (1u << (EPL & 31u)) - 1u;
+    __shared__ __align__(128) uint8_t s_stage[WARPS][STAGE_BYTES];
+    __shared__ uint32_t s_lut[sizeof(T) == 1 ? PACK_TABLE_WORDS : 1];
+    // By the slice's turn in this CTA (modulo 4: a slice is evaluated two turns ahead, one barrier
+    // per turn), and the parts of a turn's sum by its parity.
+    __shared__ uint32_t s_slice[4];                      // the slice of each turn
+    __shared__ __align__(16) uint32_t s_total[4][WARPS]; // selected elements of each warp's part of it
+    __shared__ uint32_t s_sum[4];                        // of the warps that have counted so far, and their number (bits 24 on)
+    __shared__ __align__(16) uint32_t s_red[2][WARPS];   // parts of the sum of the totals since this CTA's last slice
+    __shared__ uint32_t s_epoch, s_failed;
+    static_assert(WARPS == 8, "two vectors of warp totals");
+    using U = typename std::conditional<sizeof(T) == 1, uint8_t, typename std::conditional<sizeof(T) == 2, uint16_t,
+              typename std::conditional<sizeof(T) == 4, uint32_t, uint64_t>::type>::type>::type;
     const uint32_t lane = threadIdx.x & 31u;
-    const T lo = from_bits<T>(pp.lo), hi = from_bits<T>(pp.hi);
-    grid_dependency_wait(); // an earlier call may still read this mask buffer
-    const uint64_t n = pp.bs.col0.n;
-    const uint64_t nw = (n + 31) / 32;
-    const uint64_t nvec = (n + VEC - 1) / VEC;
-    const T* __restrict__ in = reinterpret_cast<const T*>(pp.in);
-    uint32_t* __restrict__ mask = pp.mask;
-    // warps stride over groups of 32 vectors; a thread's vector is (group * 32 + lane)
-    const uint64_t warp_global = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    const uint64_t total_warps = (static_cast<uint64_t>(gridDim.x) * blockDim.x) >> 5;
-    const uint64_t ngroups = (nvec + 31) / 32;
-    const uint4* __restrict__ in4 = reinterpret_cast<const uint4*>(pp.in);
-    const uint64_t vstride = total_warps * 32;  // vectors between a thread's consecutive groups
-    const uint64_t wstride = total_warps * VEC; // mask words between them
-    const uint32_t sh = (lane * VEC) & 31u;
-    for (uint64_t g0 = warp_global; g0 < ngroups; g0 += UNR * total_warps) {
-        union {
-            uint4 u;
-            T e[VEC];
-        } x[UNR];
-        if ((g0 + (UNR - 1) * total_warps + 1) * 32 * VEC <= n) {
-            // every group of this iteration is complete: no per-element bounds or tail bits
-            const uint4* src = in4 + g0 * 32 + lane;
+    const uint32_t warp = threadIdx.x >> 5;
+    uint8_t* const stage = s_stage[warp];
+    const uint32_t stage_a = smem_u32(stage);
+    const uint32_t lut = sizeof(T) == 1 ? smem_u32(s_lut) + lane * 4 : 0u;
+    const T lo = from_bits<T>(p.lo), hi = from_bits<T>(p.hi);
+    const uint32_t negate = p.negate ? ROW_BITS : 0u;
+    const uint64_t n = p.n;
+    const uint8_t* __restrict__ in = p.in;
+    const bool in32 = (reinterpret_cast<uintptr_t>(in) & 31u) == 0;
+    if constexpr (sizeof(T) == 1) fill_pack_table(s_lut, WARPS * 32);
+    grid_dependency_wait();
+    if (threadIdx.x == 0) {
+        s_epoch = p.hdr->epoch;
+        s_slice[0] = atomicAdd(&p.hdr->tile_counter, 1u);
+        s_failed = 0u;
+        for (uint32_t t = 0; t < 4; ++t) s_sum[t] = 0u;
+    }
+    __syncthreads();
+    const uint32_t epoch = s_epoch;
+
+    auto item_elem = [&](uint32_t slice) -> uint64_t { return (static_cast<uint64_t>(slice) * WARPS + warp) * ITEM; };
+    // the lane's 32 bytes of row r of the item at e0, where the column ends in or before the item:
+    // the lane in which it ends goes element by element, through its place in the idle stage
+    auto load_ragged = [&](uint64_t e0, uint32_t r, uint32_t (&x)[8]) {
+        const uint64_t e = e0 + r * ROW + lane * EPL;
+        const uint8_t* src = in + e * sizeof(T);
+        if (e + EPL <= n) {
+            ldg128x2(src, x);
+        } else if (e < n) {
+            U* tmp = reinterpret_cast<U*>(stage + lane * LANE_BYTES);
+            for (uint32_t i = 0; e + i < n; ++i) tmp[i] = __ldg(reinterpret_cast<const U*>(src) + i);
 #pragma unroll
-            for (uint32_t k = 0; k < UNR; ++k) x[k].u = __ldg(src + k * vstride);
-            uint32_t* dst = mask + g0 * VEC + lane / G;
+            for (uint32_t q = 0; q < 8; ++q) x[q] = lds32(stage_a + lane * LANE_BYTES + 4 * q);
+        }
+    };
+    auto load_whole = [&](const uint8_t* src, uint32_t (&x)[8]) {
+        if (in32) ldg256(src, x);
+        else ldg128x2(src, x);
+    };
+    auto row_bits = [&](const uint32_t (&b)[PK], uint32_t r) -> uint32_t {
+        return (b[r * EPL / 32] >> (r * EPL % 32)) & ROW_BITS;
+    };
+    // this warp's part of a slice
+    auto load_item = [&](uint32_t slice, uint32_t (&x)[ROWS][8]) {
+        const uint64_t e0 = item_elem(slice);
+        if (e0 + ITEM <= n) {
+            const uint8_t* src = in + e0 * sizeof(T) + lane * LANE_BYTES;
 #pragma unroll
-            for (uint32_t k = 0; k < UNR; ++k) {
-                uint32_t bits = 0;
+            for (uint32_t r = 0; r < ROWS; ++r) load_whole(src + r * ROW_BYTES, x[r]);
+        } else {
 #pragma unroll
-                for (uint32_t i = 0; i < VEC; ++i) bits |= static_cast<uint32_t>(pred_eval<OP>(x[k].e[i], lo, hi)) << i;
-                uint32_t m = bits << sh;
+            for (uint32_t r = 0; r < ROWS; ++r) load_ragged(e0, r, x[r]);
+        }
+    };
+    // evaluates it into b; the last warp to do so publishes the slice's total
+    auto evaluate = [&](uint32_t slice, const uint32_t (&x)[ROWS][8], uint32_t (&b)[PK], uint32_t turn) {
+        const uint64_t e0 = item_elem(slice);
+        const bool whole = e0 + ITEM <= n;
+        uint32_t cnt = 0;
 #pragma unroll
-                for (uint32_t d = 1; d < G; d <<= 1) m |= __shfl_xor_sync(0xffffffffu, m, d);
-                if ((lane % G) == 0u) dst[k * wstride] = m;
+        for (int q = 0; q < PK; ++q) b[q] = 0;
+#pragma unroll
+        for (uint32_t r = 0; r < ROWS; ++r) {
+            uint32_t s = select_row<T, SIDES>(x[r], lo, hi) ^ negate;
+            if (!whole) {
+                const uint64_t e = e0 + r * ROW + lane * EPL;
+                if (e + EPL > n) s = e < n ? s & ((1u << (n - e)) - 1u) : 0u; // n - e < EPL <= 32
             }
-            continue;
+            b[r * EPL / 32] |= s << (r * EPL % 32);
         }
 #pragma unroll
-        for (uint32_t k = 0; k < UNR; ++k) {
-            const uint64_t v = (g0 + k * total_warps) * 32 + lane;
-            const uint64_t e0 = v * VEC;
-            if (e0 + VEC <= n) {
-                x[k].u = __ldg(reinterpret_cast<const uint4*>(in) + v);
+        for (int q = 0; q < PK; ++q) cnt += __popc(b[q]);
+        cnt = __reduce_add_sync(0xffffffffu, cnt);
+        if (lane == 0) {
+            s_total[turn][warp] = cnt;
+            const uint32_t before = atomicAdd(&s_sum[turn], cnt + (1u << 24));
+            if (before >> 24 == WARPS - 1) {
+                s_sum[turn] = 0u; // used again four turns on, past a barrier
+                st_relaxed_gpu(&p.status[slice], pack_status(epoch, FLAG_AGG, (before & 0xffffffu) + cnt));
+            }
+        }
+        if (p.mask) {
+            // the lane's bits of the mask words that hold an element of the column
+            const uint64_t bound = (n + 31) / 32 * 32;
+#pragma unroll
+            for (uint32_t r = 0; r < ROWS; ++r) {
+                const uint64_t e = e0 + r * ROW + lane * EPL;
+                uint8_t* mb = reinterpret_cast<uint8_t*>(p.mask) + (e >> 3);
+                const uint32_t s = row_bits(b, r);
+                if constexpr (EPL == 32) {
+                    if (e < bound) *reinterpret_cast<uint32_t*>(mb) = s;
+                } else if constexpr (EPL == 16) {
+                    if (e < bound) *reinterpret_cast<uint16_t*>(mb) = static_cast<uint16_t>(s);
+                } else if constexpr (EPL == 8) {
+                    if (e < bound) *mb = static_cast<uint8_t>(s);
+                } else {
+                    const uint32_t pair = s | (__shfl_down_sync(0xffffffffu, s, 1) << 4);
+                    if (e < bound && !(lane & 1u)) *mb = static_cast<uint8_t>(pair);
+                }
+            }
+        }
+    };
+    uint32_t bits[PK], bits1[PK]; // of the slice to be written and the one after it
+    uint64_t end = 0;  // selected elements before slice `done`
+    uint32_t done = 0; // the slices up to this CTA's last one
+    uint32_t turn = 0;
+    // The first two slices. A CTA takes each slice only when it is about to evaluate it (or, in the
+    // loop, a turn before), so that the CTAs' slices interleave: a slice in front of another CTA's
+    // is evaluated no later than that one.
+#pragma unroll
+    for (uint32_t t = 0; t < 2; ++t) {
+        const uint32_t slice = s_slice[t];
+        const bool some = slice < p.num_slices;
+        if (some) {
+            uint32_t x[ROWS][8];
+            load_item(slice, x);
+            if (t == 0) evaluate(slice, x, bits, 0);
+            else evaluate(slice, x, bits1, 1);
+        }
+        if (threadIdx.x == 0) s_slice[t + 1] = some ? atomicAdd(&p.hdr->tile_counter, 1u) : slice;
+        __syncthreads();
+    }
+    while (true) {
+        const uint32_t slice = s_slice[turn];
+        if (slice >= p.num_slices) break;
+        const uint32_t later = (turn + 2) & 3u;
+        const uint32_t next = s_slice[later]; // the slice to evaluate in this turn
+        uint32_t ahead[PK];
+        uint32_t x[ROWS][8];
+        const bool more = next < p.num_slices;
+        if (more) load_item(next, x);
+        if (threadIdx.x == 0) s_slice[(turn + 3) & 3u] = more ? atomicAdd(&p.hdr->tile_counter, 1u) : next;
+        // the totals of the slices since this CTA's last one, 512 at a time
+        uint32_t* const red = s_red[turn & 1u];
+        for (; slice - done > 2 * WARPS * 32; done += 2 * WARPS * 32) {
+            if (!poll_totals<WARPS * 32>(p.status, done, done + 2 * WARPS * 32, epoch, p.timeout_ns, red)) s_failed = 1u;
+            __syncthreads();
+#pragma unroll
+            for (uint32_t w = 0; w < WARPS; ++w) end += red[w];
+            __syncthreads();
+        }
+        if (!poll_totals<WARPS * 32>(p.status, done, slice, epoch, s_failed ? 0ull : p.timeout_ns, red)) s_failed = 1u;
+        if (more) evaluate(next, x, ahead, later);
+        // The present slice's item, from L2: few selected elements are listed and gathered, otherwise
+        // the lanes with selected elements load theirs
+        const uint64_t e0 = item_elem(slice);
+        const uint32_t mine = s_total[turn][warp];
+        const bool few = mine <= FEW;
+        if (!few) {
+            if (e0 + ITEM <= n) {
+                const uint8_t* src = in + e0 * sizeof(T) + lane * LANE_BYTES;
+#pragma unroll
+                for (uint32_t r = 0; r < ROWS; ++r)
+                    if (row_bits(bits, r)) load_whole(src + r * ROW_BYTES, x[r]);
             } else {
 #pragma unroll
-                for (uint32_t i = 0; i < VEC; ++i) x[k].e[i] = e0 + i < n ? in[e0 + i] : T(0);
+                for (uint32_t r = 0; r < ROWS; ++r)
+                    if (row_bits(bits, r)) load_ragged(e0, r, x[r]);
             }
         }
-#pragma unroll
-        for (uint32_t k = 0; k < UNR; ++k) {
-            const uint64_t g = g0 + k * total_warps;
-            if (g >= ngroups) break; // warp-uniform
-            uint32_t bits = 0;
-#pragma unroll
-            for (uint32_t i = 0; i < VEC; ++i) bits |= static_cast<uint32_t>(pred_eval<OP>(x[k].e[i], lo, hi)) << i;
-            if ((g + 1) * 32 * VEC > n) { // the last group: clear bits at positions >= n
-                const uint64_t e0 = (g * 32 + lane) * VEC;
-                bits &= e0 >= n ? 0u : (e0 + VEC <= n ? 0xffffffffu : ((1u << (n - e0)) - 1u));
+        __syncthreads(); // the sums of this turn; every warp has left the turn before
+        const uint4 t0 = lds128(s_total[turn]), t1 = lds128(s_total[turn] + 4);
+        const uint4 r0 = lds128(red), r1 = lds128(red + 4);
+        const uint64_t base = end + (static_cast<uint64_t>(r0.x) + r0.y + r0.z + r0.w) + (static_cast<uint64_t>(r1.x) + r1.y + r1.z + r1.w);
+        end = base + (t0.x + t0.y + t0.z + t0.w + t1.x + t1.y + t1.z + t1.w);
+        done = slice + 1;
+        const bool failed = s_failed != 0u;
+        if (threadIdx.x == 0) {
+            if (failed) {
+                record_error(p.hdr, DEVERR_LOOKBACK_TIMEOUT);
+                reinterpret_cast<volatile ws_header*>(p.hdr)->poison_epoch = epoch;
             }
-            uint32_t m = bits << ((lane * VEC) & 31u);
-#pragma unroll
-            for (uint32_t d = 1; d < G; d <<= 1) m |= __shfl_xor_sync(0xffffffffu, m, d);
-            const uint64_t word = g * VEC + lane / G; // a group of 32 vectors covers VEC words
-            if ((lane % G) == 0u && word < nw) mask[word] = m;
+            if (slice == p.num_slices - 1) *p.d_count = end;
         }
+        if (!failed && mine != 0u) {
+            const uint64_t off = base + (warp > 0 ? t0.x : 0u) + (warp > 1 ? t0.y : 0u) + (warp > 2 ? t0.z : 0u) + (warp > 3 ? t0.w : 0u) +
+                                 (warp > 4 ? t1.x : 0u) + (warp > 5 ? t1.y : 0u) + (warp > 6 ? t1.z : 0u);
+            if (few) {
+                uint16_t* const list = reinterpret_cast<uint16_t*>(stage);
+                // ranks row by row: at most FEW elements, so the four rows' counts fit one scanned word
+                uint32_t own = 0;
+#pragma unroll
+                for (uint32_t r = 0; r < ROWS; ++r) own |= static_cast<uint32_t>(__popc(row_bits(bits, r))) << (8 * r);
+                const uint32_t incl = warp_incl_scan(own, lane);
+                const uint32_t all = __shfl_sync(0xffffffffu, incl, 31);
+                const uint32_t excl = incl - own;
+                uint32_t before = 0;
+#pragma unroll
+                for (uint32_t r = 0; r < ROWS; ++r) {
+                    uint32_t at = before + ((excl >> (8 * r)) & 0xffu);
+                    for (uint32_t m = row_bits(bits, r); m != 0u; m &= m - 1)
+                        list[at++] = static_cast<uint16_t>(r * ROW + lane * EPL + __ffs(m) - 1);
+                    before += (all >> (8 * r)) & 0xffu;
+                }
+                __syncwarp();
+                const U* src = reinterpret_cast<const U*>(in) + e0;
+                U* dst = reinterpret_cast<U*>(p.out) + off;
+                for (uint32_t j = lane; j < mine; j += 32) dst[j] = ldg_gather(src + list[j]);
+                __syncwarp();
+            } else {
+                const uint32_t a = static_cast<uint32_t>((reinterpret_cast<uintptr_t>(p.out) / sizeof(T) + off) % VEC);
+                uint32_t rb[ROWS], pos[ROWS];
+#pragma unroll
+                for (uint32_t r = 0; r < ROWS; ++r) rb[r] = row_bits(bits, r);
+                const uint32_t run = scan_item(rb, a, pos, lane);
+                write_item<U>(x, rb, pos, a, run,
+                              p.out + (static_cast<int64_t>(off) - static_cast<int64_t>(a)) * static_cast<int64_t>(sizeof(T)),
+                              stage, lut, lane);
+            }
+        }
+        turn = (turn + 1) & 3u;
+#pragma unroll
+        for (int q = 0; q < PK; ++q) {
+            bits[q] = bits1[q];
+            bits1[q] = ahead[q];
+        }
+    }
+    // the last CTA closes the epoch, and takes the count back if a wait gave up anywhere
+    __shared__ uint32_t s_flag;
+    if (epilogue_ticket(&p.hdr->done_counter, &s_flag)) {
+        if (threadIdx.x == 0 && reinterpret_cast<volatile ws_header*>(p.hdr)->poison_epoch == epoch) *p.d_count = COUNT_ERROR;
+        epilogue_last(p.hdr, &p.hdr->tile_counter, &p.hdr->done_counter, false, 0, 0, nullptr);
     }
 }
 
-// CTAs of k_pred_mask<T, OP> resident on one SM at once (taken once). For 4- and 8-byte
-// elements the grid-stride pass is launched as one wave of them: CTAs beyond it would run
-// their whole share after the first wave finished, with a fraction of the bytes in flight.
-template <typename T, int OP>
-int pred_resident_per_sm()
+template <typename T, int SIDES>
+cudaError_t launch_s(const IfParams& p, int num_sms, cudaStream_t stream)
 {
-    static std::atomic<int> cached{0};
-    int v = cached.load(std::memory_order_relaxed);
-    if (v > 0) return v;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k_pred_mask<T, OP>, 256, 0) != cudaSuccess || v < 1) {
-        cudaGetLastError();
-        v = 4;
-    }
-    cached.store(v, std::memory_order_relaxed);
-    return v;
-}
-
-template <typename T, int OP>
-cudaError_t launch_op(const PredParams& pp, int num_sms, cudaStream_t stream)
-{
-    constexpr uint64_t VEC = 16 / sizeof(T);
-    const uint64_t nvec = (pp.bs.col0.n + VEC - 1) / VEC;
-    constexpr uint64_t UNR = PredShape<T>::UNR;
-    uint64_t blocks = (nvec + 256 * UNR - 1) / (256 * UNR); // one iteration per thread
-    const uint64_t per_sm = PredShape<T>::ONE_WAVE ? static_cast<uint64_t>(pred_resident_per_sm<T, OP>()) : 8u;
-    const uint64_t cap = static_cast<uint64_t>(num_sms) * per_sm;
-    if (blocks > cap) blocks = cap;
-    if (blocks == 0) blocks = 1;
-    return launch_pdl(k_pred_mask<T, OP>, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, stream, pp);
+    IfParams q = p;
+    q.num_slices = static_cast<uint32_t>(if_max_slices(p.n, sizeof(T)));
+    uint64_t grid = static_cast<uint64_t>(num_sms) * CTAS;
+    if (grid > q.num_slices) grid = q.num_slices;
+    return launch_pdl(k_if<T, SIDES>, dim3(static_cast<unsigned>(grid)), dim3(WARPS * 32), 0, stream, q);
 }
 
 template <typename T>
-cudaError_t launch_t(const PredParams& pp, int op, int num_sms, cudaStream_t stream)
+cudaError_t launch_t(const IfParams& p, int num_sms, cudaStream_t stream)
 {
-    switch (op) {
-        case CS_PRED_LT: return launch_op<T, CS_PRED_LT>(pp, num_sms, stream);
-        case CS_PRED_LE: return launch_op<T, CS_PRED_LE>(pp, num_sms, stream);
-        case CS_PRED_GT: return launch_op<T, CS_PRED_GT>(pp, num_sms, stream);
-        case CS_PRED_GE: return launch_op<T, CS_PRED_GE>(pp, num_sms, stream);
-        case CS_PRED_EQ: return launch_op<T, CS_PRED_EQ>(pp, num_sms, stream);
-        case CS_PRED_NE: return launch_op<T, CS_PRED_NE>(pp, num_sms, stream);
-        default: return launch_op<T, CS_PRED_BETWEEN>(pp, num_sms, stream);
-    }
+    return launch_s<T, BOTH>(p, num_sms, stream);
+}
+
+template <typename T>
+cudaError_t launch_real(const IfParams& p, int num_sms, cudaStream_t stream)
+{
+    if (p.sides == FROM) return launch_s<T, FROM>(p, num_sms, stream);
+    if (p.sides == TO) return launch_s<T, TO>(p, num_sms, stream);
+    return launch_s<T, BOTH>(p, num_sms, stream);
 }
 
 } // namespace
 
-cudaError_t launch_pred_mask(const PredParams& pp, int type, int op, int num_sms, cudaStream_t stream)
+uint64_t if_max_slices(uint64_t n, uint32_t elem_bytes)
+{
+    const uint64_t items = (n * elem_bytes + ITEM_BYTES - 1) / ITEM_BYTES;
+    return (items + WARPS - 1) / WARPS;
+}
+
+cudaError_t launch_if(const IfParams& p, int type, int num_sms, cudaStream_t stream)
 {
     cudaError_t e;
     switch (type) {
-        case CS_U8: e = launch_t<uint8_t>(pp, op, num_sms, stream); break;
-        case CS_U16: e = launch_t<uint16_t>(pp, op, num_sms, stream); break;
-        case CS_U32: e = launch_t<uint32_t>(pp, op, num_sms, stream); break;
-        case CS_U64: e = launch_t<uint64_t>(pp, op, num_sms, stream); break;
-        case CS_I8: e = launch_t<int8_t>(pp, op, num_sms, stream); break;
-        case CS_I16: e = launch_t<int16_t>(pp, op, num_sms, stream); break;
-        case CS_I32: e = launch_t<int32_t>(pp, op, num_sms, stream); break;
-        case CS_I64: e = launch_t<int64_t>(pp, op, num_sms, stream); break;
-        case CS_F32: e = launch_t<float>(pp, op, num_sms, stream); break;
-        case CS_F64: e = launch_t<double>(pp, op, num_sms, stream); break;
+        case CS_U8:
+        case CS_I8: e = launch_t<uint8_t>(p, num_sms, stream); break;
+        case CS_U16:
+        case CS_I16: e = launch_t<uint16_t>(p, num_sms, stream); break;
+        case CS_U32:
+        case CS_I32: e = launch_t<uint32_t>(p, num_sms, stream); break;
+        case CS_U64:
+        case CS_I64: e = launch_t<uint64_t>(p, num_sms, stream); break;
+        case CS_F32: e = launch_real<float>(p, num_sms, stream); break;
+        case CS_F64: e = launch_real<double>(p, num_sms, stream); break;
         default: return cudaErrorInvalidValue;
     }
     note_launch();

@@ -332,49 +332,16 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS<SHIFT>) k_writeout_warp(const
         const uint64_t start = off0 + blk; // of the chunk
         const uint64_t off = start + before;
 
-        // positions: two rows (at most 1024 elements each) per packed scan
         uint32_t pos[ROWS];
         const uint32_t a = static_cast<uint32_t>((reinterpret_cast<uintptr_t>(C.out) / sizeof(T) + off) % VEC);
-        uint32_t run = a;
-#pragma unroll
-        for (uint32_t r = 0; r < ROWS; r += 2) {
-            const uint32_t own = __popc(bits[r]) | (__popc(bits[r + 1]) << 16);
-            const uint32_t incl = warp_incl_scan(own, lane);
-            const uint32_t all = __shfl_sync(0xffffffffu, incl, 31);
-            pos[r] = run + ((incl - own) & 0xffffu);
-            run += all & 0xffffu;
-            pos[r + 1] = run + ((incl - own) >> 16);
-            run += all >> 16;
-        }
+        const uint32_t run = scan_item(bits, a, pos, lane);
         if (start > n || off + (run - a) > n) { // inconsistent offsets never write
             if (start != POISON && lane == 0) record_error(p.hdr, DEVERR_RANGE);
             continue;
         }
-        __syncwarp(); // the ragged lanes have read their places in the stage
-        uint32_t swz = 0u;
-        Tail tail[ROWS];
-        if ((sizeof(T) == 2 || sizeof(T) == 4) && run - a > ITEM / 16 * 15) {
-            // nearly all of the item is selected: the lanes' elements lie 8 words apart (2^28 u32 runs of
-            // 4096 262 -> 239 us, 2^28 u16 205 -> 170, p = 0.99 247 -> 204; with every item 2^28 u16
-            // p = 0.5 151 -> 162)
-            swz = 0x70u;
-#pragma unroll
-            for (uint32_t r = 0; r < ROWS; ++r)
-                place_row<T, (sizeof(T) > 1)>(x[r], bits[r], stage_a + pos[r] * static_cast<uint32_t>(sizeof(T)), lut);
-        } else {
-#pragma unroll
-            for (uint32_t r = 0; r < ROWS; ++r)
-                tail[r] = place_row<T, false>(x[r], bits[r], stage_a + pos[r] * static_cast<uint32_t>(sizeof(T)), lut);
-        }
-        if constexpr (sizeof(T) == 1) {
-            __syncwarp(); // every whole word is in the stage before the partial ones
-#pragma unroll
-            for (uint32_t r = 0; r < ROWS; ++r) place_tail(tail[r]);
-        }
-        __syncwarp();
-        emit_stage<T>(C.out + (static_cast<int64_t>(off) - static_cast<int64_t>(a)) * static_cast<int64_t>(sizeof(T)), stage,
-                      a, run, lane, swz);
-        __syncwarp(); // the stage is rewritten by the next item
+        write_item<T>(x, bits, pos, a, run,
+                      C.out + (static_cast<int64_t>(off) - static_cast<int64_t>(a)) * static_cast<int64_t>(sizeof(T)), stage,
+                      lut, lane);
     }
 
     if (!hybrid) return;
