@@ -34,6 +34,13 @@ constexpr uint64_t SHORT_UNITS_MAX = 1024;
 // ... and the deeper payload ring (mode 2) for 4- and 8-byte columns of at least this many
 // full units per SM.
 constexpr uint64_t DEEP_UNITS_PER_SM = 16;
+// Most slices per SM for which a 1-pass call of 4- and 8-byte elements runs in slices (cs_slices.cu)
+// rather than through the TMA kernel; 1- and 2-byte columns of any length do. Per call on B200, inputs
+// from HBM, TMA / slices, us: u32 p = 0.5 2^20 8.5 / 5.4, 2^22 14.3 / 11.4, 2^23 (7 per SM) 20.1 / 15.8,
+// 2^24 (14) 25.6 / 25.7, 2^28 282 / 303; p = 0.1 2^23 16.6 / 13.6, 2^24 21.1 / 21.5; u64 2^22 (7) p = 0.5
+// 18.8 / 15.1, 2^23 p = 0.1 20.1 / 22.6; u8 2^24 17.3 / 13.5, 2^28 133 / 103; u16 2^24 23.2 / 18.7, 2^26
+// 50.9 / 47.4.
+constexpr uint64_t SLICES_PER_SM = 8;
 constexpr uint64_t DEFAULT_TIMEOUT_NS = 2000000000ull;
 
 struct DeviceInfo {
@@ -256,12 +263,33 @@ int run_compaction(const void* d_in, const void* d_mask, void* d_out, uint64_t n
 
     int algo = r.algo;
     const bool tma_ok = aligned(d_in, 16) && aligned(d_out, 16) && aligned(d_mask, 16);
+    // The 1-pass form runs in slices (cs_slices.cu), or through the TMA kernel for 4- and 8-byte columns of
+    // more than SLICES_PER_SM. The slices' totals lie where the 3-pass form has its chunk offsets (which
+    // never read as a status); a caller's chunk length may leave less room than that.
+    const uint64_t slices = slices_of(n, elem_bytes);
+    const bool in_slices = slices <= l.num_chunks &&
+                           (elem_bytes <= 2 || slices <= SLICES_PER_SM * static_cast<uint64_t>(di.sms));
     if ((algo == CS_ALGO_1PASS || algo == CS_ALGO_3PASS) && !tma_ok) {
         if (!auto_route) return CS_ERR_MISALIGNED;
-        // the warp writeout takes any element-aligned pointers; it needs the block pass's offsets
-        algo = r.chunk_log2 >= 7 && r.chunk_log2 <= 12 ? CS_ALGO_3PASS : CS_ALGO_NAIVE;
+        // slices take any mask and output, the warp writeout any element-aligned pointers; the latter
+        // needs the block pass's offsets
+        if (!(algo == CS_ALGO_1PASS && in_slices && aligned(d_in, 16)))
+            algo = r.chunk_log2 >= 7 && r.chunk_log2 <= 12 ? CS_ALGO_3PASS : CS_ALGO_NAIVE;
     }
 
+    if (algo == CS_ALGO_1PASS && in_slices) {
+        SliceParams p{};
+        p.in = static_cast<const uint8_t*>(d_in);
+        p.out = static_cast<uint8_t*>(d_out);
+        p.mask_in = static_cast<const uint32_t*>(d_mask);
+        p.n = n;
+        p.d_count = d_count;
+        p.hdr = hdr;
+        p.status = reinterpret_cast<uint64_t*>(ws + l.off_offsets);
+        p.timeout_ns = r.timeout_ns;
+        p.grid = r.grid;
+        return cuda_status(launch_onepass(p, elem_bytes, di.sms, stream));
+    }
     if (algo == CS_ALGO_1PASS) {
         // a column with fewer full-size units than SMs takes one-tile units, so that about
         // four times as many SMs share it
@@ -423,7 +451,7 @@ int check_workspace_error(void* d_ws, cudaStream_t stream)
 // The predicate as lo <= x <= hi, negated for NE (and for a selection of nothing): inclusive bounds
 // of whole numbers, hi as the distance from lo; of floating numbers the neighbouring values.
 template <typename T>
-void predicate_bounds_t(const cs_predicate& pr, IfParams& p)
+void predicate_bounds_t(const cs_predicate& pr, SliceParams& p)
 {
     constexpr bool REAL = std::numeric_limits<T>::has_infinity;
     T a, b;
@@ -477,7 +505,7 @@ void predicate_bounds_t(const cs_predicate& pr, IfParams& p)
 }
 
 // Element width of a cs_elem_type and its bounds; 0 for an unknown type.
-uint32_t predicate_bounds(const cs_predicate& pr, IfParams& p)
+uint32_t predicate_bounds(const cs_predicate& pr, SliceParams& p)
 {
     switch (pr.type) {
         case CS_U8: predicate_bounds_t<uint8_t>(pr, p); return 1;
@@ -563,7 +591,7 @@ int compressstore_if(const void* d_in, void* d_out, uint64_t n, const cs_predica
 {
     if (!pred || !d_count) return CS_ERR_INVALID_VALUE;
     if (pred->op < CS_PRED_LT || pred->op > CS_PRED_BETWEEN) return CS_ERR_INVALID_VALUE;
-    IfParams p{};
+    SliceParams p{};
     const uint32_t w = predicate_bounds(*pred, p);
     if (w == 0) return CS_ERR_INVALID_VALUE;
     if (n > MAX_N) return CS_ERR_NOT_SUPPORTED;
@@ -575,7 +603,7 @@ int compressstore_if(const void* d_in, void* d_out, uint64_t n, const cs_predica
     DeviceInfo di;
     int st = current_device_info(&di);
     if (st) return st;
-    const size_t need = align256(sizeof(ws_header) + 8 * if_max_slices(n, w));
+    const size_t need = align256(sizeof(ws_header) + 8 * slices_of(n, w));
     void* ws = nullptr;
     size_t ws_bytes = 0;
     st = cached_workspace(need, s, &ws, &ws_bytes);

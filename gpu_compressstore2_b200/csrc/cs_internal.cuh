@@ -574,20 +574,22 @@ struct BlockScanParams {
     uint64_t keep_end;        // preserved by the epoch-wrap clear
 };
 
-// Predicate compaction (cs_predicate.cu). lo, hi: bit patterns of the element type in their low
+// Predicate compaction and the 1-pass form of the plain call (cs_slices.cu). lo, hi: bit patterns of the element type in their low
 // bytes; whole numbers: the lower bound and the distance to the upper one, modulo the width.
-struct IfParams {
+struct SliceParams {
     const uint8_t* in;
     uint8_t* out;
-    uint32_t* mask;      // null, or where the selection's words go
+    uint32_t* mask;      // comparison: null, or where the selection's words go
+    const uint32_t* mask_in; // 1-pass form: the selection (no comparison)
     uint64_t n;
     uint64_t* d_count;
     ws_header* hdr;
-    uint64_t* status;    // if_max_slices words
+    uint64_t* status;    // slices_of words
     uint64_t lo, hi;
     uint64_t timeout_ns;
     uint32_t negate;
     uint32_t sides;      // floating numbers: 1 only a lower bound, 2 only an upper one, 3 both
+    uint32_t grid;       // CTAs; 0: one resident wave
     uint32_t num_slices; // set by the launcher
 };
 
@@ -707,8 +709,10 @@ constexpr uint32_t FUSED_TILE_CHUNKS = 64; // 4096-element chunks per reduce-the
 static_assert(FUSED_TILE_CHUNKS * 4096u == (1u << SCAN_BLOCK_LOG2), "a plan tile is one scan block");
 cudaError_t launch_popc_blocks(const BlockScanParams& p, int num_sms, cudaStream_t stream);
 // Predicate compaction; 16-byte aligned pointers.
-cudaError_t launch_if(const IfParams& p, int type, int num_sms, cudaStream_t stream);
-uint64_t if_max_slices(uint64_t n, uint32_t elem_bytes); // look-back statuses it may use
+cudaError_t launch_if(const SliceParams& p, int type, int num_sms, cudaStream_t stream);
+// 1-pass form of the plain call (mask_in set): input 16-byte aligned, mask 4-byte, output by element.
+cudaError_t launch_onepass(const SliceParams& p, uint32_t elem_bytes, int num_sms, cudaStream_t stream);
+uint64_t slices_of(uint64_t n, uint32_t elem_bytes); // status words of either
 __host__ __device__ constexpr uint64_t sparse_items_for(uint64_t n)
 {
     return ((n + 1023) / 1024 + 15) / 16; // items of 16 blocks of 1024 elements

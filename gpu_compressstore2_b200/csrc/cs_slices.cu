@@ -1,20 +1,22 @@
-// cs_predicate.cu — predicate compaction (compressstore_if): the selection is a comparison
-// evaluated on the payload, in one kernel that reads the payload from HBM once.
+// cs_slices.cu — compaction in one kernel and one pass over HBM, for predicate compaction
+// (compressstore_if: the selection is a comparison evaluated on the payload) and for the 1-pass form of
+// the plain call (the selection is a mask in memory).
 //
 // The column is cut into slices of 32 KB: 8 warps x an item of 4 KB (cs_place.cuh). CTAs take slices
 // in order from a device counter and work two slices ahead of themselves. In each turn a CTA
-//   evaluates the slice two turns ahead: loads its payload, keeps its mask bits in registers and
-//             publishes its count; the payload itself is dropped and stays in L2;
+//   evaluates the slice two turns ahead: loads its mask, or its payload to compare, keeps the mask bits
+//             in registers and publishes their count; a compared payload is dropped and stays in L2;
 //   sums      the counts of the slices between its last one and the present one (about one per
 //             CTA; published two turns ago, so it rarely waits): with the selected elements
 //             before its last slice, which it carries along, that is the present slice's offset;
-//   writes    the present slice: loads the payload again, now from L2, places and stores the
-//             selected elements (an item with few is listed and gathered instead).
+//   writes    the present slice: loads the payload (a comparison's again, now from L2), places and
+//             stores the selected elements (an item with few is listed and gathered instead).
 // The warps of a CTA meet at one barrier per turn. A CTA only ever waits for slices that running
 // CTAs already hold, in order. Waits are bounded; one that gives up records an error, the CTA
-// writes nothing more and the count reads CS_COUNT_ERROR.
+// writes nothing more and the count reads CS_COUNT_ERROR. The epoch closes as soon as the last CTA
+// has summed up for the last time, so nothing follows the writes (2^20 u32: 7.1 -> 5.4 us).
 //
-// What bounds it is instructions: the evaluation and the placing together take about as long as
+// What bounds the predicate is instructions: the evaluation and the placing together take about as long as
 // 16 warps' issue of an SM allows while the payload streams at 4 to 5 TB/s. Per call on B200
 // against a mask pass, pass 1 + 2 and the writeout, which read the payload from HBM twice, before ->
 // now: 2^28 f32 x > c with 0.5 selected 459 -> 328 us, 0.01 259 -> 227, 0.1 414 -> 274, 0.9 556 -> 410;
@@ -22,7 +24,8 @@
 // Tried: a look-back over slices instead of the carried sum (it grows with the number of slices: 494
 // us at the best slice size), evaluating one slice ahead (365), slices of two items per warp
 // (374 .. 384), 2 and 4 CTAs per SM (408, 378), the evaluated payload through shared memory by bulk
-// copies (377).
+// copies (377). The 1-pass form's figures stand at SLICES_PER_SM in cs_api.cu; what bounds it is the
+// start (ticket, mask, payload one after another) for short columns and the barrier for long ones.
 //
 // A comparison of whole numbers is (x - lo) <= (hi - lo) in unsigned arithmetic, whatever the sign
 // (the host turns each operator into bounds), one of floating numbers lo <= x && x <= hi; != is the
@@ -61,7 +64,7 @@ __device__ __forceinline__ T from_bits(uint64_t b)
 }
 
 // Which bounds a comparison of floating numbers has (whole numbers take both in one).
-enum Sides { FROM = 1, TO = 2, BOTH = 3 };
+enum Sides { FROM = 1, TO = 2, BOTH = 3, MASK = 4 }; // MASK: no comparison, the selection is a mask in memory
 
 // Selected elements of a lane's 32 bytes, as bits.
 template <typename T, int SIDES>
@@ -93,12 +96,13 @@ __device__ __forceinline__ uint32_t select_row(const uint32_t (&x)[8], T lo, T h
 
 // T: uint8_t .. uint64_t (bounds lo and hi - lo), float, double (bounds lo, hi).
 template <typename T, int SIDES>
-__global__ void __launch_bounds__(WARPS * 32, CTAS) k_if(const IfParams p)
+__global__ void __launch_bounds__(WARPS * 32, CTAS) k_if(const SliceParams p)
 {
     constexpr uint32_t EPL = LANE_BYTES / sizeof(T);
     constexpr uint32_t ROW = 32 * EPL;
     constexpr uint32_t ITEM = ROWS * ROW;
     constexpr uint32_t VEC = 16 / sizeof(T);
+    constexpr bool MASKED = SIDES == MASK;
     constexpr int PK = EPL * ROWS > 32 ? EPL * ROWS / 32 : 1; // words that hold a lane's bits of an item
     constexpr uint32_t ROW_BITS = EPL == 32 ? 0xffffffffu : (1u << (EPL & 31u)) - 1u;
     __shared__ __align__(128) uint8_t s_stage[WARPS][STAGE_BYTES];
@@ -169,7 +173,23 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS) k_if(const IfParams p)
         }
     };
     // evaluates it into b; the last warp to do so publishes the slice's total
-    auto evaluate = [&](uint32_t slice, const uint32_t (&x)[ROWS][8], uint32_t (&b)[PK], uint32_t turn) {
+    // the mask bits of this warp's part of a slice
+    auto load_bits = [&](uint32_t slice, uint32_t (&m)[ROWS]) {
+        const uint64_t e0 = item_elem(slice);
+        const uint8_t* mb = reinterpret_cast<const uint8_t*>(p.mask_in);
+#pragma unroll
+        for (uint32_t r = 0; r < ROWS; ++r) {
+            const uint64_t e = e0 + r * ROW + lane * EPL;
+            uint32_t v = 0;
+            if (e < n) {
+                if constexpr (EPL == 32) v = __ldg(reinterpret_cast<const uint32_t*>(mb + (e >> 3)));
+                else if constexpr (EPL == 16) v = __ldg(reinterpret_cast<const uint16_t*>(mb + (e >> 3)));
+                else v = __ldg(mb + (e >> 3));
+            }
+            m[r] = v;
+        }
+    };
+    auto evaluate = [&](uint32_t slice, const uint32_t (&m)[ROWS], const uint32_t (&x)[ROWS][8], uint32_t (&b)[PK], uint32_t turn) {
         const uint64_t e0 = item_elem(slice);
         const bool whole = e0 + ITEM <= n;
         uint32_t cnt = 0;
@@ -177,7 +197,10 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS) k_if(const IfParams p)
         for (int q = 0; q < PK; ++q) b[q] = 0;
 #pragma unroll
         for (uint32_t r = 0; r < ROWS; ++r) {
-            uint32_t s = select_row<T, SIDES>(x[r], lo, hi) ^ negate;
+            uint32_t s;
+            if constexpr (!MASKED) s = select_row<T, SIDES>(x[r], lo, hi) ^ negate;
+            else if constexpr (EPL == 4) s = (m[r] >> ((lane & 1u) * 4)) & 0xfu;
+            else s = m[r];
             if (!whole) {
                 const uint64_t e = e0 + r * ROW + lane * EPL;
                 if (e + EPL > n) s = e < n ? s & ((1u << (n - e)) - 1u) : 0u; // n - e < EPL <= 32
@@ -195,7 +218,7 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS) k_if(const IfParams p)
                 st_relaxed_gpu(&p.status[slice], pack_status(epoch, FLAG_AGG, (before & 0xffffffu) + cnt));
             }
         }
-        if (p.mask) {
+        if (!MASKED && p.mask) {
             // the lane's bits of the mask words that hold an element of the column
             const uint64_t bound = (n + 31) / 32 * 32;
 #pragma unroll
@@ -220,31 +243,75 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS) k_if(const IfParams p)
     uint64_t end = 0;  // selected elements before slice `done`
     uint32_t done = 0; // the slices up to this CTA's last one
     uint32_t turn = 0;
-    // The first two slices. A CTA takes each slice only when it is about to evaluate it (or, in the
-    // loop, a turn before), so that the CTAs' slices interleave: a slice in front of another CTA's
-    // is evaluated no later than that one.
+    // The first two slices, evaluated before any wait. A CTA takes each slice only when it is about to
+    // evaluate it (or, in the loop, a turn before), so that the CTAs' slices interleave: a slice in front
+    // of another CTA's is evaluated no later than that one.
 #pragma unroll
     for (uint32_t t = 0; t < 2; ++t) {
         const uint32_t slice = s_slice[t];
         const bool some = slice < p.num_slices;
         if (some) {
-            uint32_t x[ROWS][8];
-            load_item(slice, x);
-            if (t == 0) evaluate(slice, x, bits, 0);
-            else evaluate(slice, x, bits1, 1);
+            uint32_t x[ROWS][8], m[ROWS];
+            if constexpr (MASKED) load_bits(slice, m);
+            else load_item(slice, x);
+            if (t == 0) evaluate(slice, m, x, bits, 0);
+            else evaluate(slice, m, x, bits1, 1);
         }
-        if (threadIdx.x == 0) s_slice[t + 1] = some ? atomicAdd(&p.hdr->tile_counter, 1u) : slice;
+        // (no second slice to ask for where every CTA has one)
+        if (threadIdx.x == 0)
+            s_slice[t + 1] = some && p.num_slices > gridDim.x ? atomicAdd(&p.hdr->tile_counter, 1u) : p.num_slices;
         __syncthreads();
     }
+    // Thread 0 of every CTA, once its CTA has summed up for the last time: the last one to come closes the
+    // epoch, and takes the count back if a wait gave up anywhere.
+    auto leave = [&]() {
+        if (atomicAdd(&p.hdr->done_counter, 1u) != gridDim.x - 1) return;
+        volatile ws_header* vh = p.hdr;
+        if (vh->poison_epoch == epoch) *p.d_count = COUNT_ERROR;
+        uint32_t following = epoch + 1u;
+        if (following > EPOCH_MAX) {
+            uint4* w = reinterpret_cast<uint4*>(p.hdr);
+            for (uint64_t i = sizeof(ws_header) / 16u; i < vh->ws_bytes / 16u; ++i) w[i] = make_uint4(0, 0, 0, 0);
+            vh->poison_epoch = 0u; // a new cycle must not meet an old one's mark
+            following = EPOCH_MIN;
+        }
+        vh->tile_counter = 0u;
+        vh->done_counter = 0u;
+        vh->epoch = following;
+    };
+    if (threadIdx.x == 0 && s_slice[0] >= p.num_slices) leave();
     while (true) {
         const uint32_t slice = s_slice[turn];
         if (slice >= p.num_slices) break;
         const uint32_t later = (turn + 2) & 3u;
-        const uint32_t next = s_slice[later]; // the slice to evaluate in this turn
+        const uint32_t next = s_slice[later]; // to be evaluated in this turn
         uint32_t ahead[PK];
         uint32_t x[ROWS][8];
         const bool more = next < p.num_slices;
-        if (more) load_item(next, x);
+        const uint64_t e0 = item_elem(slice);
+        const uint32_t mine = s_total[turn][warp];
+        const bool few = mine <= FEW;
+        // This warp's item of the slice (of a comparison: from L2): few selected elements are listed and
+        // gathered, otherwise the lanes with selected elements load theirs.
+        auto load_selected = [&]() {
+            if (few) return;
+            if (e0 + ITEM <= n) {
+                const uint8_t* src = in + e0 * sizeof(T) + lane * LANE_BYTES;
+#pragma unroll
+                for (uint32_t r = 0; r < ROWS; ++r)
+                    if (row_bits(bits, r)) load_whole(src + r * ROW_BYTES, x[r]);
+            } else {
+#pragma unroll
+                for (uint32_t r = 0; r < ROWS; ++r)
+                    if (row_bits(bits, r)) load_ragged(e0, r, x[r]);
+            }
+        };
+        if constexpr (MASKED) load_selected();
+        uint32_t m[ROWS];
+        if (more) {
+            if constexpr (MASKED) load_bits(next, m);
+            else load_item(next, x);
+        }
         if (threadIdx.x == 0) s_slice[(turn + 3) & 3u] = more ? atomicAdd(&p.hdr->tile_counter, 1u) : next;
         // the totals of the slices since this CTA's last one, 512 at a time
         uint32_t* const red = s_red[turn & 1u];
@@ -256,24 +323,8 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS) k_if(const IfParams p)
             __syncthreads();
         }
         if (!poll_totals<WARPS * 32>(p.status, done, slice, epoch, s_failed ? 0ull : p.timeout_ns, red)) s_failed = 1u;
-        if (more) evaluate(next, x, ahead, later);
-        // The present slice's item, from L2: few selected elements are listed and gathered, otherwise
-        // the lanes with selected elements load theirs
-        const uint64_t e0 = item_elem(slice);
-        const uint32_t mine = s_total[turn][warp];
-        const bool few = mine <= FEW;
-        if (!few) {
-            if (e0 + ITEM <= n) {
-                const uint8_t* src = in + e0 * sizeof(T) + lane * LANE_BYTES;
-#pragma unroll
-                for (uint32_t r = 0; r < ROWS; ++r)
-                    if (row_bits(bits, r)) load_whole(src + r * ROW_BYTES, x[r]);
-            } else {
-#pragma unroll
-                for (uint32_t r = 0; r < ROWS; ++r)
-                    if (row_bits(bits, r)) load_ragged(e0, r, x[r]);
-            }
-        }
+        if (more) evaluate(next, m, x, ahead, later);
+        if constexpr (!MASKED) load_selected();
         __syncthreads(); // the sums of this turn; every warp has left the turn before
         const uint4 t0 = lds128(s_total[turn]), t1 = lds128(s_total[turn] + 4);
         const uint4 r0 = lds128(red), r1 = lds128(red + 4);
@@ -287,6 +338,10 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS) k_if(const IfParams p)
                 reinterpret_cast<volatile ws_header*>(p.hdr)->poison_epoch = epoch;
             }
             if (slice == p.num_slices - 1) *p.d_count = end;
+            if (s_slice[(turn + 1) & 3u] >= p.num_slices) { // the CTA's last slice
+                if (failed || slice == p.num_slices - 1) __threadfence(); // the mark, the count before `leave`
+                leave();
+            }
         }
         if (!failed && mine != 0u) {
             const uint64_t off = base + (warp > 0 ? t0.x : 0u) + (warp > 1 ? t0.y : 0u) + (warp > 2 ? t0.z : 0u) + (warp > 3 ? t0.w : 0u) +
@@ -331,32 +386,27 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS) k_if(const IfParams p)
             bits1[q] = ahead[q];
         }
     }
-    // the last CTA closes the epoch, and takes the count back if a wait gave up anywhere
-    __shared__ uint32_t s_flag;
-    if (epilogue_ticket(&p.hdr->done_counter, &s_flag)) {
-        if (threadIdx.x == 0 && reinterpret_cast<volatile ws_header*>(p.hdr)->poison_epoch == epoch) *p.d_count = COUNT_ERROR;
-        epilogue_last(p.hdr, &p.hdr->tile_counter, &p.hdr->done_counter, false, 0, 0, nullptr);
-    }
 }
 
 template <typename T, int SIDES>
-cudaError_t launch_s(const IfParams& p, int num_sms, cudaStream_t stream)
+cudaError_t launch_s(const SliceParams& p, int num_sms, cudaStream_t stream)
 {
-    IfParams q = p;
-    q.num_slices = static_cast<uint32_t>(if_max_slices(p.n, sizeof(T)));
-    uint64_t grid = static_cast<uint64_t>(num_sms) * CTAS;
+    SliceParams q = p;
+    q.num_slices = static_cast<uint32_t>(slices_of(p.n, sizeof(T)));
+    uint64_t grid = p.grid ? p.grid : static_cast<uint64_t>(num_sms) * CTAS;
     if (grid > q.num_slices) grid = q.num_slices;
     return launch_pdl(k_if<T, SIDES>, dim3(static_cast<unsigned>(grid)), dim3(WARPS * 32), 0, stream, q);
 }
 
 template <typename T>
-cudaError_t launch_t(const IfParams& p, int num_sms, cudaStream_t stream)
+cudaError_t launch_t(const SliceParams& p, int num_sms, cudaStream_t stream)
 {
+    if (p.mask_in) return launch_s<T, MASK>(p, num_sms, stream);
     return launch_s<T, BOTH>(p, num_sms, stream);
 }
 
 template <typename T>
-cudaError_t launch_real(const IfParams& p, int num_sms, cudaStream_t stream)
+cudaError_t launch_real(const SliceParams& p, int num_sms, cudaStream_t stream)
 {
     if (p.sides == FROM) return launch_s<T, FROM>(p, num_sms, stream);
     if (p.sides == TO) return launch_s<T, TO>(p, num_sms, stream);
@@ -365,13 +415,13 @@ cudaError_t launch_real(const IfParams& p, int num_sms, cudaStream_t stream)
 
 } // namespace
 
-uint64_t if_max_slices(uint64_t n, uint32_t elem_bytes)
+uint64_t slices_of(uint64_t n, uint32_t elem_bytes)
 {
     const uint64_t items = (n * elem_bytes + ITEM_BYTES - 1) / ITEM_BYTES;
     return (items + WARPS - 1) / WARPS;
 }
 
-cudaError_t launch_if(const IfParams& p, int type, int num_sms, cudaStream_t stream)
+cudaError_t launch_if(const SliceParams& p, int type, int num_sms, cudaStream_t stream)
 {
     cudaError_t e;
     switch (type) {
@@ -385,6 +435,20 @@ cudaError_t launch_if(const IfParams& p, int type, int num_sms, cudaStream_t str
         case CS_I64: e = launch_t<uint64_t>(p, num_sms, stream); break;
         case CS_F32: e = launch_real<float>(p, num_sms, stream); break;
         case CS_F64: e = launch_real<double>(p, num_sms, stream); break;
+        default: return cudaErrorInvalidValue;
+    }
+    note_launch();
+    return e;
+}
+
+cudaError_t launch_onepass(const SliceParams& p, uint32_t elem_bytes, int num_sms, cudaStream_t stream)
+{
+    cudaError_t e;
+    switch (elem_bytes) {
+        case 1: e = launch_t<uint8_t>(p, num_sms, stream); break;
+        case 2: e = launch_t<uint16_t>(p, num_sms, stream); break;
+        case 4: e = launch_t<uint32_t>(p, num_sms, stream); break;
+        case 8: e = launch_t<uint64_t>(p, num_sms, stream); break;
         default: return cudaErrorInvalidValue;
     }
     note_launch();
