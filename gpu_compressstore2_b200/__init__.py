@@ -48,10 +48,22 @@ def _torch():
     return torch
 
 
+_current_raw_stream = None  # () -> handle of the current device's current stream, once CUDA is up
+
+
 def _stream_handle(stream) -> int | None:
-    torch = _torch()
+    """cudaStream_t of a torch stream, a handle, or (None) the current stream. The current stream is asked
+    of torch's binding directly: torch.cuda.current_stream builds a Stream object per call, 3.5 us of
+    the 9 us that a short call took; 0.3 us this way."""
+    global _current_raw_stream
     if stream is None:
-        stream = torch.cuda.current_stream()
+        if _current_raw_stream is None:
+            torch = _torch()
+            handle = torch.cuda.current_stream().cuda_stream  # initialises CUDA
+            raw, device = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
+            _current_raw_stream = lambda: raw(device())  # noqa: E731
+            return handle or None
+        return _current_raw_stream() or None
     if isinstance(stream, int):
         return stream or None
     return stream.cuda_stream or None
@@ -90,16 +102,16 @@ def compressstore(d_in, d_mask, d_out, n: int, d_count, *, algo: int = ALGO_AUTO
     selectivity bucket."""
     w = d_in.element_size()
     s = _stream_handle(stream)
-    cfg = make_config(algo, chunk_length, grid_dim, skip, timeout_ns, selectivity)
-    if workspace is None:
-        if algo == ALGO_AUTO and not (chunk_length or grid_dim or skip or timeout_ns or selectivity):
-            st = lib().compressstore(_ptr(d_in), _ptr(d_mask), _ptr(d_out), n, w, _ptr(d_count), s)
-        else:
+    if workspace is None and algo == ALGO_AUTO and not (chunk_length or grid_dim or skip or timeout_ns or selectivity):
+        st = lib().compressstore(_ptr(d_in), _ptr(d_mask), _ptr(d_out), n, w, _ptr(d_count), s)
+    else:
+        cfg = make_config(algo, chunk_length, grid_dim, skip, timeout_ns, selectivity)
+        if workspace is None:
             st = lib().compressstore_cfg(_ptr(d_in), _ptr(d_mask), _ptr(d_out), n, w, _ptr(d_count),
                                          ctypes.byref(cfg), s)
-    else:
-        st = lib().compressstore_ex(_ptr(d_in), _ptr(d_mask), _ptr(d_out), n, w, _ptr(d_count),
-                                    workspace.ptr, workspace.nbytes, ctypes.byref(cfg), s)
+        else:
+            st = lib().compressstore_ex(_ptr(d_in), _ptr(d_mask), _ptr(d_out), n, w, _ptr(d_count),
+                                        workspace.ptr, workspace.nbytes, ctypes.byref(cfg), s)
     check(st, "compressstore")
 
 
