@@ -595,16 +595,19 @@ struct SliceParams {
 
 // Last CTA of a reduce-then-scan pass (all 256 threads): turns the block sums into the
 // exclusive prefix of every block within its column (blk_base) and writes every column's
-// count, or CS_COUNT_ERROR when the pass is not `clean`. s_scan: 8 words of shared memory.
-__device__ __forceinline__ void blocks_last_cta(const BlockScanParams& p, uint64_t* s_scan, bool clean)
+// count, or CS_COUNT_ERROR when the pass is not `clean`. s_scan: 8 words of shared memory; s_prefix:
+// prefix_room more, in which a plan's blocks, if they are no more, keep their flat prefixes.
+__device__ __forceinline__ void blocks_last_cta(const BlockScanParams& p, uint64_t* s_scan, bool clean,
+                                                uint64_t* s_prefix, uint64_t prefix_room)
 {
     const uint32_t tid = threadIdx.x;
     const uint32_t lane = tid & 31u;
     const uint32_t warp = tid >> 5;
-    // flat exclusive scan of the block sums (ascending, into blk_base); a thread takes V
+    // flat exclusive scan of the block sums (ascending, into blk_base or s_prefix); a thread takes V
     // consecutive sums per round so up to 1024 blocks (2^28 elements) need one round
     constexpr uint32_t V = 4;
     const uint64_t T = p.num_blocks;
+    const bool kept = p.cols && T <= prefix_room;
     uint64_t carry = 0;
     for (uint64_t base = 0; base < T; base += 256 * V) {
         const uint64_t t0 = base + static_cast<uint64_t>(tid) * V;
@@ -626,11 +629,42 @@ __device__ __forceinline__ void blocks_last_cta(const BlockScanParams& p, uint64
         }
 #pragma unroll
         for (uint32_t k = 0; k < V; ++k) {
-            if (t0 + k < T) p.blk_base[t0 + k] = run;
+            if (t0 + k < T) {
+                if (kept) s_prefix[t0 + k] = run;
+                else p.blk_base[t0 + k] = run;
+            }
             run += v[k];
         }
         carry += tot;
         __syncthreads();
+    }
+    if (kept) {
+        // every block's prefix from its column's first block, and each column's count at its last block,
+        // independently of one another
+        for (uint64_t base = 0; base < T; base += 256 * V) {
+            uint32_t ci[V];
+            uint64_t first[V], len[V];
+            uint64_t* out[V];
+#pragma unroll
+            for (uint32_t k = 0; k < V; ++k) ci[k] = base + k * 256 + tid < T ? __ldg(p.blk_col + base + k * 256 + tid) : 0u;
+#pragma unroll
+            for (uint32_t k = 0; k < V; ++k) {
+                first[k] = p.cols[ci[k]].tile_base;
+                len[k] = p.cols[ci[k]].n;
+                out[k] = p.cols[ci[k]].d_count;
+            }
+#pragma unroll
+            for (uint32_t k = 0; k < V; ++k) {
+                const uint64_t t = base + k * 256 + tid;
+                if (t >= T) continue;
+                const uint64_t before = s_prefix[first[k]];
+                p.blk_base[t] = s_prefix[t] - before;
+                const uint64_t col_blocks = (len[k] + (1ull << SCAN_BLOCK_LOG2) - 1) >> SCAN_BLOCK_LOG2;
+                if (t - first[k] == col_blocks - 1)
+                    *out[k] = clean ? (t + 1 < T ? s_prefix[t + 1] : carry) - before : COUNT_ERROR;
+            }
+        }
+        return;
     }
     if (!p.cols) {
         // one column: its first block is block 0, so the flat prefixes are final

@@ -258,7 +258,8 @@ cudaError_t launch_scan(const ScanParams& p, int num_sms, cudaStream_t stream)
 // one epoch cycle ago costs the gather one test of the offsets, never a wrong write).
 // s_warp / s_whalf: selected elements in each warp's 8 rows and in their first 4 rows.
 // Called by all threads after those are written.
-__device__ __forceinline__ void mark_sparse_units(const BlockScanParams& p, const ColumnDesc& col, uint64_t bl,
+template <typename Col>
+__device__ __forceinline__ void mark_sparse_units(const BlockScanParams& p, const Col& col, uint64_t bl,
                                                   const uint32_t* s_warp, const uint32_t* s_whalf, uint32_t epoch)
 {
     const uint32_t w = col.elem_bytes;
@@ -294,37 +295,79 @@ __device__ __forceinline__ void mark_sparse_units(const BlockScanParams& p, cons
 // src/kernels/kernel_3pass.cuh:59-214).
 // ---------------------------------------------------------------------------------
 
-// This warp's 8 rows (32 uint4 each) of block `bl` of `col`, read from global memory: the
-// last word of the column has its bits past n cleared, and words past the column read 0. A mask
-// that starts inside a 16-byte group (4-byte aligned) is read word by word.
-__device__ __forceinline__ void popc_block_load(const ColumnDesc& col, uint64_t bl, uint32_t warp, uint32_t lane,
-                                                uint4 (&q)[8])
+// A block's share of its column's mask: `words` words, of which the first 4 * groups are whole
+// 16-byte groups that can be read as such (none where the mask starts inside a group).
+struct PopcShare {
+    uint32_t words;
+    uint32_t groups;
+    uint32_t last_bits; // bits of the last word, 0 if all 32
+};
+
+template <typename Col>
+__device__ __forceinline__ PopcShare popc_share(const Col& col, uint64_t bl)
 {
-    const uint64_t n = col.n;
-    const uint64_t nw = (n + 31) / 32;
-    const uint32_t* __restrict__ mask = col.mask;
-    const uint4* mv = reinterpret_cast<const uint4*>(mask);
-    const uint64_t row0 = bl * 64 + warp * 8; // this warp's first row (4096 elements each)
-    const bool vec = (reinterpret_cast<uintptr_t>(mask) & 15u) == 0;
+    const uint64_t left = col.n - (bl << SCAN_BLOCK_LOG2);
+    if (left >= (1ull << SCAN_BLOCK_LOG2)) {
+        constexpr uint32_t WORDS = (1u << SCAN_BLOCK_LOG2) / 32;
+        return {WORDS, (reinterpret_cast<uintptr_t>(col.mask) & 15u) == 0 ? WORDS / 4 : 0u, 0u};
+    }
+    const uint32_t l = static_cast<uint32_t>(left);
+    const uint32_t words = (l + 31u) / 32u;
+    return {words, (reinterpret_cast<uintptr_t>(col.mask) & 15u) == 0 ? words / 4u : 0u, l & 31u};
+}
+
+// The end of a column's mask, once its whole groups are in q and the rest of q is 0: the words past
+// the last whole group are read one by one, and the bits past the column's end cleared.
+__device__ __forceinline__ void popc_mask_end(const uint32_t* words, const PopcShare& sh, uint32_t warp, uint32_t lane,
+                                              uint4 (&q)[8])
+{
+    const uint32_t g = (sh.words - 1u) / 4u; // the group with the last word
+    if (g / 256u != warp || (g & 31u) != lane) return;
+    uint32_t w4[4];
 #pragma unroll
-    for (int r = 0; r < 8; ++r) {
-        const uint64_t vi = (row0 + r) * 32 + lane;
-        if (vec && vi * 4 + 3 < nw) {
-            q[r] = __ldg(mv + vi);
-            if (vi * 4 + 3 == nw - 1 && (n & 31u)) q[r].w &= (1u << (n & 31u)) - 1u;
-        } else {
-            uint32_t w4[4];
+    for (uint32_t k = 0; k < 4; ++k) w4[k] = (g >= sh.groups && 4 * g + k < sh.words) ? __ldg(words + 4 * g + k) : 0u;
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const uint64_t wi = vi * 4 + k;
-                w4[k] = 0;
-                if (wi < nw) {
-                    w4[k] = __ldg(mask + wi);
-                    if (wi == nw - 1 && (n & 31u)) w4[k] &= (1u << (n & 31u)) - 1u;
-                }
-            }
-            q[r] = make_uint4(w4[0], w4[1], w4[2], w4[3]);
+    for (uint32_t r = 0; r < 8; ++r) {
+        if ((g / 32u) % 8u != r) continue;
+        if (g >= sh.groups) q[r] = make_uint4(w4[0], w4[1], w4[2], w4[3]);
+        const uint32_t keep = sh.last_bits ? (1u << sh.last_bits) - 1u : 0xffffffffu;
+        const uint32_t last = (sh.words - 1u) & 3u;
+        if (last == 0) q[r].x &= keep;
+        if (last == 1) q[r].y &= keep;
+        if (last == 2) q[r].z &= keep;
+        if (last == 3) q[r].w &= keep;
+    }
+}
+
+// This warp's 8 rows (32 uint4 each) of block `bl` of `col`, read from global memory: bits and words
+// past the column's end read 0. All loads are in flight together (at a column's end too: a branch
+// per row made the last block of a column wait for its rows one after another). A mask that starts
+// inside a 16-byte group (4-byte aligned) is read word by word.
+template <typename Col>
+__device__ __forceinline__ void popc_block_load(const Col& col, uint64_t bl, const PopcShare& sh, uint32_t warp,
+                                                uint32_t lane, uint4 (&q)[8])
+{
+    const uint32_t* __restrict__ words = col.mask + bl * ((1u << SCAN_BLOCK_LOG2) / 32);
+    if ((reinterpret_cast<uintptr_t>(col.mask) & 15u) == 0) {
+#pragma unroll
+        for (uint32_t r = 0; r < 8; ++r) {
+            const uint32_t v = (warp * 8 + r) * 32 + lane;
+            q[r] = make_uint4(0u, 0u, 0u, 0u);
+            if (v < sh.groups) q[r] = __ldg(reinterpret_cast<const uint4*>(words) + v);
         }
+        if (4u * sh.groups != sh.words || sh.last_bits) popc_mask_end(words, sh, warp, lane, q);
+        return;
+    }
+#pragma unroll
+    for (uint32_t r = 0; r < 8; ++r) {
+        uint32_t w4[4];
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k) {
+            const uint32_t w = ((warp * 8 + r) * 32 + lane) * 4 + k;
+            w4[k] = w < sh.words ? __ldg(words + w) : 0u;
+            if (w == sh.words - 1u && sh.last_bits) w4[k] &= (1u << sh.last_bits) - 1u;
+        }
+        q[r] = make_uint4(w4[0], w4[1], w4[2], w4[3]);
     }
 }
 
@@ -332,8 +375,8 @@ __device__ __forceinline__ void popc_block_load(const ColumnDesc& col, uint64_t 
 // the block sum, the sparse hint (sparse_seen) and, in the hybrid form, the sparse-unit
 // marks. Called by all 256 threads; returns after a barrier, so s_warp may be rewritten.
 // s_epoch (written by thread 0 before its first call) is read after the first barrier here.
-template <int LPC>
-__device__ __forceinline__ void popc_block_finish(const BlockScanParams& p, const ColumnDesc& col, uint64_t blk,
+template <int LPC, typename Col>
+__device__ __forceinline__ void popc_block_finish(const BlockScanParams& p, const Col& col, uint64_t blk,
                                                   uint64_t bl, const uint4 (&q)[8], uint32_t* s_warp,
                                                   uint32_t* s_whalf, const uint32_t* s_epoch, bool& sparse_seen)
 {
@@ -396,7 +439,8 @@ __device__ __forceinline__ void popc_block_finish(const BlockScanParams& p, cons
 // saw a sparse block (no flag array to read). The last CTA scans the block sums and closes
 // the epoch; the call's scan is marked clean unless a CTA poisoned this epoch.
 __device__ __forceinline__ void popc_blocks_finish_grid(const BlockScanParams& p, bool sparse_seen,
-                                                        const uint32_t* s_epoch, uint32_t* s_flag, uint64_t* s_scan)
+                                                        const uint32_t* s_epoch, uint32_t* s_flag, uint64_t* s_scan,
+                                                        uint64_t* s_prefix, uint64_t prefix_room)
 {
     const uint32_t tid = threadIdx.x;
     const bool cta_sparse = __syncthreads_or(sparse_seen) != 0;
@@ -412,7 +456,7 @@ __device__ __forceinline__ void popc_blocks_finish_grid(const BlockScanParams& p
     if (!(fin & 1u)) return;
     __threadfence(); // every other CTA's block sums (and any poison mark) are visible
     const bool clean = reinterpret_cast<volatile ws_header*>(p.hdr)->poison_epoch != epoch;
-    blocks_last_cta(p, s_scan, clean);
+    blocks_last_cta(p, s_scan, clean, s_prefix, prefix_room);
     epilogue_last_blocks(p.hdr, epoch, (fin & 2u) != 0u, p.keep_begin, p.keep_end, clean);
 }
 
@@ -422,6 +466,7 @@ __global__ void __launch_bounds__(256, 4) k_popc_blocks(const BlockScanParams p)
     __shared__ uint32_t s_warp[8];
     __shared__ uint32_t s_whalf[8];
     __shared__ uint64_t s_scan[8];
+    __shared__ uint64_t s_prefix[1024];
     __shared__ uint32_t s_flag;
     __shared__ uint32_t s_epoch;
     const uint32_t tid = threadIdx.x;
@@ -432,10 +477,10 @@ __global__ void __launch_bounds__(256, 4) k_popc_blocks(const BlockScanParams p)
         const ColumnDesc& col = column_of(p.col0, p.cols, p.blk_col, blk);
         const uint64_t bl = blk - col.tile_base; // block within its column
         uint4 q[8];
-        popc_block_load(col, bl, tid >> 5, tid & 31u, q);
+        popc_block_load(col, bl, popc_share(col, bl), tid >> 5, tid & 31u, q);
         popc_block_finish<LPC>(p, col, blk, bl, q, s_warp, s_whalf, &s_epoch, sparse_seen);
     }
-    popc_blocks_finish_grid(p, sparse_seen, &s_epoch, &s_flag, s_scan);
+    popc_blocks_finish_grid(p, sparse_seen, &s_epoch, &s_flag, s_scan, s_prefix, 1024);
 }
 
 // ---------------------------------------------------------------------------------
@@ -445,12 +490,15 @@ __global__ void __launch_bounds__(256, 4) k_popc_blocks(const BlockScanParams p)
 // blocks; thread 0 streams them through POPC_STAGES shared-memory stages of 32 KB with 1-D
 // bulk copies (cp.async.bulk, no multicast), so the next block of every CTA is in flight
 // while its warps count the current one. A stage is refilled once every warp has left the
-// block it held (the barrier that ends popc_block_finish). A block that is not whole (the
-// last block of a column whose length is not a multiple of 2^18) is read from global memory
-// as in k_popc_blocks. The per-block work and the end are those of k_popc_blocks.
+// block it held (the barrier that ends popc_block_finish). Of a column's last block the whole
+// 16-byte groups are copied, and the words after them (all words of a mask that starts inside such
+// a group) written into the stage by the threads. The per-block work and the end are those of k_popc_blocks.
 // The shape was measured on B200 at 2^28 f32 and 2^29 u8/u16 (3-pass calls, us per call):
 // 3 CTAs x 2 stages beat 1 x 6 (the counting of one CTA's 8 warps is latency-bound, so one
-// CTA per SM left the copies waiting on it), 2 x 3 and 4 x 1.
+// CTA per SM left the copies waiting on it), 2 x 3 and 4 x 1. All blocks are counted by the same
+// code out of the stage: with a second source (global memory, for a column's last block) the
+// registers of both met at the count, and the kernel, alone, took 39 us instead of 25 for the 1470
+// blocks of 256 uneven columns.
 // A stage wait that runs out records DEVERR_PIPELINE_TIMEOUT and poisons the call's scan;
 // the CTA then issues no further copies and waits (bounded) for the ones in flight.
 // ---------------------------------------------------------------------------------
@@ -466,6 +514,35 @@ constexpr uint32_t MASK_BLOCK_BYTES = (1u << SCAN_BLOCK_LOG2) / 8; // 32 KB of m
 constexpr uint64_t POPC_WAIT_NS = 2000000000ull; // bound on one stage wait (a copy lands in microseconds)
 constexpr uint32_t POPC_STREAM_SMEM = POPC_STAGES * MASK_BLOCK_BYTES;
 
+// What the copy left out of a block, into its stage: the words past the whole groups, with the bits
+// past the column's end cleared, and zeros after them. All 256 threads.
+__device__ __forceinline__ void popc_fill_rest(const uint32_t* words, const PopcShare& sh, uint4* stage)
+{
+    const uint32_t keep = sh.last_bits ? (1u << sh.last_bits) - 1u : 0xffffffffu;
+    uint32_t* sw = reinterpret_cast<uint32_t*>(stage);
+    constexpr uint32_t WORDS = MASK_BLOCK_BYTES / 4;
+    if (4u * sh.groups == sh.words && threadIdx.x == 0) sw[sh.words - 1u] &= keep;
+#pragma unroll 8
+    for (uint32_t w = 4u * sh.groups + threadIdx.x; w < WORDS; w += 256) {
+        uint32_t x = w < sh.words ? __ldg(words + w) : 0u;
+        if (w == sh.words - 1u) x &= keep;
+        sw[w] = x;
+    }
+}
+
+// What k_popc_stream needs of the column that a block belongs to. In a plan a CTA keeps these of its
+// next blocks in shared memory, read by all its threads at once: finding a block's column is two
+// dependent loads, which thread 0 otherwise made before each copy and every warp before each block.
+struct PopcBlock {
+    const uint32_t* mask;
+    uint64_t* offsets;
+    uint64_t n;
+    uint64_t bl; // block within its column
+    uint64_t item_base;
+    uint32_t elem_bytes;
+};
+constexpr uint32_t POPC_TABLE = 64; // blocks; refilled by halves
+
 template <int LPC>
 __global__ void __launch_bounds__(256, POPC_STREAM_CTAS) k_popc_stream(const BlockScanParams p)
 {
@@ -477,6 +554,7 @@ __global__ void __launch_bounds__(256, POPC_STREAM_CTAS) k_popc_stream(const Blo
     __shared__ uint32_t s_flag;
     __shared__ uint32_t s_epoch;
     __shared__ uint32_t s_fail;
+    __shared__ PopcBlock s_block[POPC_TABLE];
     const uint32_t tid = threadIdx.x;
     const uint32_t lane = tid & 31u;
     const uint32_t warp = tid >> 5;
@@ -488,19 +566,31 @@ __global__ void __launch_bounds__(256, POPC_STREAM_CTAS) k_popc_stream(const Blo
         s_fail = 0u;
     }
     grid_dependency_wait(); // the mask may come from the previous kernel, the workspace too
-    // a block is copied in bulk when all its bits lie inside its column and its mask is 16-byte aligned
-    auto whole = [&](const ColumnDesc& c, uint64_t bl) -> bool {
-        return ((bl + 1) << SCAN_BLOCK_LOG2) <= c.n && (reinterpret_cast<uintptr_t>(c.mask) & 15u) == 0;
+    // blocks [from, from + count) of this CTA into the table
+    auto describe = [&](uint64_t from, uint32_t count) {
+        if (tid >= count || from + tid >= b1) return;
+        const uint64_t blk = from + tid;
+        const ColumnDesc& c = p.cols[__ldg(p.blk_col + blk)];
+        s_block[(blk - b0) % POPC_TABLE] = PopcBlock{c.mask, c.offsets, c.n, blk - c.tile_base, c.item_base, c.elem_bytes};
     };
+    auto block_at = [&](uint64_t blk) -> PopcBlock {
+        if (p.cols) return s_block[(blk - b0) % POPC_TABLE];
+        return PopcBlock{p.col0.mask, p.col0.offsets, p.col0.n, blk, 0, p.col0.elem_bytes};
+    };
+    // a block's whole 16-byte groups are copied in bulk, if it has any
     uint32_t pending = 0; // thread 0: stages with a copy in flight
     auto issue = [&](uint64_t blk, uint32_t s) {
-        const ColumnDesc& c = column_of(p.col0, p.cols, p.blk_col, blk);
-        const uint64_t bl = blk - c.tile_base;
-        if (!whole(c, bl)) return;
-        mbar_arrive_expect_tx(&s_full[s], MASK_BLOCK_BYTES);
-        bulk_g2s(smem + s * MASK_BLOCK_BYTES, c.mask + bl * (MASK_BLOCK_BYTES / 4), MASK_BLOCK_BYTES, &s_full[s]);
+        const PopcBlock c = block_at(blk);
+        const uint32_t bytes = popc_share(c, c.bl).groups * 16u;
+        if (bytes == 0) return;
+        mbar_arrive_expect_tx(&s_full[s], bytes);
+        bulk_g2s(smem + s * MASK_BLOCK_BYTES, c.mask + c.bl * (MASK_BLOCK_BYTES / 4), bytes, &s_full[s]);
         pending |= 1u << s;
     };
+    if (p.cols) {
+        describe(b0, POPC_TABLE);
+        __syncthreads();
+    }
     if (tid == 0) {
         // the first copies go out before the header read (thread 0 initialised the barriers)
         for (uint32_t k = 0; k < POPC_STAGES && b0 + k < b1; ++k) issue(b0 + k, k);
@@ -513,29 +603,34 @@ __global__ void __launch_bounds__(256, POPC_STREAM_CTAS) k_popc_stream(const Blo
     for (uint64_t i = 0; b0 + i < b1; ++i) {
         const uint64_t blk = b0 + i;
         const uint32_t s = static_cast<uint32_t>(i % POPC_STAGES);
-        const ColumnDesc& col = column_of(p.col0, p.cols, p.blk_col, blk);
-        const uint64_t bl = blk - col.tile_base;
-        uint4 q[8];
-        if (whole(col, bl)) {
-            // after a failure no stage is refilled, so nothing more is waited for
-            if (*reinterpret_cast<volatile uint32_t*>(&s_fail) == 0u) {
-                if (mbar_wait_bounded(&s_full[s], (parity >> s) & 1u, POPC_WAIT_NS)) {
-                    parity ^= 1u << s;
-                    if (tid == 0) pending &= ~(1u << s);
-                } else {
-                    atomicOr(&s_fail, 1u);
-                    if (lane == 0) {
-                        record_error(p.hdr, DEVERR_PIPELINE_TIMEOUT);
-                        reinterpret_cast<volatile ws_header*>(p.hdr)->poison_epoch = epoch;
-                    }
+        const PopcBlock col = block_at(blk);
+        const uint64_t bl = col.bl;
+        // the half of the table whose blocks are done (the barrier ending popc_block_finish)
+        if (p.cols && i != 0 && i % (POPC_TABLE / 2) == 0) describe(blk + POPC_TABLE / 2, POPC_TABLE / 2);
+        const PopcShare sh = popc_share(col, bl);
+        uint4* sv = reinterpret_cast<uint4*>(smem + s * MASK_BLOCK_BYTES);
+        // after a failure no stage is refilled, so nothing more is waited for
+        if (sh.groups != 0u && *reinterpret_cast<volatile uint32_t*>(&s_fail) == 0u) {
+            if (mbar_wait_bounded(&s_full[s], (parity >> s) & 1u, POPC_WAIT_NS)) {
+                parity ^= 1u << s;
+                if (tid == 0) pending &= ~(1u << s);
+            } else {
+                atomicOr(&s_fail, 1u);
+                if (lane == 0) {
+                    record_error(p.hdr, DEVERR_PIPELINE_TIMEOUT);
+                    reinterpret_cast<volatile ws_header*>(p.hdr)->poison_epoch = epoch;
                 }
             }
-            const uint4* sv = reinterpret_cast<const uint4*>(smem + s * MASK_BLOCK_BYTES);
-#pragma unroll
-            for (int r = 0; r < 8; ++r) q[r] = sv[(warp * 8 + r) * 32 + lane];
-        } else {
-            popc_block_load(col, bl, warp, lane, q);
         }
+        // the rest of the block into the stage, so that all blocks are counted by the same code
+        if (sh.groups != MASK_BLOCK_BYTES / 16 || sh.last_bits != 0u) {
+            popc_fill_rest(col.mask + bl * (MASK_BLOCK_BYTES / 4), sh, sv);
+            fence_proxy_async(); // before the next copy into this stage
+            __syncthreads();
+        }
+        uint4 q[8];
+#pragma unroll
+        for (uint32_t r = 0; r < 8; ++r) q[r] = sv[(warp * 8 + r) * 32 + lane];
         popc_block_finish<LPC>(p, col, blk, bl, q, s_warp, s_whalf, &s_epoch, sparse_seen);
         // every warp has left stage s (the barrier ending popc_block_finish): refill it
         if (tid == 0 && b0 + i + POPC_STAGES < b1 && s_fail == 0u) issue(b0 + i + POPC_STAGES, s);
@@ -546,7 +641,8 @@ __global__ void __launch_bounds__(256, POPC_STREAM_CTAS) k_popc_stream(const Blo
         for (uint32_t s = 0; s < POPC_STAGES; ++s)
             if ((pending >> s) & 1u) mbar_wait_bounded(&s_full[s], (parity >> s) & 1u, POPC_WAIT_NS);
     }
-    popc_blocks_finish_grid(p, sparse_seen, &s_epoch, &s_flag, s_scan);
+    // (no copy is in flight any more: the stages hold the block prefixes)
+    popc_blocks_finish_grid(p, sparse_seen, &s_epoch, &s_flag, s_scan, reinterpret_cast<uint64_t*>(smem), POPC_STREAM_SMEM / 8);
 }
 
 // Masks of more than this many blocks per SM take the streaming form.
