@@ -12,6 +12,7 @@
 // Selectivity is measured when the plan is built (CS_ALGO_AUTO, and only when the table has a
 // 1-pass entry): one popcount pass over the masks into plan-owned count words. The choice
 // changes speed, never results, so masks that change between runs stay correct.
+#include <algorithm>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -28,6 +29,7 @@ struct cs_batch {
     int sms = 0;
     std::vector<uint64_t*> empty_counts; // d_count of n == 0 columns
     void* dmem = nullptr;
+    size_t device_bytes = 0;
     PlanLayout layout;
     PlanDevice dev;
     PlanCounts counts;
@@ -46,6 +48,16 @@ namespace {
 // bytes HBM moves in the 40 us their extra launches take).
 constexpr uint64_t PLAN_3PASS_MIN_BYTES = 256ull << 20;
 
+// A plan of at least this much payload, at least half of it in columns where the 3-pass form moves
+// its bytes faster, is run as 3-pass altogether: its chain is then one per plan and long since
+// hidden, while a plan of both forms pays both. Where the lines lie (graph replays on B200, plans of
+// equal columns, us, 1-pass / 3-pass): u8 half selected 254 / 210 at 512 MB; u32 half selected
+// 80 / 80 at 256 MB, 154 / 149 at 512 MB, 320 / 288 at 1 GB; u64 0.9 selected 373 / 326 at 1 GB;
+// but u32 0.1 selected 117 / 122 at 512 MB, 227 / 226 at 1 GB. Uneven u32 and u64 columns of 2.2 GB,
+// any selectivity: 615 / 578.
+constexpr uint64_t PLAN_ALL_3PASS_BYTES = 512ull << 20;
+constexpr double PLAN_3PASS_SELECTED = 0.3; // 4- and 8-byte columns: least selected fraction
+
 inline int to_status(cudaError_t e)
 {
     if (e == cudaSuccess) return CS_SUCCESS;
@@ -63,8 +75,12 @@ int run_direct(cs_batch* b, cudaStream_t s)
 }
 
 // Selected fraction of every column, from one reduce-then-scan popcount pass over the masks
-// (into count words of a temporary plan, so nothing of the caller's is written).
-int measure_selectivity(const cs_column* cols, uint32_t ncols, int sms, cudaStream_t s, std::vector<double>& sel)
+// (into count words of a temporary plan, so nothing of the caller's is written). The temporary
+// plan lies in *dmem, allocated here with the *room that the plan itself needs whatever the
+// columns' forms turn out to be: device allocations are most of the time that making a plan takes
+// (0.35 ms each, and 0.3 ms to free one, beside 0.2 ms of other work for 256 columns).
+int measure_selectivity(const cs_column* cols, uint32_t ncols, int sms, cudaStream_t s, std::vector<double>& sel,
+                        void** dmem, size_t* room)
 {
     sel.assign(ncols, 0.0);
     std::vector<ColumnDesc> desc;
@@ -75,13 +91,21 @@ int measure_selectivity(const cs_column* cols, uint32_t ncols, int sms, cudaStre
     if (st != CS_SUCCESS) return st;
     if (!c.tiles) return CS_SUCCESS;
     const PlanLayout L = plan_layout(c, true);
-    void* mem = nullptr;
-    if (cudaMalloc(&mem, L.total) != cudaSuccess) {
+    PlanCounts c3, c1;
+    const std::vector<uint8_t> all1(ncols, 1);
+    std::vector<ColumnDesc> desc_unused;
+    std::vector<uint64_t> base_unused;
+    if ((st = plan_columns(cols, ncols, desc_unused, base_unused, c3, nullptr)) != CS_SUCCESS) return st;
+    if ((st = plan_columns(cols, ncols, desc_unused, base_unused, c1, nullptr, &all1)) != CS_SUCCESS) return st;
+    const size_t bytes = std::max(L.total, plan_layout(c3, false).total + plan_layout(c1, false).total);
+    if (cudaMalloc(dmem, bytes) != cudaSuccess) {
         cudaGetLastError();
+        *dmem = nullptr;
         return CS_ERR_OUT_OF_MEMORY;
     }
+    *room = bytes;
     const PlanMaps m = plan_maps(c);
-    const PlanDevice d = plan_device(static_cast<uint8_t*>(mem), L, m);
+    const PlanDevice d = plan_device(static_cast<uint8_t*>(*dmem), L, m);
     for (uint32_t i = 0; i < ncols; ++i) desc[i].d_count = d.counts + i;
     std::vector<uint8_t> img(m.bytes);
     plan_write_image(img.data(), m, d, desc, chunk_base);
@@ -103,8 +127,7 @@ int measure_selectivity(const cs_column* cols, uint32_t ncols, int sms, cudaStre
     }
     if (e == cudaSuccess && ncols) e = cudaMemcpyAsync(counts.data(), d.counts, 8 * ncols, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    cudaFree(mem);
-    if (e != cudaSuccess) return to_status(e);
+    if (e != cudaSuccess) return to_status(e); // (the caller frees *dmem)
     for (uint32_t i = 0; i < ncols; ++i)
         if (cols[i].n) sel[i] = static_cast<double>(counts[i]) / static_cast<double>(cols[i].n);
     return CS_SUCCESS;
@@ -137,24 +160,31 @@ int cs_batch_create(cs_batch** out, const cs_column* cols, uint32_t ncols, const
 
     // per column: 1-pass or 3-pass (forced by cfg->algo, else the batch table's bucket)
     std::vector<uint8_t> one_pass(ncols, algo == CS_ALGO_1PASS ? 1 : 0);
+    size_t room = 0; // of b->dmem, if it is already there
     if (algo == CS_ALGO_AUTO && tune_batch_any_1pass()) {
         std::vector<double> sel;
-        const int st = measure_selectivity(cols, ncols, b->sms, s, sel);
+        const int st = measure_selectivity(cols, ncols, b->sms, s, sel, &b->dmem, &room);
         if (st != CS_SUCCESS) {
+            cudaFree(b->dmem);
             delete b;
             return st;
         }
         for (uint32_t i = 0; i < ncols; ++i)
             one_pass[i] = cols[i].n && tune_batch_lookup(cols[i].n, cols[i].elem_bytes, sel[i]) == CS_ALGO_1PASS;
-        // Beside 1-pass columns, the 3-pass ones add a chain of their own (pass 1+2, the
-        // sparse gather, a writeout per width: about 40 us of launches that wait on one
-        // another on B200), and what their form saves is at most their payload reads. Below
+        // Beside 1-pass columns, the 3-pass ones add a chain of their own (pass 1+2, a writeout
+        // per width: about 30 us of launches that wait on one another on B200), and what their form saves is at most their payload reads. Below
         // PLAN_3PASS_MIN_BYTES of 3-pass payload they join the 1-pass kernels (batch256:
         // 0.602 -> 0.571 ms per replay with its six sparse columns moved).
         uint64_t bytes3 = 0, bytes1 = 0;
         for (uint32_t i = 0; i < ncols; ++i)
             (one_pass[i] ? bytes1 : bytes3) += cols[i].n * static_cast<uint64_t>(cols[i].elem_bytes);
-        if (bytes1 && bytes3 < PLAN_3PASS_MIN_BYTES)
+        uint64_t faster3 = 0;
+        for (uint32_t i = 0; i < ncols; ++i)
+            if (!one_pass[i] || cols[i].elem_bytes <= 2 || sel[i] >= PLAN_3PASS_SELECTED)
+                faster3 += cols[i].n * static_cast<uint64_t>(cols[i].elem_bytes);
+        if (bytes1 + bytes3 >= PLAN_ALL_3PASS_BYTES && faster3 >= (bytes1 + bytes3) / 2)
+            one_pass.assign(ncols, 0);
+        else if (bytes1 && bytes3 < PLAN_3PASS_MIN_BYTES)
             for (uint32_t i = 0; i < ncols; ++i) one_pass[i] = cols[i].n ? 1 : 0;
     }
     for (uint32_t i = 0; i < ncols; ++i) b->one_pass_cols += one_pass[i] && cols[i].n ? 1u : 0u;
@@ -163,11 +193,19 @@ int cs_batch_create(cs_batch** out, const cs_column* cols, uint32_t ncols, const
     std::vector<uint64_t> chunk_base;
     int st = plan_columns(cols, ncols, desc, chunk_base, b->counts, &b->empty_counts, &one_pass);
     if (st != CS_SUCCESS) {
+        cudaFree(b->dmem);
         delete b;
         return st;
     }
     b->layout = plan_layout(b->counts, false);
-    cudaError_t e = cudaMalloc(&b->dmem, b->layout.total);
+    cudaError_t e = cudaSuccess;
+    if (b->layout.total > room) {
+        cudaFree(b->dmem);
+        b->dmem = nullptr;
+        room = b->layout.total;
+        e = cudaMalloc(&b->dmem, room);
+    }
+    b->device_bytes = room;
     if (e != cudaSuccess) {
         cudaGetLastError();
         delete b;
@@ -264,7 +302,7 @@ uint32_t cs_batch_one_pass_columns(const cs_batch* b)
 
 uint64_t cs_batch_device_bytes(const cs_batch* b)
 {
-    return b ? b->layout.total : 0;
+    return b ? b->device_bytes : 0;
 }
 
 uint32_t cs_batch_launches(const cs_batch* b)
