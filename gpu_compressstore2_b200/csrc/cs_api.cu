@@ -37,10 +37,14 @@ constexpr uint64_t DEEP_UNITS_PER_SM = 16;
 // Most slices per SM for which a 1-pass call of 4- and 8-byte elements runs in slices (cs_slices.cu)
 // rather than through the TMA kernel; 1- and 2-byte columns of any length do. Per call on B200, inputs
 // from HBM, TMA / slices, us: u32 p = 0.5 2^20 8.5 / 5.4, 2^22 14.3 / 11.4, 2^23 (7 per SM) 20.1 / 15.8,
-// 2^24 (14) 25.6 / 25.7, 2^28 282 / 303; p = 0.1 2^23 16.6 / 13.6, 2^24 21.1 / 21.5; u64 2^22 (7) p = 0.5
-// 18.8 / 15.1, 2^23 p = 0.1 20.1 / 22.6; u8 2^24 17.3 / 13.5, 2^28 133 / 103; u16 2^24 23.2 / 18.7, 2^26
-// 50.9 / 47.4.
-constexpr uint64_t SLICES_PER_SM = 8;
+// 1.5 x 2^23 (10) 22.9 / 20.5, 2^24 (14) 25.7 / 25.4, 1.25 x 2^24 (17) 30.7 / 29.2, 2^28 282 / 303;
+// p = 0.1 2^23 16.6 / 13.6, 1.5 x 2^23 19.9 / 17.6, 2^24 21.2 / 21.3, 2^25 (28) 35.1 / 35.5; u64 2^22 (7)
+// p = 0.5 18.8 / 15.1, 2^23 (14) p = 0.1 20.1 / 22.6; u8 2^24 17.3 / 13.5, 2^28 133 / 103; u16 2^24
+// 23.2 / 18.7, 2^26 50.9 / 47.4.
+constexpr uint64_t slices_per_sm(uint32_t elem_bytes)
+{
+    return elem_bytes == 4 ? 18 : 8;
+}
 constexpr uint64_t DEFAULT_TIMEOUT_NS = 2000000000ull;
 
 struct DeviceInfo {
@@ -264,11 +268,12 @@ int run_compaction(const void* d_in, const void* d_mask, void* d_out, uint64_t n
     int algo = r.algo;
     const bool tma_ok = aligned(d_in, 16) && aligned(d_out, 16) && aligned(d_mask, 16);
     // The 1-pass form runs in slices (cs_slices.cu), or through the TMA kernel for 4- and 8-byte columns of
-    // more than SLICES_PER_SM. The slices' totals lie where the 3-pass form has its chunk offsets (which
+    // more than slices_per_sm. The slices' totals lie where the 3-pass form has its chunk offsets (which
     // never read as a status); a caller's chunk length may leave less room than that.
     const uint64_t slices = slices_of(n, elem_bytes);
-    const bool in_slices = slices <= l.num_chunks &&
-                           (elem_bytes <= 2 || slices <= SLICES_PER_SM * static_cast<uint64_t>(di.sms));
+    const bool in_slices =
+        slices <= l.num_chunks &&
+        (elem_bytes <= 2 || slices <= slices_per_sm(elem_bytes) * static_cast<uint64_t>(di.sms));
     if ((algo == CS_ALGO_1PASS || algo == CS_ALGO_3PASS) && !tma_ok) {
         if (!auto_route) return CS_ERR_MISALIGNED;
         // slices take any mask and output, the warp writeout any element-aligned pointers; the latter

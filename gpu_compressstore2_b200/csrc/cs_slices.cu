@@ -24,7 +24,7 @@
 // Tried: a look-back over slices instead of the carried sum (it grows with the number of slices: 494
 // us at the best slice size), evaluating one slice ahead (365), slices of two items per warp
 // (374 .. 384), 2 and 4 CTAs per SM (408, 378), the evaluated payload through shared memory by bulk
-// copies (377). The 1-pass form's figures stand at SLICES_PER_SM in cs_api.cu; what bounds it is the
+// copies (377). The 1-pass form's figures stand at slices_per_sm in cs_api.cu; what bounds it is the
 // start (ticket, mask, payload one after another) for short columns and the barrier for long ones.
 //
 // A comparison of whole numbers is (x - lo) <= (hi - lo) in unsigned arithmetic, whatever the sign

@@ -18,10 +18,17 @@ std::atomic<uint32_t> g_batch[TUNE_WIDTHS][TUNE_SIZES][TUNE_SELS];
 // Plain call with a stated selectivity: packed like g_table. Zero = unset (use g_table).
 std::atomic<uint32_t> g_sel[TUNE_WIDTHS][TUNE_SIZES][TUNE_SELS];
 
+// What an unset entry means. An entry holds for a factor of four in length, and the two in which the
+// 1-pass form stops being the faster one are left unset in the packaged table: 4-byte columns of 2^24 ..
+// 2^26 elements, 8-byte ones of 2^22 .. 2^24. On B200, us, 1-pass / 3-pass: u32 2^24 p = 0.1 21.5 / 24.7
+// (0.01: 20.2 / 13.9), 1.25 x 2^24 24.3 / 25.2, 2^25 35.5 / 34.8 (0.01: 33 / 17), 2^25.5 p = 0.9 71 / 68;
+// u64 2^23 p = 0.5 24.5 / 25.2, 2^23.5 35.3 / 31.3 (0.01: 26 / 12).
 TuneChoice default_choice(uint64_t n, uint32_t elem_bytes)
 {
-    (void)n;
-    (void)elem_bytes;
+    constexpr uint64_t ONE_PASS_BYTES = 76ull << 20;
+    const int b = tune_size_bucket(n);
+    const bool turns = (elem_bytes == 4 && b == 12) || (elem_bytes == 8 && b == 11);
+    if (turns && n * elem_bytes <= ONE_PASS_BYTES) return TuneChoice{CS_ALGO_1PASS, 1024u};
     return TuneChoice{CS_ALGO_3PASS, 1024u};
 }
 } // namespace

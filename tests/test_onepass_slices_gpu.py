@@ -60,3 +60,19 @@ def test_auto_unaligned_mask_and_output(cuda, oracle, w):
         assert k == len(exp)
         assert np.array_equal(out[out_off:out_off + k], exp)
         assert np.all(np.concatenate([out[:out_off], out[out_off + k:]]).view(np.uint8) == 0xAB)
+
+
+@pytest.mark.parametrize("w,n", [(4, 18 * 148 * 8192), (4, 18 * 148 * 8192 + 1), (4, (76 << 20) // 4), (4, (76 << 20) // 4 + 1),
+                                 (8, (76 << 20) // 8), (8, (76 << 20) // 8 + 1), (4, (1 << 24) + 4099)])
+def test_where_the_forms_change(cuda, oracle, w, n):
+    """Both sides of the lines between slices, the other 1-pass kernel and the 3-pass form."""
+    import gpu_compressstore2_b200 as cs
+
+    rng = np.random.default_rng(n)
+    payload = rng.integers(0, 256, size=n * w, dtype=np.uint8).view(UNSIGNED[w])
+    mask = rng.integers(0, 1 << 32, size=(n + 31) // 32, dtype=np.uint64).astype(np.uint32)
+    check_against_oracle(oracle, payload, mask, n, "1pass")
+    check_against_oracle(oracle, payload, mask, n, "auto")  # its scratch sized
+    before = cs.launch_count()
+    check_against_oracle(oracle, payload, mask, n, "auto")
+    assert (cs.launch_count() - before == 1) == (n * w <= 76 << 20)
