@@ -163,10 +163,8 @@ __global__ void __launch_bounds__(DENSE_WARPS * 32, DENSE_CTAS)
                     if (in32) ldg256(src + k * ROW_BYTES, x[k]);
                     else ldg128x2(src + k * ROW_BYTES, x[k]);
                 } else {
-                    // the lane in which the column ends: element by element, through the idle stage
-                    const T* last = reinterpret_cast<const T*>(in) + e;
-                    T* tmp = reinterpret_cast<T*>(stage + lane * LANE_BYTES);
-                    for (uint32_t i = 0; e + i < n; ++i) tmp[i] = __ldg(last + i);
+                    // the lane in which the column ends: through the idle stage
+                    load_end(src + k * ROW_BYTES, static_cast<uint32_t>(n - e) * static_cast<uint32_t>(sizeof(T)), stage_a + lane * LANE_BYTES);
 #pragma unroll
                     for (uint32_t w = 0; w < 8; ++w) x[k][w] = lds32(stage_a + lane * LANE_BYTES + 4 * w);
                 }

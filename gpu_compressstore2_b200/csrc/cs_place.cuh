@@ -158,6 +158,34 @@ __device__ __forceinline__ void fill_pack_table(uint32_t* table, uint32_t thread
     }
 }
 
+// The end of a column, `bytes` < LANE_BYTES from `src` (16-byte aligned) to `tmp` in shared memory, by one
+// lane: both halves go out together and hold no registers (elements one after another through a loop: 1-pass
+// calls of 3 x 10^6 u8 6.97 -> 5.89 us).
+__device__ __forceinline__ void load_end(const uint8_t* src, uint32_t bytes, uint32_t tmp)
+{
+    const uint32_t first = bytes < 16u ? bytes : 16u;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(tmp), "l"(src), "r"(first) : "memory");
+    if (bytes > 16u)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(tmp + 16u), "l"(src + 16), "r"(bytes - 16u) : "memory");
+    asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
+// The same for an element-aligned `in` and up to LANE_BYTES, eight elements at a time.
+template <typename T>
+__device__ __forceinline__ void load_end_unaligned(const T* __restrict__ in, uint32_t count, T* tmp)
+{
+    constexpr uint32_t BATCH = LANE_BYTES / sizeof(T) < 8 ? LANE_BYTES / sizeof(T) : 8;
+    for (uint32_t i = 0; i < count; i += BATCH) {
+        T v[BATCH];
+#pragma unroll
+        for (uint32_t k = 0; k < BATCH; ++k)
+            if (i + k < count) v[k] = __ldg(in + i + k);
+#pragma unroll
+        for (uint32_t k = 0; k < BATCH; ++k)
+            if (i + k < count) tmp[i + k] = v[k];
+    }
+}
+
 // Elements [a, run) of the stage (placed with swizzle m) to gdst + the same positions (gdst 16-byte
 // aligned, a within its first vector): whole 16-byte vectors, and the ragged ends element by
 // element (lanes 0-15 the head, lanes 16-31 the tail).

@@ -140,15 +140,14 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS) k_if(const SliceParams p)
 
     auto item_elem = [&](uint32_t slice) -> uint64_t { return (static_cast<uint64_t>(slice) * WARPS + warp) * ITEM; };
     // the lane's 32 bytes of row r of the item at e0, where the column ends in or before the item:
-    // the lane in which it ends goes element by element, through its place in the idle stage
+    // the lane in which it ends goes through its place in the idle stage
     auto load_ragged = [&](uint64_t e0, uint32_t r, uint32_t (&x)[8]) {
         const uint64_t e = e0 + r * ROW + lane * EPL;
         const uint8_t* src = in + e * sizeof(T);
         if (e + EPL <= n) {
             ldg128x2(src, x);
         } else if (e < n) {
-            U* tmp = reinterpret_cast<U*>(stage + lane * LANE_BYTES);
-            for (uint32_t i = 0; e + i < n; ++i) tmp[i] = __ldg(reinterpret_cast<const U*>(src) + i);
+            load_end(src, static_cast<uint32_t>(n - e) * static_cast<uint32_t>(sizeof(T)), stage_a + lane * LANE_BYTES);
 #pragma unroll
             for (uint32_t q = 0; q < 8; ++q) x[q] = lds32(stage_a + lane * LANE_BYTES + 4 * q);
         }

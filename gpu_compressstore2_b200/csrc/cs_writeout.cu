@@ -309,10 +309,12 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS<SHIFT>) k_writeout_warp(const
                     else ldg128x2(src + r * ROW_BYTES, x[r]);
                 } else {
                     // the lane in which the column ends (or, shifted, begins or all but ends):
-                    // element by element, through its place in the idle stage
-                    const T* in = reinterpret_cast<const T*>(C.in) + e;
-                    T* tmp = reinterpret_cast<T*>(stage + lane * LANE_BYTES);
-                    for (uint32_t i = 0; i < EPL && e + i < n; ++i) tmp[i] = __ldg(in + i);
+                    // through its place in the idle stage
+                    const uint32_t count = n - e < EPL ? static_cast<uint32_t>(n - e) : EPL;
+                    if constexpr (SHIFT)
+                        load_end_unaligned(reinterpret_cast<const T*>(C.in) + e, count, reinterpret_cast<T*>(stage + lane * LANE_BYTES));
+                    else
+                        load_end(src + r * ROW_BYTES, count * static_cast<uint32_t>(sizeof(T)), stage_a + lane * LANE_BYTES);
 #pragma unroll
                     for (uint32_t q = 0; q < 8; ++q) x[r][q] = lds32(stage_a + lane * LANE_BYTES + 4 * q);
                 }
