@@ -378,7 +378,7 @@ __device__ __forceinline__ void popc_block_load(const Col& col, uint64_t bl, con
 template <int LPC, typename Col>
 __device__ __forceinline__ void popc_block_finish(const BlockScanParams& p, const Col& col, uint64_t blk,
                                                   uint64_t bl, const uint4 (&q)[8], uint32_t* s_warp,
-                                                  uint32_t* s_whalf, const uint32_t* s_epoch, bool& sparse_seen)
+                                                  uint32_t* s_whalf, const uint32_t* s_epoch, uint32_t& sparse_seen)
 {
     constexpr uint32_t CHUNK_LOG2 = LPC == 1 ? 7 : LPC == 2 ? 8 : LPC == 4 ? 9 : LPC == 8 ? 10 : LPC == 16 ? 11 : 12;
     static_assert((1u << CHUNK_LOG2) == LPC * 128u, "chunk length = 128 elements per lane");
@@ -410,8 +410,8 @@ __device__ __forceinline__ void popc_block_finish(const BlockScanParams& p, cons
     // sparse hint over the warp's two aligned 16K-element groups (rows 0-3, 4-7), whole ones only: the short
     // end of a column has few selected elements at any selectivity, and the gather costs a column without
     // sparse units 5 us (1.4 x 2^22 u32, half selected, ending 631 elements into a group: 20.7 -> 15.4)
-    sparse_seen |= (half <= 512u) && (row0 + 4) * 4096 <= n;
-    sparse_seen |= (run - half <= 512u) && (row0 + 8) * 4096 <= n;
+    sparse_seen += (half <= 512u) && (row0 + 4) * 4096 <= n;
+    sparse_seen += (run - half <= 512u) && (row0 + 8) * 4096 <= n;
     if (lane == 0) {
         s_warp[warp] = run;
         s_whalf[warp] = half;
@@ -436,22 +436,40 @@ __device__ __forceinline__ void popc_block_finish(const BlockScanParams& p, cons
     __syncthreads(); // s_warp is rewritten by the next block
 }
 
-// The end of both pass-1+2 kernels (all threads): the finishing ticket carries the CTA's
-// sparse hint in its upper bits, so the last CTA learns from its own atomic whether any CTA
-// saw a sparse block (no flag array to read). The last CTA scans the block sums and closes
-// the epoch; the call's scan is marked clean unless a CTA poisoned this epoch.
-__device__ __forceinline__ void popc_blocks_finish_grid(const BlockScanParams& p, bool sparse_seen,
-                                                        const uint32_t* s_epoch, uint32_t* s_flag, uint64_t* s_scan,
-                                                        uint64_t* s_prefix, uint64_t prefix_room)
+// The writeout gathers the sparse units instead of reading them whole if at least SPARSE_GROUPS_MIN of the pass's
+// groups are sparse, and half of them (long columns of 4- and 8-byte elements, and large plans: one in 12). Where
+// the lines lie (3-pass calls on B200, us, gathering / reading whole): all groups sparse (p = 0.01) 2^21 u32 (128
+// groups) 10.0 / 8.6, 2^22 11.3 / 11.5, 2^23 12.0 / 14.2, u64 11.4 / 17.8; runs of 65536 (less than half) 2^24 u8 47 / 18,
+// u32 33 / 26, 2^27 u8 110 / 61, u32 125 / 125; 2^27 u32 with its last fifth empty 170 / 181, its last tenth 183 / 188;
+// plans of 40 columns and 8 MB with a few sparse ones 29.8 / 14.8, 128 columns and 470 MB 159 / 143.
+constexpr uint64_t SPARSE_GROUPS_MIN = 256;
+constexpr uint64_t LONG_BLOCKS = 256; // 2^26 elements
+
+// The end of both pass-1+2 kernels (all threads): the finishing ticket carries in its upper bits how many
+// of the 16 groups of the CTA's average block are sparse, so the last CTA learns their share from its own
+// atomic (no array to read). The last CTA scans the block sums and closes
+// the epoch; the call's scan is marked clean unless a CTA poisoned this epoch. sparse_seen: this warp's
+// sparse groups, of `blocks` blocks; s_warp: free.
+__device__ __forceinline__ void popc_blocks_finish_grid(const BlockScanParams& p, uint32_t sparse_seen, uint32_t blocks,
+                                                        uint32_t* s_warp, const uint32_t* s_epoch, uint32_t* s_flag,
+                                                        uint64_t* s_scan, uint64_t* s_prefix, uint64_t prefix_room)
 {
     const uint32_t tid = threadIdx.x;
-    const bool cta_sparse = __syncthreads_or(sparse_seen) != 0;
+    if ((tid & 31u) == 0) s_warp[tid >> 5] = sparse_seen;
+    __syncthreads();
     const uint32_t epoch = *s_epoch; // written by thread 0 before the barrier above
     if (tid == 0) {
+        uint32_t groups = 0;
+        for (uint32_t w = 0; w < 8; ++w) groups += s_warp[w];
+        // at most 16, of 2048 CTAs
+        const uint32_t mean = static_cast<uint32_t>(__fdividef(static_cast<float>(groups), static_cast<float>(blocks)) + 0.01f);
         __threadfence(); // this CTA's offsets and block sums before its ticket
-        const uint32_t prev = atomicAdd(&p.hdr->scan_done_counter, 1u + (cta_sparse ? 0x10000u : 0u));
+        const uint32_t prev = atomicAdd(&p.hdr->scan_done_counter, 1u + (mean << 16));
         const bool last = (prev & 0xffffu) == gridDim.x - 1;
-        *s_flag = last ? (1u | ((cta_sparse || (prev >> 16) != 0u) ? 2u : 0u)) : 0u;
+        const uint32_t sum = (prev >> 16) + mean;
+        const uint32_t share = p.num_blocks > LONG_BLOCKS && (p.cols || p.col0.elem_bytes >= 4) ? 12u : 2u;
+        const bool sparse = sum * share >= 16u * gridDim.x && sum * p.num_blocks >= SPARSE_GROUPS_MIN * gridDim.x;
+        *s_flag = last ? (1u | (sparse ? 2u : 0u)) : 0u;
     }
     __syncthreads();
     const uint32_t fin = *s_flag;
@@ -474,15 +492,16 @@ __global__ void __launch_bounds__(256, 4) k_popc_blocks(const BlockScanParams p)
     const uint32_t tid = threadIdx.x;
     grid_dependency_wait(); // earlier calls may still be using this workspace
     if (tid == 0) s_epoch = p.hdr->epoch;
-    bool sparse_seen = false;
-    for (uint64_t blk = blockIdx.x; blk < p.num_blocks; blk += gridDim.x) {
+    uint32_t sparse_seen = 0;
+    uint32_t blocks = 0;
+    for (uint64_t blk = blockIdx.x; blk < p.num_blocks; blk += gridDim.x, ++blocks) {
         const ColumnDesc& col = column_of(p.col0, p.cols, p.blk_col, blk);
         const uint64_t bl = blk - col.tile_base; // block within its column
         uint4 q[8];
         popc_block_load(col, bl, popc_share(col, bl), tid >> 5, tid & 31u, q);
         popc_block_finish<LPC>(p, col, blk, bl, q, s_warp, s_whalf, &s_epoch, sparse_seen);
     }
-    popc_blocks_finish_grid(p, sparse_seen, &s_epoch, &s_flag, s_scan, s_prefix, 1024);
+    popc_blocks_finish_grid(p, sparse_seen, blocks, s_warp, &s_epoch, &s_flag, s_scan, s_prefix, 1024);
 }
 
 // ---------------------------------------------------------------------------------
@@ -600,7 +619,7 @@ __global__ void __launch_bounds__(256, POPC_STREAM_CTAS) k_popc_stream(const Blo
     }
     __syncthreads(); // barriers initialised, s_epoch and s_fail visible
     const uint32_t epoch = s_epoch;
-    bool sparse_seen = false;
+    uint32_t sparse_seen = 0;
     uint32_t parity = 0; // bit s: parity of the phase stage s completes next
     for (uint64_t i = 0; b0 + i < b1; ++i) {
         const uint64_t blk = b0 + i;
@@ -644,7 +663,8 @@ __global__ void __launch_bounds__(256, POPC_STREAM_CTAS) k_popc_stream(const Blo
             if ((pending >> s) & 1u) mbar_wait_bounded(&s_full[s], (parity >> s) & 1u, POPC_WAIT_NS);
     }
     // (no copy is in flight any more: the stages hold the block prefixes)
-    popc_blocks_finish_grid(p, sparse_seen, &s_epoch, &s_flag, s_scan, reinterpret_cast<uint64_t*>(smem), POPC_STREAM_SMEM / 8);
+    popc_blocks_finish_grid(p, sparse_seen, static_cast<uint32_t>(b1 - b0), s_warp, &s_epoch, &s_flag, s_scan, reinterpret_cast<uint64_t*>(smem),
+                            POPC_STREAM_SMEM / 8);
 }
 
 // Masks of more than this many blocks per SM take the streaming form.

@@ -1,6 +1,6 @@
 """The sparse gather of the 3-pass form where its work split can go wrong: units at exactly the
 1/32 limit and one past it, clusters that fill a warp's index list several times over, whole
-and quarter work items, columns that end inside an item, chunks shorter than a group. Bit for
+and quarter work items (columns of 2^22 elements and more), columns that end inside an item, chunks shorter than a group. Bit for
 bit against the CPU oracle. Needs a B200."""
 from __future__ import annotations
 
@@ -39,7 +39,7 @@ def _mask(n, w, rng):
 
 @pytest.mark.parametrize("w", [1, 2, 4, 8])
 @pytest.mark.parametrize("n,chunk_length", [(16384 * 3 + 1, 1024), (16384 * 3 + 1, 4096), (131072 * 13 - 33, 1024),
-                                            (131072 * 13 - 33, 4096), (WHOLE_ITEMS_N + 4097, 4096)])
+                                            (131072 * 13 - 33, 4096), (131072 * 70 - 33, 1024), (WHOLE_ITEMS_N + 4097, 4096)])
 def test_sparse_units(cuda, oracle, n, w, chunk_length):
     rng = np.random.default_rng(n + w)
     payload = rng.integers(0, 256, size=n * w, dtype=np.uint8).view({1: np.uint8, 2: np.uint16, 4: np.uint32,
