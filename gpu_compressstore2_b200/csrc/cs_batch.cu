@@ -48,16 +48,6 @@ namespace {
 // bytes HBM moves in the 40 us their extra launches take).
 constexpr uint64_t PLAN_3PASS_MIN_BYTES = 256ull << 20;
 
-// A plan of at least this much payload, at least half of it in columns where the 3-pass form moves
-// its bytes faster, is run as 3-pass altogether: its chain is then one per plan and long since
-// hidden, while a plan of both forms pays both. Where the lines lie (graph replays on B200, plans of
-// equal columns, us, 1-pass / 3-pass): u8 half selected 254 / 210 at 512 MB; u32 half selected
-// 80 / 80 at 256 MB, 154 / 149 at 512 MB, 320 / 288 at 1 GB; u64 0.9 selected 373 / 326 at 1 GB;
-// but u32 0.1 selected 117 / 122 at 512 MB, 227 / 226 at 1 GB. Uneven u32 and u64 columns of 2.2 GB,
-// any selectivity: 615 / 578.
-constexpr uint64_t PLAN_ALL_3PASS_BYTES = 512ull << 20;
-constexpr double PLAN_3PASS_SELECTED = 0.3; // 4- and 8-byte columns: least selected fraction
-
 inline int to_status(cudaError_t e)
 {
     if (e == cudaSuccess) return CS_SUCCESS;
@@ -178,13 +168,7 @@ int cs_batch_create(cs_batch** out, const cs_column* cols, uint32_t ncols, const
         uint64_t bytes3 = 0, bytes1 = 0;
         for (uint32_t i = 0; i < ncols; ++i)
             (one_pass[i] ? bytes1 : bytes3) += cols[i].n * static_cast<uint64_t>(cols[i].elem_bytes);
-        uint64_t faster3 = 0;
-        for (uint32_t i = 0; i < ncols; ++i)
-            if (!one_pass[i] || cols[i].elem_bytes <= 2 || sel[i] >= PLAN_3PASS_SELECTED)
-                faster3 += cols[i].n * static_cast<uint64_t>(cols[i].elem_bytes);
-        if (bytes1 + bytes3 >= PLAN_ALL_3PASS_BYTES && faster3 >= (bytes1 + bytes3) / 2)
-            one_pass.assign(ncols, 0);
-        else if (bytes1 && bytes3 < PLAN_3PASS_MIN_BYTES)
+        if (bytes1 && bytes3 < PLAN_3PASS_MIN_BYTES)
             for (uint32_t i = 0; i < ncols; ++i) one_pass[i] = cols[i].n ? 1 : 0;
     }
     for (uint32_t i = 0; i < ncols; ++i) b->one_pass_cols += one_pass[i] && cols[i].n ? 1u : 0u;
