@@ -166,7 +166,6 @@ struct cs_server {
     PlanCounts caps;
     PlanLayout layout;
     size_t ws_bytes = 0; // per-call workspace bytes (count word follows)
-    int bps[4] = {1, 1, 1, 1};
     std::vector<Slot> slots;
 
     std::mutex mu;
@@ -506,7 +505,6 @@ int cs_server_create(cs_server** out, const cs_server_config* cfg)
         s->ws_bytes = a256(s->ws_bytes);
         slot_bytes = s->ws_bytes;
     }
-    for (int wi = 0; wi < 4; ++wi) s->bps[wi] = std::max(1, compact_tma_blocks_per_sm(1u << wi, 1));
 
     cudaError_t e = cudaMalloc(&s->arena_base, c.out_budget_bytes);
     if (e != cudaSuccess) {
