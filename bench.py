@@ -687,7 +687,7 @@ def reference_gpu_run(workload: str, reps: int = 5, sweep=REF_GPU_SWEEP, timeout
 def kernel_roofline(cs, torch, args, n, w, d_in, d_mask, d_out, d_count, B, step_ms, stream, peaks, workload):
     """Roofline of the dominant kernel, timed alone with CUDA events on its stream.
 
-    1-pass: the step is the single k_compact_tma launch, so the step time is its time.
+    1-pass: the step is one launch, so the step time is its time.
     3-pass: k_writeout_warp is launched alone through cs_writeout, over the same
     inputs with the chunk offsets of the same chunk length, and timed; its algorithmic bytes
     are the call's (every payload byte read once, mask read, selected written; the counts and
@@ -701,7 +701,7 @@ def kernel_roofline(cs, torch, args, n, w, d_in, d_mask, d_out, d_count, B, step
         chunk = int(c.value)
     if algo != "3pass":
         kms = step_ms
-        kernel = "k_compact_tma (1-pass: the whole step is this one kernel)" if algo == "1pass" else \
+        kernel = "1-pass: the whole step is one kernel (k_if in slices, or k_compact_tma)" if algo == "1pass" else \
             f"whole {algo} step"
         launches_timed = args.steps
     else:
@@ -794,7 +794,7 @@ def run_ours(args, workload: str):
     if pattern_path or pred_path:
         achieved = B / (ms * 1e-3) / 1e9
         kname = ("k_pattern (the whole step is this one kernel)" if pattern_path else
-                 "whole step: k_pred_blocks + sparse gather + k_compact_tma (payload read twice)")
+                 "k_if (the whole step is this one kernel; the payload is read from HBM once)")
         roofline = {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                     "frac": achieved / peaks["hbm_gbs"], "traffic": load_traffic(workload),
                     "peak_source": peaks["source"], "kernel": kname,
