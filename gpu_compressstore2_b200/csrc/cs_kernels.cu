@@ -288,8 +288,8 @@ __device__ __forceinline__ void mark_sparse_units(const BlockScanParams& p, cons
 // CTA to finish scans the block sums into blk_base (exclusive prefix of each block within
 // its column) and writes every column's count; consumers add the two (chunk_offset). This
 // replaces a decoupled look-back across blocks, whose waiting dominated the fused pass at
-// large n. Each CTA also records whether one of its aligned 16K-element groups holds at
-// most 512 selected elements (the sparse-unit hint of the hybrid writeout).
+// large n. Each CTA also counts its whole 16K-element groups of at most 512 selected
+// elements (the hint by which the writeout takes its gather, SPARSE_GROUPS_MIN).
 // Reference: pass 1 kernel_3pass_popc_none_striding (src/kernels/kernel_3pass.cuh:12-57)
 // and pass 2 launch_cub_pss / kernel_3pass_pss_gmem (src/cub_wraps.cuh:52-79,
 // src/kernels/kernel_3pass.cuh:59-214).

@@ -241,7 +241,7 @@ uint32_t plan_kernels(const PlanCounts& c)
 }
 
 int plan_launch(const PlanDevice& d, const PlanCounts& c, int sms, uint64_t timeout_ns, cudaStream_t s,
-                const uint32_t* grid1)
+                const uint32_t* grid1, uint32_t writeout_ctas)
 {
     if (c.tiles) {
         BlockScanParams bp{};
@@ -271,7 +271,7 @@ int plan_launch(const PlanDevice& d, const PlanCounts& c, int sms, uint64_t time
         p.item_flags = d.item_flags;
         p.hdr = d.hdr;
         p.chunk_log2 = PLAN_CHUNK_LOG2;
-        cudaError_t e = launch_writeout_warp(p, w, 0, sms, s);
+        cudaError_t e = launch_writeout_warp(p, w, writeout_ctas, sms, s);
         if (e != cudaSuccess) return to_status(e);
     }
     for (int wi = 0; wi < 4; ++wi) {
