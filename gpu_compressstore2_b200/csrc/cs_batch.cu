@@ -47,6 +47,8 @@ namespace {
 // Least payload the 3-pass columns of a mixed plan must hold to keep their form (about the
 // bytes HBM moves in the 40 us their extra launches take).
 constexpr uint64_t PLAN_3PASS_MIN_BYTES = 256ull << 20;
+// ... and the payload from which on a plan takes one form (103 columns of 303 MB, both / 3-pass: 110 / 97 us).
+constexpr uint64_t PLAN_LARGE_BYTES = 272ull << 20;
 
 inline int to_status(cudaError_t e)
 {
@@ -161,15 +163,19 @@ int cs_batch_create(cs_batch** out, const cs_column* cols, uint32_t ncols, const
         }
         for (uint32_t i = 0; i < ncols; ++i)
             one_pass[i] = cols[i].n && tune_batch_lookup(cols[i].n, cols[i].elem_bytes, sel[i]) == CS_ALGO_1PASS;
-        // Beside 1-pass columns, the 3-pass ones add a chain of their own (pass 1+2, a writeout
-        // per width: about 30 us of launches that wait on one another on B200), and what their form saves is at most their payload reads. Below
-        // PLAN_3PASS_MIN_BYTES of 3-pass payload they join the 1-pass kernels (batch256:
-        // 0.602 -> 0.571 ms per replay with its six sparse columns moved).
+        // A plan of both forms runs both chains of launches, one after the other (about 30 us on B200). So
+        // small plans, by what the 3-pass columns hold, and large ones take one form: the 3-pass form unless
+        // the columns that the table names 1-pass hold a quarter of the payload (3-pass / 1-pass, us, any
+        // selectivity: 28 columns of 9 MB 16 / 26, 101 of 40 MB 28 / 33, 256 of 2.2 GB 577 / 615).
         uint64_t bytes3 = 0, bytes1 = 0;
         for (uint32_t i = 0; i < ncols; ++i)
             (one_pass[i] ? bytes1 : bytes3) += cols[i].n * static_cast<uint64_t>(cols[i].elem_bytes);
-        if (bytes1 && bytes3 < PLAN_3PASS_MIN_BYTES)
-            for (uint32_t i = 0; i < ncols; ++i) one_pass[i] = cols[i].n ? 1 : 0;
+        const bool small = bytes3 < PLAN_3PASS_MIN_BYTES;
+        if (bytes1 && (small || bytes1 + bytes3 >= PLAN_LARGE_BYTES)) {
+            if (bytes1 < (bytes1 + bytes3) / 4) one_pass.assign(ncols, 0);
+            else if (small)
+                for (uint32_t i = 0; i < ncols; ++i) one_pass[i] = cols[i].n ? 1 : 0;
+        }
     }
     for (uint32_t i = 0; i < ncols; ++i) b->one_pass_cols += one_pass[i] && cols[i].n ? 1u : 0u;
 
