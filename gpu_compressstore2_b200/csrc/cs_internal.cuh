@@ -22,12 +22,14 @@ namespace cs {
 // needed: the last CTA of every look-back kernel advances the epoch. Epochs live in
 // [EPOCH_MIN, EPOCH_MAX]; the lower bound keeps any u32/u64 count or offset left in the
 // workspace by an earlier call from ever decoding as a valid status (their bits 42..63
-// are below 2^7). On wrap the workspace after the header is cleared, except the results
-// of the call that wrapped.
+// are below 2^7), the upper one an offset of POISON. Marks that a pass leaves beside them
+// (epoch_mark) have 17 bits, so two in one word do not decode as one either. On wrap the
+// workspace after the header is cleared, except the results of the call that wrapped,
+// and of those every word that reads as a status (wrap_clear).
 // ---------------------------------------------------------------------------------
 constexpr uint32_t WS_MAGIC = 0x43535753u; // "CSWS"
 constexpr uint32_t EPOCH_MIN = 128u;
-constexpr uint32_t EPOCH_MAX = (1u << 22) - 1u;
+constexpr uint32_t EPOCH_MAX = (1u << 22) - 2u;
 constexpr uint64_t STATUS_VALUE_MASK = (1ull << 40) - 1ull;
 constexpr uint32_t FLAG_AGG = 1u;
 constexpr uint32_t FLAG_PREFIX = 2u;
@@ -350,6 +352,37 @@ __host__ __device__ __forceinline__ uint32_t prev_epoch(uint32_t e)
     return e == EPOCH_MIN ? EPOCH_MAX : e - 1u;
 }
 
+// The mark that pass 1 leaves for its epoch: 17 bits, never 0 (a cleared word). A mark of an
+// earlier epoch that comes out the same costs its reader one look at the counts.
+__host__ __device__ __forceinline__ uint32_t epoch_mark(uint32_t e)
+{
+    return 1u + e % 131071u;
+}
+
+// The clear at the end of an epoch cycle, by all threads of the last CTA: everything after the header but
+// [keep_begin, keep_end), the regions of this call's results, and there (scrub: a plain call) the words
+// that read as a status. A call writes only a part of its regions, and an earlier one of another length
+// may have left its statuses in the rest, to be met again when their epoch comes round. A plan's
+// regions stay where they are, and hold maps, whose words may look like anything.
+__device__ __forceinline__ void wrap_clear(ws_header* hdr, uint64_t keep_begin, uint64_t keep_end, bool scrub)
+{
+    __syncthreads(); // this CTA's own results are written
+    uint4* p = reinterpret_cast<uint4*>(hdr);
+    const uint64_t n16 = hdr->ws_bytes / 16u;
+    const uint64_t k0 = keep_begin / 16u, k1 = (keep_end + 15u) / 16u;
+    for (uint64_t i = sizeof(ws_header) / 16u + threadIdx.x; i < n16; i += blockDim.x) {
+        if (i < k0 || i >= k1) {
+            p[i] = make_uint4(0, 0, 0, 0);
+            continue;
+        }
+        if (!scrub) continue;
+        uint64_t* const w = reinterpret_cast<uint64_t*>(p + i);
+        if (status_epoch(__ldcg(w)) >= EPOCH_MIN) w[0] = 0ull;
+        if (status_epoch(__ldcg(w + 1)) >= EPOCH_MIN) w[1] = 0ull;
+    }
+    __threadfence();
+}
+
 // End of a look-back kernel, in two steps. epilogue_ticket (every CTA, all threads) counts
 // the CTA as finished and returns, uniformly within the CTA, whether it was the last one.
 // epilogue_last (the last CTA only, all its threads) resets the dynamic tile counter,
@@ -378,12 +411,7 @@ __device__ __forceinline__ void epilogue_last(ws_header* hdr, uint32_t* tile_cou
     const uint32_t cur = vh->epoch;
     uint32_t next = cur + 1u;
     if (next > EPOCH_MAX) {
-        uint4* p = reinterpret_cast<uint4*>(hdr);
-        const uint64_t n16 = hdr->ws_bytes / 16u;
-        const uint64_t k0 = keep_begin / 16u, k1 = (keep_end + 15u) / 16u;
-        for (uint64_t i = sizeof(ws_header) / 16u + threadIdx.x; i < n16; i += blockDim.x)
-            if (i < k0 || i >= k1) p[i] = make_uint4(0, 0, 0, 0);
-        __threadfence();
+        wrap_clear(hdr, keep_begin, keep_end, is_scan);
         next = EPOCH_MIN;
     }
     // fold pass 1's per-CTA sparse flags (written before this point of the call)
@@ -391,7 +419,7 @@ __device__ __forceinline__ void epilogue_last(ws_header* hdr, uint32_t* tile_cou
     if (popc_flags) {
         const uint32_t nctas = vh->popc_ctas;
         const uint32_t nf = nctas < 2048u ? nctas : 2048u; // POPC_FLAG_SLOTS
-        for (uint32_t i = threadIdx.x; i < nf; i += blockDim.x) any_sparse |= (popc_flags[i] == cur) ? 1u : 0u;
+        for (uint32_t i = threadIdx.x; i < nf; i += blockDim.x) any_sparse |= (popc_flags[i] == epoch_mark(cur)) ? 1u : 0u;
     }
     any_sparse = __syncthreads_or(any_sparse);
     if (threadIdx.x == 0) {
@@ -409,18 +437,13 @@ __device__ __forceinline__ void epilogue_last(ws_header* hdr, uint32_t* tile_cou
 // epilogue_last for the reduce-then-scan pass (the last CTA, all its threads): `cur` is the
 // epoch the kernel read at its start, `any_sparse` whether a CTA saw a sparse block and
 // `clean` whether every CTA's waits completed (the pass has no look-back; only the streaming
-// form waits, on its own copies). Same wrap clear as epilogue_last.
+// form waits, on its own copies). `plain`: the pass of a plain call, not of a plan.
 __device__ __forceinline__ void epilogue_last_blocks(ws_header* hdr, uint32_t cur, bool any_sparse,
-                                                     uint64_t keep_begin, uint64_t keep_end, bool clean)
+                                                     uint64_t keep_begin, uint64_t keep_end, bool clean, bool plain)
 {
     uint32_t next = cur + 1u;
     if (next > EPOCH_MAX) {
-        uint4* q = reinterpret_cast<uint4*>(hdr);
-        const uint64_t n16 = hdr->ws_bytes / 16u;
-        const uint64_t k0 = keep_begin / 16u, k1 = (keep_end + 15u) / 16u;
-        for (uint64_t i = sizeof(ws_header) / 16u + threadIdx.x; i < n16; i += blockDim.x)
-            if (i < k0 || i >= k1) q[i] = make_uint4(0, 0, 0, 0);
-        __threadfence();
+        wrap_clear(hdr, keep_begin, keep_end, plain);
         next = EPOCH_MIN;
     }
     __syncthreads();

@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(256) k_popc_chunks_vec(const uint32_t* __restr
         __syncthreads();
         if (threadIdx.x == 0) {
             if (blockIdx.x == 0) hdr->popc_ctas = gridDim.x;
-            cta_flags[blockIdx.x] = s_sparse ? hdr->epoch : 0u;
+            cta_flags[blockIdx.x] = s_sparse ? epoch_mark(hdr->epoch) : 0u;
         }
     }
 }
@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(256) k_popc_chunks(const uint32_t* __restrict_
     const uint64_t total_warps = (static_cast<uint64_t>(gridDim.x) * blockDim.x) >> 5;
     if (hdr && blockIdx.x == 0 && threadIdx.x == 0) {
         hdr->popc_ctas = 1;
-        cta_flags[0] = hdr->epoch;
+        cta_flags[0] = epoch_mark(hdr->epoch);
     }
     if (wpc_log2 <= 5) {
         const uint32_t wpc = 1u << wpc_log2;
@@ -254,8 +254,8 @@ cudaError_t launch_scan(const ScanParams& p, int num_sms, cudaStream_t stream)
 // Pass 1 of the hybrid writeout: the units of block `bl` of a column (UE = 131072 / w
 // elements = 32 / w rows of 4096, always whole inside a 2^18-element block) whose count is
 // at most UE / 32 belong to the sparse gather: their 16K-element items get this call's
-// epoch in p.item_flags, and the gather visits only items so marked (a flag left by a call
-// one epoch cycle ago costs the gather one test of the offsets, never a wrong write).
+// epoch_mark in p.item_flags, and the gather visits only items so marked (an earlier call's mark that
+// is the same costs the gather one test of the offsets, never a wrong write).
 // s_warp / s_whalf: selected elements in each warp's 8 rows and in their first 4 rows.
 // Called by all threads after those are written.
 template <typename Col>
@@ -276,7 +276,8 @@ __device__ __forceinline__ void mark_sparse_units(const BlockScanParams& p, cons
     const uint64_t e0 = (bl << SCAN_BLOCK_LOG2) + static_cast<uint64_t>(t) * ue;
     if (e0 >= col.n || cnt > ue / 32) return;
     const uint64_t e1 = e0 + ue < col.n ? e0 + ue : col.n;
-    for (uint64_t it = e0 / 16384; it < (e1 + 16383) / 16384; ++it) p.item_flags[col.item_base + it] = epoch;
+    const uint32_t mark = epoch_mark(epoch);
+    for (uint64_t it = e0 / 16384; it < (e1 + 16383) / 16384; ++it) p.item_flags[col.item_base + it] = mark;
 }
 
 // ---------------------------------------------------------------------------------
@@ -477,7 +478,7 @@ __device__ __forceinline__ void popc_blocks_finish_grid(const BlockScanParams& p
     __threadfence(); // every other CTA's block sums (and any poison mark) are visible
     const bool clean = reinterpret_cast<volatile ws_header*>(p.hdr)->poison_epoch != epoch;
     blocks_last_cta(p, s_scan, clean, s_prefix, prefix_room);
-    epilogue_last_blocks(p.hdr, epoch, (fin & 2u) != 0u, p.keep_begin, p.keep_end, clean);
+    epilogue_last_blocks(p.hdr, epoch, (fin & 2u) != 0u, p.keep_begin, p.keep_end, clean, p.cols == nullptr);
 }
 
 template <int LPC>

@@ -127,7 +127,7 @@ __device__ __forceinline__ void sparse_groups(const ColumnDesc& c, uint64_t e0, 
     const uint64_t u0 = e0 & ~(UE - 1);                                  // an item never straddles units
     const uint64_t off_b = chunk_offset(c, u0 >> chunk_log2, chunk_log2);
     const uint64_t off_e = u0 + UE >= n ? *c.d_count : chunk_offset(c, (u0 + UE) >> chunk_log2, chunk_log2);
-    if (off_e - off_b > UE / 32) return; // a mark of an earlier epoch cycle: the dense part owns the unit
+    if (off_e - off_b > UE / 32) return; // an earlier call's mark: the dense part owns the unit
 
     uint32_t rank[GROUPS], cnt[GROUPS]; // rank of the lane's first selected element of each group
     uint32_t total = 0;
@@ -347,10 +347,10 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS<SHIFT>) k_writeout_warp(const
     }
 
     if (!hybrid) return;
-    // The items of sparse units. Those that pass 1 marked carry the epoch of that pass, the one
+    // The items of sparse units. Those that pass 1 marked carry the mark of that pass's epoch, the one
     // before the current; without marks every item is tested. A warp looks at 32 work items at
     // a time, taken round robin over all warps so that marked items spread evenly.
-    const uint32_t mark = p.item_flags ? prev_epoch(*reinterpret_cast<const volatile uint32_t*>(&p.hdr->epoch)) : 0u;
+    const uint32_t mark = p.item_flags ? epoch_mark(prev_epoch(*reinterpret_cast<const volatile uint32_t*>(&p.hdr->epoch))) : 0u;
     uint16_t* const list = reinterpret_cast<uint16_t*>(stage);
     const uint32_t split = p.num_sparse_items * 4 <= 2ull * total_warps ? 4u : 1u; // work items per 16K-element item
     const uint64_t num_work = p.num_sparse_items * split;
