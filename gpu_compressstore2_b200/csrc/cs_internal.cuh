@@ -308,12 +308,23 @@ __device__ __forceinline__ uint64_t lookback_cta(uint64_t* status, uint64_t tile
     return excl;
 }
 
+// What a slice publishes: its total beside the upper bits of an AGG status of the epoch.
+__device__ __forceinline__ uint32_t slice_tag(uint32_t epoch)
+{
+    return epoch << 2 | FLAG_AGG;
+}
+__device__ __forceinline__ uint64_t slice_status(uint32_t tag, uint32_t total)
+{
+    return static_cast<uint64_t>(tag) << 40 | total;
+}
+
 // Sum of the totals published for slices [from, to), read by a whole CTA of NT threads: a thread
-// polls its slices' statuses (any flag but POISON of this epoch), each warp leaves its part of the
-// sum in red[0 .. NT / 32). Returns, per thread, whether all of them appeared in time; the caller
-// adds up `red` after a barrier. For to - from <= 2 * NT and slices of less than 2^22 elements.
+// polls its slices' statuses (published: with this epoch's slice_tag, the only one that slices write), each
+// warp leaves its part of the sum in red[0 .. NT / 32). Returns, per thread, whether all of them appeared
+// in time; the caller adds up `red` after a barrier. For to - from <= 2 * NT and slices of less than
+// 2^22 elements.
 template <int NT>
-__device__ __forceinline__ bool poll_totals(const uint64_t* status, uint32_t from, uint32_t to, uint32_t epoch,
+__device__ __forceinline__ bool poll_totals(const uint64_t* status, uint32_t from, uint32_t to, uint32_t tag,
                                             uint64_t timeout_ns, uint32_t* red)
 {
     uint32_t sum = 0;
@@ -322,12 +333,12 @@ __device__ __forceinline__ bool poll_totals(const uint64_t* status, uint32_t fro
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
         const uint32_t at = from + threadIdx.x + i * NT;
-        s[i] = at < to ? ld_relaxed_gpu(status + at) : pack_status(epoch, FLAG_AGG, 0);
+        s[i] = at < to ? ld_relaxed_gpu(status + at) : slice_status(tag, 0u);
     }
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
         const uint32_t at = from + threadIdx.x + i * NT;
-        if (status_epoch(s[i]) != epoch) {
+        if (static_cast<uint32_t>(s[i] >> 40) != tag) {
             const uint64_t t0 = globaltimer_ns();
             uint32_t spins = 0;
             do {
@@ -335,9 +346,9 @@ __device__ __forceinline__ bool poll_totals(const uint64_t* status, uint32_t fro
                 s[i] = ld_relaxed_gpu(status + at);
                 if ((++spins & 63u) == 0u && globaltimer_ns() - t0 > timeout_ns) {
                     ok = false;
-                    s[i] = pack_status(epoch, FLAG_AGG, 0);
+                    s[i] = slice_status(tag, 0u);
                 }
-            } while (status_epoch(s[i]) != epoch);
+            } while (static_cast<uint32_t>(s[i] >> 40) != tag);
         }
         sum += static_cast<uint32_t>(status_value(s[i]));
     }

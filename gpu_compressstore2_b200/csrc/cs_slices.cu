@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS) k_if(const SliceParams p)
         for (uint32_t t = 0; t < 4; ++t) s_sum[t] = 0u;
     }
     __syncthreads();
-    const uint32_t epoch = s_epoch;
+    const uint32_t tag = slice_tag(s_epoch); // the epoch, but for two bits
 
     auto item_elem = [&](uint32_t slice) -> uint64_t { return (static_cast<uint64_t>(slice) * WARPS + warp) * ITEM; };
     // the lane's 32 bytes of row r of the item at e0, where the column ends in or before the item:
@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS) k_if(const SliceParams p)
             const uint32_t before = atomicAdd(&s_sum[turn], cnt + (1u << 24));
             if (before >> 24 == WARPS - 1) {
                 s_sum[turn] = 0u; // used again four turns on, past a barrier
-                st_relaxed_gpu(&p.status[slice], pack_status(epoch, FLAG_AGG, (before & 0xffffffu) + cnt));
+                st_relaxed_gpu(&p.status[slice], slice_status(tag, (before & 0xffffffu) + cnt));
             }
         }
         if (!MASKED && p.mask) {
@@ -266,6 +266,7 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS) k_if(const SliceParams p)
     auto leave = [&]() {
         if (atomicAdd(&p.hdr->done_counter, 1u) != gridDim.x - 1) return;
         volatile ws_header* vh = p.hdr;
+        const uint32_t epoch = tag >> 2;
         if (vh->poison_epoch == epoch) *p.d_count = COUNT_ERROR;
         uint32_t following = epoch + 1u;
         if (following > EPOCH_MAX) {
@@ -315,13 +316,13 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS) k_if(const SliceParams p)
         // the totals of the slices since this CTA's last one, 512 at a time
         uint32_t* const red = s_red[turn & 1u];
         for (; slice - done > 2 * WARPS * 32; done += 2 * WARPS * 32) {
-            if (!poll_totals<WARPS * 32>(p.status, done, done + 2 * WARPS * 32, epoch, p.timeout_ns, red)) s_failed = 1u;
+            if (!poll_totals<WARPS * 32>(p.status, done, done + 2 * WARPS * 32, tag, p.timeout_ns, red)) s_failed = 1u;
             __syncthreads();
 #pragma unroll
             for (uint32_t w = 0; w < WARPS; ++w) end += red[w];
             __syncthreads();
         }
-        if (!poll_totals<WARPS * 32>(p.status, done, slice, epoch, s_failed ? 0ull : p.timeout_ns, red)) s_failed = 1u;
+        if (!poll_totals<WARPS * 32>(p.status, done, slice, tag, s_failed ? 0ull : p.timeout_ns, red)) s_failed = 1u;
         if (more) evaluate(next, m, x, ahead, later);
         if constexpr (!MASKED) load_selected();
         __syncthreads(); // the sums of this turn; every warp has left the turn before
@@ -334,7 +335,7 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS) k_if(const SliceParams p)
         if (threadIdx.x == 0) {
             if (failed) {
                 record_error(p.hdr, DEVERR_LOOKBACK_TIMEOUT);
-                reinterpret_cast<volatile ws_header*>(p.hdr)->poison_epoch = epoch;
+                reinterpret_cast<volatile ws_header*>(p.hdr)->poison_epoch = tag >> 2;
             }
             if (slice == p.num_slices - 1) *p.d_count = end;
             if (s_slice[(turn + 1) & 3u] >= p.num_slices) { // the CTA's last slice
