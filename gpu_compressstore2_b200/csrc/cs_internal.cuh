@@ -320,15 +320,16 @@ __device__ __forceinline__ uint64_t slice_status(uint32_t tag, uint32_t total)
 
 // Sum of the totals published for slices [from, to), read by a whole CTA of NT threads: a thread
 // polls its slices' statuses (published: with this epoch's slice_tag, the only one that slices write), each
-// warp leaves its part of the sum in red[0 .. NT / 32). Returns, per thread, whether all of them appeared
-// in time; the caller adds up `red` after a barrier. For to - from <= 2 * NT and slices of less than
-// 2^22 elements.
-template <int NT>
-__device__ __forceinline__ bool poll_totals(const uint64_t* status, uint32_t from, uint32_t to, uint32_t tag,
-                                            uint64_t timeout_ns, uint32_t* red)
+// warp leaves its part of the sum in red[0 .. NT / 32); the caller adds up `red` after a barrier. Returns,
+// per thread, 0 or what went wrong: a total that did not appear in time, or one larger than a slice of
+// MOST elements, so that no sum leads past the column's end. For to - from <= 2 * NT.
+template <int NT, uint32_t MOST>
+__device__ __forceinline__ uint32_t poll_totals(const uint64_t* status, uint32_t from, uint32_t to, uint32_t tag,
+                                                uint64_t timeout_ns, uint32_t* red)
 {
     uint32_t sum = 0;
-    bool ok = true;
+    uint32_t wrong = 0;
+    static_assert(MOST < 1u << 22, "sums of 2 * NT totals in 32 bits");
     uint64_t s[2];
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
@@ -345,17 +346,19 @@ __device__ __forceinline__ bool poll_totals(const uint64_t* status, uint32_t fro
                 __nanosleep(spins < 16 ? 20 : 100);
                 s[i] = ld_relaxed_gpu(status + at);
                 if ((++spins & 63u) == 0u && globaltimer_ns() - t0 > timeout_ns) {
-                    ok = false;
+                    wrong = DEVERR_LOOKBACK_TIMEOUT;
                     s[i] = slice_status(tag, 0u);
                 }
             } while (static_cast<uint32_t>(s[i] >> 40) != tag);
         }
-        sum += static_cast<uint32_t>(status_value(s[i]));
+        const uint32_t total = static_cast<uint32_t>(s[i]);
+        if (total > MOST) wrong = DEVERR_RANGE;
+        sum += total;
     }
     __syncwarp();
     sum = __reduce_add_sync(0xffffffffu, sum);
     if ((threadIdx.x & 31u) == 0u) red[threadIdx.x >> 5] = sum;
-    return ok;
+    return wrong;
 }
 
 __host__ __device__ __forceinline__ uint32_t prev_epoch(uint32_t e)

@@ -12,9 +12,10 @@
 //   writes    the present slice: loads the payload (a comparison's again, now from L2), places and
 //             stores the selected elements (an item with few is listed and gathered instead).
 // The warps of a CTA meet at one barrier per turn. A CTA only ever waits for slices that running
-// CTAs already hold, in order. Waits are bounded; one that gives up records an error, the CTA
-// writes nothing more and the count reads CS_COUNT_ERROR. The epoch closes as soon as the last CTA
-// has summed up for the last time, so nothing follows the writes (2^20 u32: 7.1 -> 5.4 us).
+// CTAs already hold, in order. Waits are bounded; a CTA that gives one up, or reads a total that no
+// slice can have, records an error and writes nothing more, and the count reads CS_COUNT_ERROR. The epoch
+// closes as soon as the last CTA has summed up for the last time, so nothing follows the writes (2^20
+// u32: 7.1 -> 5.4 us).
 //
 // What bounds the predicate is instructions: the evaluation and the placing together take about as long as
 // 16 warps' issue of an SM allows while the payload streams at 4 to 5 TB/s. Per call on B200
@@ -113,7 +114,7 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS) k_if(const SliceParams p)
     __shared__ __align__(16) uint32_t s_total[4][WARPS]; // selected elements of each warp's part of it
     __shared__ uint32_t s_sum[4];                        // of the warps that have counted so far, and their number (bits 24 on)
     __shared__ __align__(16) uint32_t s_red[2][WARPS];   // parts of the sum of the totals since this CTA's last slice
-    __shared__ uint32_t s_epoch, s_failed;
+    __shared__ uint32_t s_epoch, s_failed; // s_failed: what went wrong
     static_assert(WARPS == 8, "two vectors of warp totals");
     using U = typename std::conditional<sizeof(T) == 1, uint8_t, typename std::conditional<sizeof(T) == 2, uint16_t,
               typename std::conditional<sizeof(T) == 4, uint32_t, uint64_t>::type>::type>::type;
@@ -316,13 +317,15 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS) k_if(const SliceParams p)
         // the totals of the slices since this CTA's last one, 512 at a time
         uint32_t* const red = s_red[turn & 1u];
         for (; slice - done > 2 * WARPS * 32; done += 2 * WARPS * 32) {
-            if (!poll_totals<WARPS * 32>(p.status, done, done + 2 * WARPS * 32, tag, p.timeout_ns, red)) s_failed = 1u;
+            const uint32_t wrong = poll_totals<WARPS * 32, WARPS * ITEM>(p.status, done, done + 2 * WARPS * 32, tag, p.timeout_ns, red);
+            if (wrong) s_failed = wrong;
             __syncthreads();
 #pragma unroll
             for (uint32_t w = 0; w < WARPS; ++w) end += red[w];
             __syncthreads();
         }
-        if (!poll_totals<WARPS * 32>(p.status, done, slice, tag, s_failed ? 0ull : p.timeout_ns, red)) s_failed = 1u;
+        const uint32_t wrong = poll_totals<WARPS * 32, WARPS * ITEM>(p.status, done, slice, tag, s_failed ? 0ull : p.timeout_ns, red);
+        if (wrong) s_failed = wrong;
         if (more) evaluate(next, m, x, ahead, later);
         if constexpr (!MASKED) load_selected();
         __syncthreads(); // the sums of this turn; every warp has left the turn before
@@ -334,7 +337,7 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS) k_if(const SliceParams p)
         const bool failed = s_failed != 0u;
         if (threadIdx.x == 0) {
             if (failed) {
-                record_error(p.hdr, DEVERR_LOOKBACK_TIMEOUT);
+                record_error(p.hdr, s_failed);
                 reinterpret_cast<volatile ws_header*>(p.hdr)->poison_epoch = tag >> 2;
             }
             if (slice == p.num_slices - 1) *p.d_count = end;

@@ -43,3 +43,11 @@ def test_another_flag_is_no_total(cuda, oracle):
     import gpu_compressstore2_b200 as cs
 
     _refused(oracle, POISON, 0, cs._lib.ERR_TIMEOUT)
+
+
+def test_a_total_larger_than_a_slice(cuda, oracle):
+    """It would lead past the end of the output."""
+    import gpu_compressstore2_b200 as cs
+
+    for value in (8193, 1 << 30, (1 << 32) - 1):
+        _refused(oracle, AGG, value, cs._lib.ERR_INVALID_VALUE)
