@@ -266,6 +266,7 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS) k_if(const SliceParams p)
     // epoch, and takes the count back if a wait gave up anywhere.
     auto leave = [&]() {
         if (atomicAdd(&p.hdr->done_counter, 1u) != gridDim.x - 1) return;
+        __threadfence(); // the other CTAs' mark and count, before the mark is read and the count replaced
         volatile ws_header* vh = p.hdr;
         const uint32_t epoch = tag >> 2;
         if (vh->poison_epoch == epoch) *p.d_count = COUNT_ERROR;
