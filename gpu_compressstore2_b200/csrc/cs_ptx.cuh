@@ -165,6 +165,13 @@ __device__ __forceinline__ uint64_t ld_relaxed_gpu(const uint64_t* p)
     return v;
 }
 
+__device__ __forceinline__ uint32_t atom_add_acquire_gpu(uint32_t* p, uint32_t v)
+{
+    uint32_t old;
+    asm volatile("atom.add.acquire.gpu.global.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
+    return old;
+}
+
 __device__ __forceinline__ void st_relaxed_gpu(uint64_t* p, uint64_t v)
 {
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");

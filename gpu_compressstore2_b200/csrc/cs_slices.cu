@@ -265,8 +265,9 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS) k_if(const SliceParams p)
     // Thread 0 of every CTA, once its CTA has summed up for the last time: the last one to come closes the
     // epoch, and takes the count back if a wait gave up anywhere.
     auto leave = [&]() {
-        if (atomicAdd(&p.hdr->done_counter, 1u) != gridDim.x - 1) return;
-        __threadfence(); // the other CTAs' mark and count, before the mark is read and the count replaced
+        // acquire: the other CTAs' mark and count, before the mark is read and the count replaced (a fence
+        // here costs 0.4 us at 2^20 u32: it waits for this thread's own stores)
+        if (atom_add_acquire_gpu(&p.hdr->done_counter, 1u) != gridDim.x - 1) return;
         volatile ws_header* vh = p.hdr;
         const uint32_t epoch = tag >> 2;
         if (vh->poison_epoch == epoch) *p.d_count = COUNT_ERROR;
