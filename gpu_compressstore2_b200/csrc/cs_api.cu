@@ -226,12 +226,14 @@ ColumnDesc make_column(const void* d_in, const void* d_mask, void* d_out, uint64
 
 // Pass 3 of the 3-pass form over chunk offsets already in the workspace: independent warps for
 // chunk lengths up to 4096 (hybrid: units with at most 1/32 selected are gathered), the
-// TMA-staged writeout for longer ones.
+// TMA-staged writeout for longer ones and for skip = 2 (whole tiles are loaded, which warps never do), if
+// the pointers allow it.
 int launch_writeout_3pass(const ColumnDesc& col, const Layout& l, ws_header* hdr, const Resolved& r, bool hybrid,
                           const uint32_t* item_flags, const DeviceInfo& di, cudaStream_t stream)
 {
     const uint32_t elem_bytes = col.elem_bytes;
-    if (r.chunk_log2 <= 12) {
+    const bool whole_tiles = !r.skip && aligned(col.in, 16) && aligned(col.out, 16) && aligned(col.mask, 16);
+    if (r.chunk_log2 <= 12 && !whole_tiles) {
         WriteoutParams p{};
         p.col0 = col;
         p.num_units = l.num_tiles;
@@ -268,11 +270,12 @@ int run_compaction(const void* d_in, const void* d_mask, void* d_out, uint64_t n
     int algo = r.algo;
     const bool tma_ok = aligned(d_in, 16) && aligned(d_out, 16) && aligned(d_mask, 16);
     // The 1-pass form runs in slices (cs_slices.cu), or through the TMA kernel for 4- and 8-byte columns of
-    // more than slices_per_sm. The slices' totals lie where the 3-pass form has its chunk offsets (which
-    // never read as a status); a caller's chunk length may leave less room than that.
+    // more than slices_per_sm and for skip = 2 (as in launch_writeout_3pass). The slices' totals lie where
+    // the 3-pass form has its chunk offsets (which never read as a status); a caller's chunk length may leave
+    // less room than that.
     const uint64_t slices = slices_of(n, elem_bytes);
     const bool in_slices =
-        slices <= l.num_chunks &&
+        r.skip && slices <= l.num_chunks &&
         (elem_bytes <= 2 || slices <= slices_per_sm(elem_bytes) * static_cast<uint64_t>(di.sms));
     if ((algo == CS_ALGO_1PASS || algo == CS_ALGO_3PASS) && !tma_ok) {
         if (!auto_route) return CS_ERR_MISALIGNED;
