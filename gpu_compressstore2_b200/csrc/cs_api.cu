@@ -270,12 +270,12 @@ int run_compaction(const void* d_in, const void* d_mask, void* d_out, uint64_t n
     int algo = r.algo;
     const bool tma_ok = aligned(d_in, 16) && aligned(d_out, 16) && aligned(d_mask, 16);
     // The 1-pass form runs in slices (cs_slices.cu), or through the TMA kernel for 4- and 8-byte columns of
-    // more than slices_per_sm and for skip = 2 (as in launch_writeout_3pass). The slices' totals lie where
-    // the 3-pass form has its chunk offsets (which never read as a status); a caller's chunk length may leave
-    // less room than that.
+    // more than slices_per_sm and for skip = 2 (as in launch_writeout_3pass). The slices' totals take the
+    // workspace from its look-back statuses on, where a 1-pass call has nothing else: room for 1.19 times as
+    // many and more, whatever the chunk length (the least: 2-byte elements, 65536).
     const uint64_t slices = slices_of(n, elem_bytes);
     const bool in_slices =
-        r.skip && slices <= l.num_chunks &&
+        r.skip && 8 * slices <= l.total - l.off_status &&
         (elem_bytes <= 2 || slices <= slices_per_sm(elem_bytes) * static_cast<uint64_t>(di.sms));
     if ((algo == CS_ALGO_1PASS || algo == CS_ALGO_3PASS) && !tma_ok) {
         if (!auto_route) return CS_ERR_MISALIGNED;
@@ -293,7 +293,7 @@ int run_compaction(const void* d_in, const void* d_mask, void* d_out, uint64_t n
         p.n = n;
         p.d_count = d_count;
         p.hdr = hdr;
-        p.status = reinterpret_cast<uint64_t*>(ws + l.off_offsets);
+        p.status = reinterpret_cast<uint64_t*>(ws + l.off_status);
         p.timeout_ns = r.timeout_ns;
         p.grid = r.grid;
         return cuda_status(launch_onepass(p, elem_bytes, di.sms, stream));
