@@ -271,6 +271,12 @@ __global__ void __launch_bounds__(Roles<MODE>::NTHREADS, 1) k_compact_tma(const 
     if (MODE == 0) __syncthreads();
     const uint32_t epoch = (MODE == 0) ? p.hdr->epoch : 0u;
     const bool scan_ok = (hflags & 1u) != 0u; // 3-pass: pass 2 completed cleanly
+    // a warp whose wait ran out: this CTA leaves units unfinished
+    auto give_up = [&]() {
+        if (lane != 0) return;
+        record_error(p.hdr, DEVERR_PIPELINE_TIMEOUT);
+        if (MODE == 0) reinterpret_cast<volatile ws_header*>(p.hdr)->lost_epoch = epoch;
+    };
 
     if (warp == 0) {
         // ------------------------------------------------------------- producer
@@ -300,7 +306,7 @@ __global__ void __launch_bounds__(Roles<MODE>::NTHREADS, 1) k_compact_tma(const 
             const uint32_t slot = j % MSLOTS;
             if (j >= (uint32_t)MSLOTS &&
                 !mbar_wait_warp(&mask_empty[slot], ((j / MSLOTS) - 1) & 1u, p.timeout_ns, lane)) {
-                if (lane == 0) record_error(p.hdr, DEVERR_PIPELINE_TIMEOUT);
+                give_up();
                 return false;
             }
             if (unit >= p.num_tiles) { // num_tiles holds the unit count
@@ -383,7 +389,7 @@ __global__ void __launch_bounds__(Roles<MODE>::NTHREADS, 1) k_compact_tma(const 
             // the unit's mask must have landed before segments can be skipped
             const bool use_skip = p.skip != 0u;
             if (use_skip && !mbar_wait_warp(&mask_full[slot], (j / MSLOTS) & 1u, p.timeout_ns, lane)) {
-                if (lane == 0) record_error(p.hdr, DEVERR_PIPELINE_TIMEOUT);
+                give_up();
                 failed = true;
                 break;
             }
@@ -391,7 +397,7 @@ __global__ void __launch_bounds__(Roles<MODE>::NTHREADS, 1) k_compact_tma(const 
                 const uint32_t s = tseq % S;
                 const uint32_t u = tseq / S;
                 if (u > 0 && !mbar_wait_warp(&empty_pay[s], (u - 1) & 1u, p.timeout_ns, lane)) {
-                    if (lane == 0) record_error(p.hdr, DEVERR_PIPELINE_TIMEOUT);
+                    give_up();
                     failed = true;
                     break;
                 }
@@ -471,7 +477,7 @@ __global__ void __launch_bounds__(Roles<MODE>::NTHREADS, 1) k_compact_tma(const 
         for (uint32_t j = 0;; ++j) {
             const uint32_t slot = j % MSLOTS;
             if (!mbar_wait_warp(&mask_full[slot], (j / MSLOTS) & 1u, p.timeout_ns, lane)) {
-                if (lane == 0) record_error(p.hdr, DEVERR_PIPELINE_TIMEOUT);
+                give_up();
                 break;
             }
             const int64_t unit = meta[slot].unit;
@@ -522,7 +528,7 @@ __global__ void __launch_bounds__(Roles<MODE>::NTHREADS, 1) k_compact_tma(const 
         for (uint32_t j = 0;; ++j) {
             const uint32_t slot = j % MSLOTS;
             if (!mbar_wait_warp(&counted[slot], (j / MSLOTS) & 1u, p.timeout_ns, lane)) {
-                if (lane == 0) record_error(p.hdr, DEVERR_PIPELINE_TIMEOUT);
+                give_up();
                 break;
             }
             const int64_t unit = meta[slot].unit;
@@ -556,7 +562,7 @@ __global__ void __launch_bounds__(Roles<MODE>::NTHREADS, 1) k_compact_tma(const 
         for (uint32_t j = 0; !failed; ++j) {
             const uint32_t slot = j % MSLOTS;
             if (!mbar_wait_warp(&ready[slot], (j / MSLOTS) & 1u, p.timeout_ns, lane)) {
-                if (lane == 0) record_error(p.hdr, DEVERR_PIPELINE_TIMEOUT);
+                give_up();
                 break;
             }
             const int64_t unit = meta[slot].unit;
@@ -570,7 +576,7 @@ __global__ void __launch_bounds__(Roles<MODE>::NTHREADS, 1) k_compact_tma(const 
             for (uint32_t k = 0; k < ntiles; ++k, ++tseq) {
                 const uint32_t s = tseq % S;
                 if (!mbar_wait_warp(&full_pay[s], (tseq / S) & 1u, p.timeout_ns, lane)) {
-                    if (lane == 0) record_error(p.hdr, DEVERR_PIPELINE_TIMEOUT);
+                    give_up();
                     failed = true;
                     break;
                 }
@@ -611,9 +617,12 @@ __global__ void __launch_bounds__(Roles<MODE>::NTHREADS, 1) k_compact_tma(const 
         }
     }
 
-    if (MODE == 0)
-        lookback_kernel_epilogue(p.hdr, &p.hdr->tile_counter, &p.hdr->done_counter, &s_flag, false, p.keep_begin,
-                                 p.keep_end);
+    if (MODE == 0 && epilogue_ticket(&p.hdr->done_counter, &s_flag)) {
+        // units left unfinished: a column's count comes from its last unit, which may be one of them
+        if (reinterpret_cast<volatile ws_header*>(p.hdr)->lost_epoch == epoch)
+            for (uint64_t u = threadIdx.x; u < p.num_tiles; u += blockDim.x) *col_of_unit(u).d_count = COUNT_ERROR;
+        epilogue_last(p.hdr, &p.hdr->tile_counter, &p.hdr->done_counter, false, p.keep_begin, p.keep_end, nullptr);
+    }
 }
 
 // ---------------------------------------------------------------------------------

@@ -58,7 +58,7 @@ struct alignas(256) ws_header {
     uint32_t scan_ok_epoch;     // epoch of the latest scan that completed with no poisoned tile
     uint32_t sparse_epoch;      // epoch of the latest pass 1 that saw a sparse 16K block
     uint32_t popc_ctas;         // CTAs of the latest pass 1 (entries of its flag array)
-    uint32_t reserved0;
+    uint32_t lost_epoch;        // epoch of the latest 1-pass launch in which a CTA left units unfinished
     uint64_t count_word;        // a count slot inside the header: a caller that points d_count here
                                 // reads count and error word back with one copy of the header
     uint64_t reserved1[24];
@@ -439,8 +439,8 @@ __device__ __forceinline__ void epilogue_last(ws_header* hdr, uint32_t* tile_cou
     if (threadIdx.x == 0) {
         if (any_sparse) vh->sparse_epoch = cur;
         if (is_scan && vh->poison_epoch != cur) vh->scan_ok_epoch = cur; // == prev_epoch(next)
-        // a new epoch cycle must not meet an old cycle's poison mark (0 is no epoch)
-        if (next == EPOCH_MIN) vh->poison_epoch = 0u;
+        // a new epoch cycle must not meet an old cycle's marks (0 is no epoch)
+        if (next == EPOCH_MIN) vh->poison_epoch = vh->lost_epoch = 0u;
         *tile_counter = 0u;
         *done_counter = 0u;
         vh->epoch = next;
@@ -465,7 +465,7 @@ __device__ __forceinline__ void epilogue_last_blocks(ws_header* hdr, uint32_t cu
         volatile ws_header* vh = hdr;
         if (any_sparse) vh->sparse_epoch = cur;
         if (clean) vh->scan_ok_epoch = cur;
-        if (next == EPOCH_MIN) vh->poison_epoch = 0u;
+        if (next == EPOCH_MIN) vh->poison_epoch = vh->lost_epoch = 0u;
         vh->scan_tile_counter = 0u;
         vh->scan_done_counter = 0u;
         vh->epoch = next;

@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS) k_if(const SliceParams p)
         if (following > EPOCH_MAX) {
             uint4* w = reinterpret_cast<uint4*>(p.hdr);
             for (uint64_t i = sizeof(ws_header) / 16u; i < vh->ws_bytes / 16u; ++i) w[i] = make_uint4(0, 0, 0, 0);
-            vh->poison_epoch = 0u; // a new cycle must not meet an old one's mark
+            vh->poison_epoch = vh->lost_epoch = 0u; // a new cycle must not meet an old one's marks
             following = EPOCH_MIN;
         }
         vh->tile_counter = 0u;
