@@ -27,9 +27,7 @@
 namespace cs {
 
 // Chunk length of a plan's 3-pass columns: the smallest item of the writeout (4 KB of 8-byte
-// elements), so that no item starts inside a chunk. (With 4096-element chunks a warp popcounts
-// the chunk before its item: the plain call at 2^28 f32 takes 297 us instead of 268, at 2^27 u64
-// 288 instead of 255.)
+// elements), so that no item starts inside a chunk (the plans' writeout has no form for that).
 constexpr uint32_t PLAN_CHUNK_LOG2 = 9;
 
 struct PlanCounts {

@@ -181,7 +181,12 @@ __device__ __forceinline__ void sparse_groups(const ColumnDesc& c, uint64_t e0, 
     }
 }
 
-template <typename T, bool MULTI, bool SHIFT>
+// LONG: chunks longer than an item, which may then start inside one: the selected elements of the chunk before
+// it come from its mask, one vector per lane, asked for with the item's own mask. (Word by word behind the
+// payload's loads: 3-pass calls at chunk 4096, us, 2^27 u64 p = 0.5 286 -> 256, 0.9 382 -> 328, 2^28 u32 0.5 297
+// -> 267, 0.9 396 -> 343, 2^28 u16 0.5 168 -> 155; 2^22 u64 17.6 -> 18.2.) A kernel of its own: in the other one
+// its registers cost 2^28 u32 at chunk 1024 265 -> 296.
+template <typename T, bool MULTI, bool SHIFT, bool LONG>
 __global__ void __launch_bounds__(WARPS * 32, CTAS<SHIFT>) k_writeout_warp(const WriteoutParams p)
 {
     constexpr uint32_t EPL = LANE_BYTES / sizeof(T); // elements per lane and row
@@ -260,6 +265,7 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS<SHIFT>) k_writeout_warp(const
     };
 
     uint32_t m[ROWS]; // the present item's mask bits, loaded one item ahead
+    uint4 head = make_uint4(0u, 0u, 0u, 0u); // LONG: and a lane's share of its chunk's mask before it
     auto load_mask = [&](uint32_t it) {
         const ColumnDesc& C = column(it);
         const uint64_t e0 = first_elem(C, it);
@@ -275,6 +281,16 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS<SHIFT>) k_writeout_warp(const
             }
             m[r] = v;
         }
+        if constexpr (LONG) {
+            // less than a chunk of 4096 elements: 128 words, four to a lane
+            const uint64_t w0 = ((e0 >> p.chunk_log2) << p.chunk_log2) >> 5;
+            head = make_uint4(0u, 0u, 0u, 0u);
+            if (e0 < C.n && lane * 4u < static_cast<uint32_t>((e0 >> 5) - w0)) {
+                const uint32_t* hw = C.mask + w0 + lane * 4u;
+                if ((reinterpret_cast<uintptr_t>(C.mask) & 15u) == 0) head = __ldg(reinterpret_cast<const uint4*>(hw));
+                else head = make_uint4(__ldg(hw), __ldg(hw + 1), __ldg(hw + 2), __ldg(hw + 3));
+            }
+        }
     };
     uint32_t it = next_item();
     if (it != NONE) load_mask(it);
@@ -287,6 +303,8 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS<SHIFT>) k_writeout_warp(const
             if (it != NONE) load_mask(it);
             continue;
         }
+        uint32_t before = 0; // selected elements of the chunk before the item
+        if constexpr (LONG) before = __reduce_add_sync(0xffffffffu, __popc(head.x) + __popc(head.y) + __popc(head.z) + __popc(head.w));
         uint32_t bits[ROWS];
         uint32_t x[ROWS][8];
         const uint8_t* src = C.in + e0 * sizeof(T) + lane * LANE_BYTES;
@@ -323,12 +341,6 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS<SHIFT>) k_writeout_warp(const
         const uint64_t ch = e0 >> p.chunk_log2;
         const uint64_t off0 = C.offsets[ch];
         const uint64_t blk = C.blk_base ? C.blk_base[ch >> (SCAN_BLOCK_LOG2 - p.chunk_log2)] : 0ull;
-        uint32_t before = 0;
-        if (ITEM_LOG2 < p.chunk_log2) {
-            // the item starts inside a chunk: the selected elements of the chunk before it
-            for (uint64_t w = ((ch << p.chunk_log2) >> 5) + lane; w < e0 >> 5; w += 32) before += __popc(__ldg(C.mask + w));
-            before = __reduce_add_sync(0xffffffffu, before);
-        }
         it = next_item();
         if (it != NONE) load_mask(it);
         const uint64_t start = off0 + blk; // of the chunk
@@ -383,9 +395,12 @@ cudaError_t launch_t(const WriteoutParams& p, uint32_t requested, int num_sms, c
     pp.throttle = !p.cols && p.col0.d_count && items >= 8 * blocks * WARPS ? throttle_warps<T> : 0u;
     const dim3 g(static_cast<unsigned>(blocks)), b(WARPS * 32);
     cudaError_t e;
-    if constexpr (SHIFT) e = launch_pdl(k_writeout_warp<T, false, true>, g, b, 0, stream, pp);
-    else e = p.cols ? launch_pdl(k_writeout_warp<T, true, false>, g, b, 0, stream, pp)
-                    : launch_pdl(k_writeout_warp<T, false, false>, g, b, 0, stream, pp);
+    const bool inside = (1u << p.chunk_log2) > ITEM_BYTES / sizeof(T); // items that start inside a chunk
+    if (SHIFT && sizeof(T) > 1 && inside) e = launch_pdl(k_writeout_warp<T, false, SHIFT, (sizeof(T) > 1)>, g, b, 0, stream, pp);
+    else if (SHIFT) e = launch_pdl(k_writeout_warp<T, false, SHIFT, false>, g, b, 0, stream, pp);
+    else if (p.cols) e = launch_pdl(k_writeout_warp<T, true, false, false>, g, b, 0, stream, pp);
+    else if (sizeof(T) > 1 && inside) e = launch_pdl(k_writeout_warp<T, false, false, (sizeof(T) > 1)>, g, b, 0, stream, pp);
+    else e = launch_pdl(k_writeout_warp<T, false, false, false>, g, b, 0, stream, pp);
     note_launch();
     return e;
 }
