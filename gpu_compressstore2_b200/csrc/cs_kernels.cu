@@ -446,11 +446,11 @@ __device__ __forceinline__ void popc_block_finish(const BlockScanParams& p, cons
 constexpr uint64_t SPARSE_GROUPS_MIN = 256;
 constexpr uint64_t LONG_BLOCKS = 256; // 2^26 elements
 
-// The end of both pass-1+2 kernels (all threads): the finishing ticket carries in its upper bits how many
-// of the 16 groups of the CTA's average block are sparse, so the last CTA learns their share from its own
-// atomic (no array to read). The last CTA scans the block sums and closes
-// the epoch; the call's scan is marked clean unless a CTA poisoned this epoch. sparse_seen: this warp's
-// sparse groups, of `blocks` blocks; s_warp: free.
+// The end of both pass-1+2 kernels (all threads): the finishing ticket carries in its upper 20 bits how many
+// of the 16 groups of the CTA's average block are sparse, in sixteenths (in whole groups an evenly spread share
+// loses up to half of itself), so the last CTA learns their share from its own atomic (no array to read).
+// The last CTA scans the block sums and closes the epoch; the call's scan is marked clean unless a CTA
+// poisoned this epoch. sparse_seen: this warp's sparse groups, of `blocks` blocks; s_warp: free.
 __device__ __forceinline__ void popc_blocks_finish_grid(const BlockScanParams& p, uint32_t sparse_seen, uint32_t blocks,
                                                         uint32_t* s_warp, const uint32_t* s_epoch, uint32_t* s_flag,
                                                         uint64_t* s_scan, uint64_t* s_prefix, uint64_t prefix_room)
@@ -462,14 +462,14 @@ __device__ __forceinline__ void popc_blocks_finish_grid(const BlockScanParams& p
     if (tid == 0) {
         uint32_t groups = 0;
         for (uint32_t w = 0; w < 8; ++w) groups += s_warp[w];
-        // at most 16, of 2048 CTAs
-        const uint32_t mean = static_cast<uint32_t>(__fdividef(static_cast<float>(groups), static_cast<float>(blocks)) + 0.01f);
+        // at most 256, of at most 2048 CTAs, which 12 bits count
+        const uint32_t mean = static_cast<uint32_t>(__fdividef(static_cast<float>(groups) * 16.0f, static_cast<float>(blocks)) + 0.01f);
         __threadfence(); // this CTA's offsets and block sums before its ticket
-        const uint32_t prev = atomicAdd(&p.hdr->scan_done_counter, 1u + (mean << 16));
-        const bool last = (prev & 0xffffu) == gridDim.x - 1;
-        const uint32_t sum = (prev >> 16) + mean;
+        const uint32_t prev = atomicAdd(&p.hdr->scan_done_counter, 1u + (mean << 12));
+        const bool last = (prev & 0xfffu) == gridDim.x - 1;
+        const uint64_t sum = (prev >> 12) + mean;
         const uint32_t share = p.num_blocks > LONG_BLOCKS && (p.cols || p.col0.elem_bytes >= 4) ? 12u : 2u;
-        const bool sparse = sum * share >= 16u * gridDim.x && sum * p.num_blocks >= SPARSE_GROUPS_MIN * gridDim.x;
+        const bool sparse = sum * share >= 256u * gridDim.x && sum * p.num_blocks >= 16u * SPARSE_GROUPS_MIN * gridDim.x;
         *s_flag = last ? (1u | (sparse ? 2u : 0u)) : 0u;
     }
     __syncthreads();
