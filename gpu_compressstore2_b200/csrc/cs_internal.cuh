@@ -740,10 +740,11 @@ __device__ __forceinline__ void blocks_last_cta(const BlockScanParams& p, uint64
 struct WriteoutParams {
     ColumnDesc col0;          // the column (cols null); unit_base and item_base 0
     const ColumnDesc* cols;   // batch: unit u belongs to cols[unit_col[u]], sparse item t to
-    const uint32_t* unit_col; // cols[item_col[t]]; items of other widths are another launch's
+    const uint32_t* unit_col; // cols[item_col[t]], where it is item t + first_item of the plan
     const uint32_t* item_col;
     uint64_t num_units;       // 128 KB units of this launch's width over all columns
-    uint64_t num_sparse_items; // 16K-element items over all columns
+    uint64_t first_item;      // batch: the first sparse item of this launch's width
+    uint64_t num_sparse_items; // 16K-element items over all columns of this launch
     uint64_t sparse_max;      // hybrid: units with at most this many selected are gathered (0: none)
     const uint32_t* item_flags; // items pass 1 marked with its epoch (the sparse ones); null: test every item
     ws_header* hdr;

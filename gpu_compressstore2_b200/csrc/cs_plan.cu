@@ -181,14 +181,22 @@ int plan_columns(const cs_column* cols, uint32_t ncols, std::vector<ColumnDesc>&
             continue;
         }
         d.tile_base = tot.tiles;
-        d.item_base = tot.items;
+        d.item_base = tot.width_items[wi]; // within its width, for now
         d.unit_base = tot.units[wi];
         chunk_base[c] = tot.chunks;
         tot.tiles += tiles;
         tot.items += items;
+        tot.width_items[wi] += items;
         tot.units[wi] += units;
         tot.chunks += chunks;
     }
+    // A width's items lie together, so that its writeout meets no others: a few columns of another width take
+    // few warps, and each of those stepped over its share of a long sparse column's items (2^28 u8, 1 in 100
+    // selected, beside seven short columns of all widths: 355 us, now 85).
+    uint64_t first[4] = {0, 0, 0, 0};
+    for (int wi = 1; wi < 4; ++wi) first[wi] = first[wi - 1] + tot.width_items[wi - 1];
+    for (ColumnDesc& d : desc)
+        if (d.n && !d.one_pass) d.item_base += first[plan_width_index(d.elem_bytes)];
     if (tot.tiles > 0xffffffffull || tot.items > 0xffffffffull) return CS_ERR_NOT_SUPPORTED;
     return CS_SUCCESS;
 }
@@ -258,17 +266,20 @@ int plan_launch(const PlanDevice& d, const PlanCounts& c, int sms, uint64_t time
         cudaError_t e = launch_popc_blocks(bp, sms, s);
         if (e != cudaSuccess) return to_status(e);
     }
+    uint64_t first_item = 0;
     for (int wi = 0; wi < 4; ++wi) {
         if (!c.units[wi]) continue;
         const uint32_t w = 1u << wi;
         WriteoutParams p{};
         p.cols = d.cols;
         p.unit_col = d.unit_col[wi];
-        p.item_col = d.item_col;
+        p.item_col = d.item_col + first_item;
+        p.first_item = first_item;
         p.num_units = c.units[wi];
-        p.num_sparse_items = c.items;
+        p.num_sparse_items = c.width_items[wi];
         p.sparse_max = unit_elems_for(w) / 32;
-        p.item_flags = d.item_flags;
+        p.item_flags = d.item_flags + first_item;
+        first_item += c.width_items[wi];
         p.hdr = d.hdr;
         p.chunk_log2 = PLAN_CHUNK_LOG2;
         cudaError_t e = launch_writeout_warp(p, w, writeout_ctas, sms, s);

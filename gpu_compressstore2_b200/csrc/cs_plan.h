@@ -33,6 +33,7 @@ constexpr uint32_t PLAN_CHUNK_LOG2 = 9;
 struct PlanCounts {
     uint64_t tiles = 0;               // 2^18-element blocks over the 3-pass columns
     uint64_t items = 0;               // sparse items (16K elements) over the 3-pass columns
+    uint64_t width_items[4] = {0, 0, 0, 0}; // of each width, in this order one after the other
     uint64_t units[4] = {0, 0, 0, 0}; // 128 KB units of the 3-pass columns per width index (1, 2, 4, 8 bytes)
     uint64_t units1[4] = {0, 0, 0, 0}; // TMA units of the 1-pass columns per width index
     uint64_t chunks = 0;              // PLAN_CHUNK-element chunks over the 3-pass columns (offsets array)

@@ -375,8 +375,7 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS<SHIFT>) k_writeout_warp(const
             todo &= todo - 1;
             const uint64_t item = work / split;
             const ColumnDesc& c = MULTI ? p.cols[__ldg(p.item_col + item)] : p.col0;
-            if (MULTI && c.elem_bytes != sizeof(T)) continue; // another width's launch gathers it
-            const uint64_t e0 = (item - c.item_base) * 16384ull;
+            const uint64_t e0 = (MULTI ? item + p.first_item - c.item_base : item) * 16384ull;
             if (split == 1u) sparse_groups<T, 4>(c, e0, p.chunk_log2, lane, list);
             else sparse_groups<T, 1>(c, e0 + (work & 3u) * 4096ull, p.chunk_log2, lane, list);
         }
