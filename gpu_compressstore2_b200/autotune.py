@@ -209,11 +209,27 @@ def install_batch(results) -> None:
         _lib.check(L.cs_tune_batch_set(w, b, sb, algo), "cs_tune_batch_set")
 
 
+def default_turns(w: int, b: int) -> bool:
+    """Whether the library's own choice for an unset (width, size) entry changes inside the bucket
+    (clears the entry). A bucket spans a factor of four in length; where the forms change places
+    inside it, one entry would be the wrong one on one side."""
+    L = _lib.lib()
+    _lib.check(L.cs_tune_set(w, b, _lib.ALGO_AUTO, 0), "cs_tune_set")
+    seen = set()
+    for n in (1 << 2 * b, (1 << 2 * b + 2) - 1):
+        algo, chunk = ctypes.c_int32(), ctypes.c_uint32()
+        _lib.check(L.cs_tune_get(w, n, ctypes.byref(algo), ctypes.byref(chunk)), "cs_tune_get")
+        seen.add(algo.value)
+    return len(seen) > 1
+
+
 def install(results) -> None:
-    """Put measured choices in the library's table (every untuned bucket keeps the default)."""
+    """Put measured choices in the library's table (every untuned bucket keeps the default, and so do
+    those inside which the default itself changes form)."""
     L = _lib.lib()
     for (w, b), (algo, chunk, _, sel_best) in results.items():
-        _lib.check(L.cs_tune_set(w, b, algo, chunk), "cs_tune_set")
+        if not default_turns(w, b):
+            _lib.check(L.cs_tune_set(w, b, algo, chunk), "cs_tune_set")
         for sb, (a, c) in sel_best.items():
             _lib.check(L.cs_tune_sel_set(w, b, sb, a, c), "cs_tune_sel_set")
 
