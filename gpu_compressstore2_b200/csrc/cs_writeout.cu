@@ -66,19 +66,23 @@ constexpr uint32_t WARPS = 8;
 template <bool SHIFT>
 constexpr uint32_t CTAS = SHIFT ? 2 : 3;
 
+// Warps of a CTA that stay idle for a long column of which most is selected (by thousandths): there the
+// loads in flight of 24 warps per SM hold up the writes. 3-pass call on B200, us, 24 / 21 / 18 warps: 2^27 u64
+// p = 0.7 298 / 295 / 309, 0.8 348 / 333 / 314, 0.9 360 / 345 / 335, 0.99 377 / - / 347, all 371 / - / 345; 2^28 u32
+// p = 0.7 303 / 310 / 331, 0.8 339 / 326 / 334, 0.9 357 / 340 / 355, 2^27 0.996 189 / 193 / 198, 0.9995 190 / 195 /
+// 201, all 204 / 198 / 184, 2^26 all 106 / 104 / 97, 2^28 all 370 / 360 / 368, 2^26 u32 p = 0.9 102 / 94 / 94, but
+// 2^24 29.6 / 30.6 / 31.7 (few items per warp). Narrower elements are held back by their instructions: 2^28 u16
+// p = 0.9 185 / 198 / 200.
+template <typename T>
+__device__ __forceinline__ uint32_t idle_warps(uint64_t thousandths)
+{
+    if constexpr (sizeof(T) == 8) return thousandths >= 750u ? 2u : 0u;
+    if constexpr (sizeof(T) == 4) return thousandths >= 1000u ? 2u : thousandths >= 850u && thousandths < 970u ? 1u : 0u;
+    return 0u;
+}
+
 // 32 bytes from an address `d` bytes (1 .. 15, the same for the whole column) past a 16-byte
 // boundary, out of the three 16-byte vectors that hold them.
-// Warps of a CTA that stay idle for a long column of which most, but not nearly all, is selected:
-// there the loads in flight of 24 warps per SM hold up the writes. 3-pass call on B200, us, 24 / 21 /
-// 18 warps: 2^27 u64 p = 0.7 298 / 295 / 309, 0.8 348 / 333 / 314, 0.9 360 / 345 / 335, 0.99 354 / 351 /
-// 354; 2^28 u32 p = 0.7 303 / 310 / 331, 0.8 339 / 326 / 334, 0.9 357 / 340 / 355, 0.99 374 / 373 / 381;
-// 2^26 u32 p = 0.9 102 / 94 / 94, but 2^24 29.6 / 30.6 / 31.7 (few items per warp). Narrower elements
-// are held back by their instructions: 2^28 u16 p = 0.9 185 / 198 / 200.
-template <typename T>
-constexpr uint32_t throttle_warps = sizeof(T) == 8 ? 2 : sizeof(T) == 4 ? 1 : 0;
-template <typename T>
-constexpr uint32_t throttle_percent = sizeof(T) == 8 ? 75 : 85; // from this share selected on, up to 97%
-
 __device__ __forceinline__ void ldg_shifted(const uint8_t* p, uint32_t d, uint32_t (&x)[8])
 {
     const uint4* q = reinterpret_cast<const uint4*>(p - d);
@@ -212,12 +216,14 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS<SHIFT>) k_writeout_warp(const
     const uint32_t stage_a = smem_u32(stage);
     const uint32_t lut = sizeof(T) == 1 ? smem_u32(s_lut) + lane * 4 : 0u;
     const uint32_t num_items = static_cast<uint32_t>(p.num_units) * IPU; // below 2^32 for every column the library takes
-    // a long column of mostly selected elements runs better with fewer warps (throttle_warps)
-    uint32_t active = WARPS;
-    const uint64_t percent = p.throttle != 0u ? *p.col0.d_count * 100 / p.col0.n : 0u;
-    if (percent >= throttle_percent<T> && percent < 97u) {
-        active = WARPS - p.throttle;
-        if (warp >= active) return;
+    // a long column of mostly selected elements runs better with fewer warps (plans: throttle is 0, but as a
+    // constant the number costs their 8-byte form 32 bytes of spills)
+    uint32_t active = MULTI ? WARPS - p.throttle : WARPS;
+    if constexpr (!MULTI && sizeof(T) >= 4) {
+        if (p.throttle != 0u) {
+            active -= idle_warps<T>(*p.col0.d_count * 1000 / p.col0.n);
+            if (warp >= active) return;
+        }
     }
     const uint32_t warp_global = blockIdx.x * active + warp;
     const uint32_t total_warps = gridDim.x * active;
@@ -391,7 +397,7 @@ cudaError_t launch_t(const WriteoutParams& p, uint32_t requested, int num_sms, c
     if (blocks > cap) blocks = cap;
     if (blocks == 0) blocks = 1;
     WriteoutParams pp = p;
-    pp.throttle = !p.cols && p.col0.d_count && items >= 8 * blocks * WARPS ? throttle_warps<T> : 0u;
+    pp.throttle = sizeof(T) >= 4 && !p.cols && p.col0.d_count && items >= 8 * blocks * WARPS ? 1u : 0u;
     const dim3 g(static_cast<unsigned>(blocks)), b(WARPS * 32);
     cudaError_t e;
     const bool inside = (1u << p.chunk_log2) > ITEM_BYTES / sizeof(T); // items that start inside a chunk
