@@ -618,10 +618,10 @@ __global__ void __launch_bounds__(Roles<MODE>::NTHREADS, 1) k_compact_tma(const 
     }
 
     if (MODE == 0 && epilogue_ticket(&p.hdr->done_counter, &s_flag)) {
+        const bool lost = epilogue_last(p.hdr, &p.hdr->tile_counter, &p.hdr->done_counter, false, p.keep_begin, p.keep_end, nullptr);
         // units left unfinished: a column's count comes from its last unit, which may be one of them
-        if (reinterpret_cast<volatile ws_header*>(p.hdr)->lost_epoch == epoch)
+        if (lost)
             for (uint64_t u = threadIdx.x; u < p.num_tiles; u += blockDim.x) *col_of_unit(u).d_count = COUNT_ERROR;
-        epilogue_last(p.hdr, &p.hdr->tile_counter, &p.hdr->done_counter, false, p.keep_begin, p.keep_end, nullptr);
     }
 }
 

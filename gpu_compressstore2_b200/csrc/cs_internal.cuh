@@ -417,12 +417,14 @@ __device__ __forceinline__ bool epilogue_ticket(uint32_t* done_counter, uint32_t
     return last;
 }
 
-__device__ __forceinline__ void epilogue_last(ws_header* hdr, uint32_t* tile_counter, uint32_t* done_counter,
+// Returns, in every thread, whether a CTA of this launch left units unfinished (lost_epoch).
+__device__ __forceinline__ bool epilogue_last(ws_header* hdr, uint32_t* tile_counter, uint32_t* done_counter,
                                               bool is_scan, uint64_t keep_begin, uint64_t keep_end,
                                               const uint32_t* popc_flags)
 {
     volatile ws_header* vh = hdr;
     const uint32_t cur = vh->epoch;
+    const bool lost = vh->lost_epoch == cur;
     uint32_t next = cur + 1u;
     if (next > EPOCH_MAX) {
         wrap_clear(hdr, keep_begin, keep_end, is_scan);
@@ -446,6 +448,7 @@ __device__ __forceinline__ void epilogue_last(ws_header* hdr, uint32_t* tile_cou
         vh->epoch = next;
         __threadfence();
     }
+    return lost;
 }
 
 // epilogue_last for the reduce-then-scan pass (the last CTA, all its threads): `cur` is the
