@@ -60,11 +60,11 @@ static_assert(SPARSE_LIST * 2 <= STAGE_BYTES, "the list lies in the stage");
 // 8 warps per CTA and 3 CTAs per SM: 80 registers hold an item's 4 loads per lane without spills.
 // More resident warps with fewer registers were slower (64 registers x 4 CTAs spill; 2 rows per
 // item x 5 CTAs: 2^28 f32 p = 0.5 291 against 281 us, 2^29 u8 210 against 194), and so were fewer
-// (2 CTAs: 300 and 209) and items of 8 rows (2 x 8 KB per SM-warp: 269, 194). Shifted loads hold
-// three vectors per row.
+// (2 CTAs: 300 and 209) and items of 8 rows (2 x 8 KB per SM-warp: 269, 194). Shifted loads of narrower
+// elements than 8 bytes hold three vectors per row.
 constexpr uint32_t WARPS = 8;
-template <bool SHIFT>
-constexpr uint32_t CTAS = SHIFT ? 2 : 3;
+template <typename T, bool SHIFT>
+constexpr uint32_t CTAS = SHIFT && sizeof(T) < 8 ? 2 : 3;
 
 // Warps of a CTA that stay idle for a long column of which most is selected (by thousandths): there the
 // loads in flight of 24 warps per SM hold up the writes. 3-pass call on B200, us, 24 / 21 / 18 warps: 2^27 u64
@@ -81,21 +81,30 @@ __device__ __forceinline__ uint32_t idle_warps(uint64_t thousandths)
     return 0u;
 }
 
-// 32 bytes from an address `d` bytes (1 .. 15, the same for the whole column) past a 16-byte
-// boundary, out of the three 16-byte vectors that hold them.
+// 32 bytes from an address `d` bytes (1 .. 15, the same for the whole column) past a 16-byte boundary: out of
+// the three 16-byte vectors that hold them, or, for 8-byte elements (d = 8), as the halves of two and the one
+// between them, which need no selection (2^26 u64 p = 0.1 225 -> 97 us, 0.5 251 -> 133, 0.9 338 -> 170; and 80 registers, three CTAs per SM).
+template <typename T>
 __device__ __forceinline__ void ldg_shifted(const uint8_t* p, uint32_t d, uint32_t (&x)[8])
 {
-    const uint4* q = reinterpret_cast<const uint4*>(p - d);
-    const uint4 a = __ldg(q), b = __ldg(q + 1), c = __ldg(q + 2);
-    const uint32_t w[12] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c.x, c.y, c.z, c.w};
-    const uint32_t s = (d & 3u) * 8u;
+    if constexpr (sizeof(T) == 8) {
+        const uint2 a = __ldg(reinterpret_cast<const uint2*>(p));
+        const uint4 b = __ldg(reinterpret_cast<const uint4*>(p + 8));
+        const uint2 c = __ldg(reinterpret_cast<const uint2*>(p + 24));
+        x[0] = a.x, x[1] = a.y, x[2] = b.x, x[3] = b.y, x[4] = b.z, x[5] = b.w, x[6] = c.x, x[7] = c.y;
+    } else {
+        const uint4* q = reinterpret_cast<const uint4*>(p - d);
+        const uint4 a = __ldg(q), b = __ldg(q + 1), c = __ldg(q + 2);
+        const uint32_t w[12] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c.x, c.y, c.z, c.w};
+        const uint32_t s = (d & 3u) * 8u;
 #pragma unroll
-    for (uint32_t i = 0; i < 8; ++i) {
-        uint32_t lo = w[i], hi = w[i + 1];
-        if (d >= 12u) lo = w[i + 3], hi = w[i + 4 < 12 ? i + 4 : 11];
-        else if (d >= 8u) lo = w[i + 2], hi = w[i + 3];
-        else if (d >= 4u) lo = w[i + 1], hi = w[i + 2];
-        x[i] = __funnelshift_r(lo, hi, s);
+        for (uint32_t i = 0; i < 8; ++i) {
+            uint32_t lo = w[i], hi = w[i + 1];
+            if (d >= 12u) lo = w[i + 3], hi = w[i + 4 < 12 ? i + 4 : 11];
+            else if (d >= 8u) lo = w[i + 2], hi = w[i + 3];
+            else if (d >= 4u) lo = w[i + 1], hi = w[i + 2];
+            x[i] = sizeof(T) == 4 ? lo : __funnelshift_r(lo, hi, s); // (whole words: s = 0)
+        }
     }
 }
 
@@ -191,7 +200,7 @@ __device__ __forceinline__ void sparse_groups(const ColumnDesc& c, uint64_t e0, 
 // -> 267, 0.9 396 -> 343, 2^28 u16 0.5 168 -> 155; 2^22 u64 17.6 -> 18.2.) A kernel of its own: in the other one
 // its registers cost 2^28 u32 at chunk 1024 265 -> 296.
 template <typename T, bool MULTI, bool SHIFT, bool LONG>
-__global__ void __launch_bounds__(WARPS * 32, CTAS<SHIFT>) k_writeout_warp(const WriteoutParams p)
+__global__ void __launch_bounds__(WARPS * 32, CTAS<T, SHIFT>) k_writeout_warp(const WriteoutParams p)
 {
     constexpr uint32_t EPL = LANE_BYTES / sizeof(T); // elements per lane and row
     constexpr uint32_t ROW = 32 * EPL;
@@ -325,10 +334,10 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS<SHIFT>) k_writeout_warp(const
             if (!whole && e + EPL > n) b &= e < n ? (1u << (n - e)) - 1u : 0u; // n - e < EPL <= 32
             bits[r] = b;
             if (b) {
-                // a shifted load takes whole 16-byte vectors, which must lie inside the column
-                const bool inside = SHIFT ? e > 0 && e * sizeof(T) + 48 - phase <= n * sizeof(T) : whole || e + EPL <= n;
+                // a shifted load of narrower elements takes whole 16-byte vectors, which must lie inside the column
+                const bool inside = SHIFT && sizeof(T) < 8 ? e > 0 && e * sizeof(T) + 48 - phase <= n * sizeof(T) : whole || e + EPL <= n;
                 if (inside) {
-                    if constexpr (SHIFT) ldg_shifted(src + r * ROW_BYTES, phase, x[r]);
+                    if constexpr (SHIFT) ldg_shifted<T>(src + r * ROW_BYTES, phase, x[r]);
                     else if (in32) ldg256(src + r * ROW_BYTES, x[r]);
                     else ldg128x2(src + r * ROW_BYTES, x[r]);
                 } else {
@@ -393,7 +402,7 @@ cudaError_t launch_t(const WriteoutParams& p, uint32_t requested, int num_sms, c
 {
     const uint64_t items = p.num_units * (UNIT_TILES * TILE_BYTES / ITEM_BYTES);
     uint64_t blocks = (items + WARPS - 1) / WARPS;
-    const uint64_t cap = requested ? requested : static_cast<uint64_t>(num_sms) * CTAS<SHIFT>; // one resident wave
+    const uint64_t cap = requested ? requested : static_cast<uint64_t>(num_sms) * CTAS<T, SHIFT>; // one resident wave
     if (blocks > cap) blocks = cap;
     if (blocks == 0) blocks = 1;
     WriteoutParams pp = p;
