@@ -3,19 +3,21 @@
 // Element i is selected when bit (i % L) of `pattern` is set (LSB-first, 1 <= L <= 32). With
 // P = popcount of the pattern's L bits, output j is input (j / P) * L + pos[j % P], pos[r]
 // being the r-th set bit: every output has a closed-form source, so there is no popcount
-// pass, no scan and no mask read. Two kernels:
+// pass, no scan and no mask read. Three kernels:
 //
 // k_pattern gathers. A warp produces runs of 128 output bytes (256 for 8-byte elements): each
 // lane 4 consecutive bytes of them (1, 2 or 4 elements) or one 8-byte element, so that one load
 // instruction of the warp falls on the few lines that its outputs come from and one store
 // instruction writes whole lines. The offsets of a lane's sources repeat every P such runs: they
-// come from a table in shared memory, and a thread divides once. A thread keeps the loads of
+// come from a table in shared memory, and a thread divides twice. A thread keeps the loads of
 // PATTERN_RUNS runs in flight before it stores. Where the selected elements lie 64 bytes and more
 // apart a load fetches 64 bytes instead of a line (2^28 u32, 1 of 32: 163 -> 91 us).
 //
 // k_pattern_dense streams the input through registers and a stage per warp as the 3-pass
 // writeout does (cs_writeout.cu), with mask bits and positions from the pattern; it runs at the HBM
 // rate from about a third selected on (2^28 u32, 31 of 32: 2.11 GB in 322 us).
+//
+// k_pattern_all copies where everything is selected.
 // Reference: bench9_pattern (src/benchmarks.cuh:397-416) over launch_pattern_proc /
 // kernel_pattern_proc (src/kernels/kernel_pattern.cuh:13-131), whose pattern is read from
 // the most significant bit (element i <-> bit 31 - i % L); pass __brev of such a pattern.
@@ -52,18 +54,29 @@ __global__ void __launch_bounds__(256) k_pattern(const T* __restrict__ in, T* __
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) *d_count = count;
     __syncthreads();
-    for (uint32_t i = threadIdx.x; i < RUN * P; i += 256) s_off[i] = static_cast<uint16_t>(i / P * L + s_pos[i % P]);
+    // (one division; the table of a dense pattern is long, and a short column has time for little else)
+    uint32_t tq = threadIdx.x / P, tr = threadIdx.x % P;
+    const uint32_t tdq = 256 / P, tdr = 256 % P;
+    for (uint32_t i = threadIdx.x; i < RUN * P; i += 256) {
+        s_off[i] = static_cast<uint16_t>(tq * L + s_pos[tr]);
+        tq += tdq;
+        tr += tdr;
+        if (tr >= P) {
+            tr -= P;
+            ++tq;
+        }
+    }
     __syncthreads();
     const uint32_t lane = threadIdx.x & 31u;
-    const uint64_t warp_global = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    const uint64_t step = ((static_cast<uint64_t>(gridDim.x) * blockDim.x) >> 5) * U; // runs between a warp's groups
+    // (numbers of warps of a resident grid: divided in 32 bits)
+    const uint32_t s_first = ((blockIdx.x * 256u + threadIdx.x) >> 5) * U;
+    const uint32_t step = gridDim.x * 8u * U; // runs between a warp's groups
     const uint64_t runs = (count + RUN - 1) / RUN;
-    const uint64_t dq = step / P;
-    const uint32_t dr = static_cast<uint32_t>(step % P);
+    const uint32_t dq = step / P, dr = step % P;
     const uint32_t period = RUN * L; // inputs of P runs
-    uint64_t q = warp_global * U / P;
-    uint32_t r = static_cast<uint32_t>(warp_global * U % P);
-    for (uint64_t s0 = warp_global * U; s0 < runs; s0 += step) {
+    uint64_t q = s_first / P;
+    uint32_t r = s_first % P;
+    for (uint64_t s0 = s_first; s0 < runs; s0 += step) {
         T x[U][G];
         const T* src = in + q * period;
         uint32_t rk = r;
@@ -106,6 +119,31 @@ __global__ void __launch_bounds__(256) k_pattern(const T* __restrict__ in, T* __
     }
 }
 
+// A pattern that selects everything: the column, 16 bytes at a time where it lies so (all pointers 16-byte
+// aligned), and what is left of it byte by byte. 2^28 u16 171 us, 1 byte 88 (the dense kernel 312 and 109).
+constexpr uint32_t COPY_CTAS = 2; // per SM (1 GB of 8-byte elements: 2 172 us, 3 180, 4 180, 8 177)
+__global__ void __launch_bounds__(256) k_pattern_all(const uint8_t* __restrict__ in, uint8_t* __restrict__ out, uint64_t bytes,
+                                                     uint64_t count, uint64_t* d_count)
+{
+    constexpr uint32_t U = 4;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *d_count = count;
+    const uint64_t vectors = bytes / 16;
+    const uint64_t step = static_cast<uint64_t>(gridDim.x) * 256 * U;
+    const uint4* __restrict__ src = reinterpret_cast<const uint4*>(in);
+    uint4* __restrict__ dst = reinterpret_cast<uint4*>(out);
+    for (uint64_t v0 = static_cast<uint64_t>(blockIdx.x) * 256 * U + threadIdx.x; v0 < vectors; v0 += step) {
+        uint4 x[U];
+#pragma unroll
+        for (uint32_t u = 0; u < U; ++u)
+            if (v0 + u * 256 < vectors) x[u] = __ldg(src + v0 + u * 256);
+#pragma unroll
+        for (uint32_t u = 0; u < U; ++u)
+            if (v0 + u * 256 < vectors) __stcs(dst + v0 + u * 256, x[u]);
+    }
+    const uint32_t rest = static_cast<uint32_t>(bytes % 16);
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x < rest) out[vectors * 16 + threadIdx.x] = in[vectors * 16 + threadIdx.x];
+}
+
 // Dense patterns: items of 4 KB of payload per warp as in the 3-pass writeout (cs_writeout.cu),
 // with the mask bits and the positions from the pattern instead of a mask and a scan: element e
 // has rank (e / L) * P + the pattern's set bits below e % L. `rep`: the pattern repeated over 64
@@ -136,15 +174,14 @@ __global__ void __launch_bounds__(DENSE_WARPS * 32, DENSE_CTAS)
     const uint32_t stage_a = smem_u32(stage);
     const uint32_t lut = sizeof(T) == 1 ? smem_u32(s_lut) + lane * 4 : 0u;
     const bool in32 = (reinterpret_cast<uintptr_t>(in) & 31u) == 0;
-    const uint64_t total_warps = static_cast<uint64_t>(gridDim.x) * DENSE_WARPS;
-    const uint64_t step = total_warps * ITEM;
-    uint64_t e0 = (static_cast<uint64_t>(blockIdx.x) * DENSE_WARPS + warp) * ITEM;
+    const uint32_t step = gridDim.x * DENSE_WARPS * ITEM; // of a resident grid: both in 32 bits
+    const uint32_t first = (blockIdx.x * DENSE_WARPS + warp) * ITEM;
+    uint64_t e0 = first;
     // the period and the place within it of this lane's first element; both advance without
     // further divisions
-    const uint64_t dq = step / L;
-    const uint32_t dr = static_cast<uint32_t>(step % L);
-    uint64_t q = (e0 + lane * EPL) / L;
-    uint32_t r = static_cast<uint32_t>((e0 + lane * EPL) % L);
+    const uint32_t dq = step / L, dr = step % L;
+    uint64_t q = (first + lane * EPL) / L;
+    uint32_t r = (first + lane * EPL) % L;
     const uint32_t row_q = ROW / L, row_r = ROW % L;
     for (; e0 < n; e0 += step) {
         const bool whole = e0 + ITEM <= n;
@@ -213,9 +250,22 @@ __global__ void __launch_bounds__(DENSE_WARPS * 32, DENSE_CTAS)
 //   8       196 / 196  209 / 214  230 / 215  241 / 230  252 / 242  306 / 282  349 / 325
 // (dense at the better of 2 and 3 CTAs per SM; one thread per 16 output bytes, which both replace:
 // 1 byte 131 .. 156 .. 297, 2 bytes 158 .. 164 .. 318, 4 bytes 213 .. 256 .. 438).
-bool dense_pattern(uint32_t w, uint32_t L, uint32_t P)
+//
+// Short columns are gathered whatever the share: the dense kernel starts more slowly. Gather / dense, us, by
+// bytes of payload (4.1 is what the launches themselves take): 1 byte, 4 of 8, 1 MB 4.1 / 6.1, 2 MB 4.4 / 6.2, 4 MB
+// 6.2 / 6.2; 2 bytes, 6 of 7, 1 MB 4.1 / 6.2, 2 MB 5.2 / 6.2, 2 of 3, 2 MB 4.2 / 4.2; 4 bytes 2 MB 4.0 / 4.2. 8 bytes stay
+// with it longer: 4 of 8, 32 MB 14.2 / 14.2, 64 MB 19.1 / 20.4, but 6 of 7, 64 MB 24.6 / 23.5, 512 MB 167 / 166.
+// And so are halves in runs of 32 bytes and more, of which the gather reads whole sectors and has nothing to
+// pack: 8 bytes, 16 of 32 in one run, 2^26 94 / 111, 2^24 27 / 32; 4 bytes 65.7 / 72 at 2^26, 262 / 264 at 2^28.
+bool dense_pattern(uint32_t w, uint32_t L, uint32_t P, uint32_t pattern, uint64_t n)
 {
-    return P * 100 >= L * (w == 1 || w == 8 ? 30u : 36u);
+    const uint64_t bytes = n * w;
+    if (bytes <= (w == 8 ? 40ull << 20 : w == 2 ? 3ull << 19 : 3ull << 20)) return false;
+    const bool late = w == 8 && bytes <= 96ull << 20;
+    if (P * 100 < L * (late ? 70u : w == 1 || w == 8 ? 30u : 36u)) return false;
+    uint32_t runs = 0; // of selected elements in a period
+    for (uint32_t i = 0; i < L; ++i) runs += (pattern >> i & 1u) && !(pattern >> (i ? i - 1 : L - 1) & 1u);
+    return !(w > 1 && P * w >= 32 * runs && P * 100 <= L * 55u);
 }
 
 // CTAs of the dense kernel per SM. 3 keep enough loads in flight for what is mostly read; where as
@@ -239,7 +289,16 @@ cudaError_t launch_t(const void* in, void* out, uint64_t n, uint32_t pattern, ui
     if (blocks == 0) blocks = 1;
     const bool vec = (reinterpret_cast<uintptr_t>(out) & 3u) == 0;
     const bool apart = sizeof(T) * L >= 64 * P;
-    if (dense_pattern(sizeof(T), L, P) && (reinterpret_cast<uintptr_t>(in) & 15u) == 0) {
+    if (P == L && ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0) {
+        uint64_t ctas = (n * sizeof(T) + 256 * 4 * 16 - 1) / (256 * 4 * 16);
+        const uint64_t most = static_cast<uint64_t>(sms) * COPY_CTAS;
+        if (ctas > most) ctas = most;
+        k_pattern_all<<<static_cast<unsigned>(ctas), 256, 0, s>>>(static_cast<const uint8_t*>(in), static_cast<uint8_t*>(out),
+                                                                 n * sizeof(T), count, d_count);
+        note_launch();
+        return cudaGetLastError();
+    }
+    if (dense_pattern(sizeof(T), L, P, pattern, n) && (reinterpret_cast<uintptr_t>(in) & 15u) == 0) {
         uint64_t rep = 0;
         for (uint32_t i = 0; i < 64; ++i) rep |= static_cast<uint64_t>((pattern >> (i % L)) & 1u) << i;
         const uint64_t items = (n * sizeof(T) + ITEM_BYTES - 1) / ITEM_BYTES;
