@@ -34,6 +34,7 @@ struct cs_batch {
     PlanDevice dev;
     PlanCounts counts;
     uint32_t grid1[4] = {0, 0, 0, 0};
+    uint32_t idle[4] = {0, 0, 0, 0}; // warps per CTA of each width's writeout
     uint32_t one_pass_cols = 0;
     std::vector<cs_column> cols; // for the per-call loop
     uint64_t timeout_ns = 2000000000ull;
@@ -50,6 +51,37 @@ constexpr uint64_t PLAN_3PASS_MIN_BYTES = 256ull << 20;
 // ... and the payload from which on a plan takes one form (103 columns of 303 MB, both / 3-pass: 110 / 97 us).
 constexpr uint64_t PLAN_LARGE_BYTES = 272ull << 20;
 
+// Columns of one width are one launch in the 1-pass form and two in the 3-pass form, which shows where there is
+// little to do, and in the middle, where the second launch waits for the first's tail. 1-pass / 3-pass, us, by
+// plan: columns up to 2^14 elements, 4 bytes 1 column 10.3 / 11.6, 32 10.3 / 12.3, 256 15.2 / 17.5, 8 bytes 8.9 / 11.3,
+// 10.3 / 12.3, 14.2 / 16.4, 2 bytes 1 10.9 / 12.3, 64 13.0 / 12.3, 256 16.4 / 18.4; 30 to 80 MB with 0.5 selected, 4 bytes
+// 4 columns 20.6 / 22.6, 32 31.0 / 34.6, 256 24.9 / 26.5 (0.1: 18.7 / 19.9, 26.7 / 30.7, 22.7 / 24.4; 0.01: 18.5 / 14.3), 8 bytes 2
+// 19.7 / 22.6, 16 32.2 / 33.7, 17 MB 4 15.1 / 16.4 (0.1: 18.3 / 17.8, 25.3 / 28.5), 2 bytes 32 24.7 / 26.6 (0.1: 22.7 / 22.6). 17 MB, 4 bytes
+// 15.9 / 15.9 and 17.9 / 16.4, 100 MB 8 bytes 39.0 / 37.3; several widths: 4 and 8 bytes 34 MB 30.5 / 26.6. 1-byte
+// columns are placed faster by the 3-pass form's warps at every size (14.3 / 12.3).
+bool plan_one_launch(uint32_t widths, uint32_t columns, uint64_t longest, uint64_t bytes, double selected)
+{
+    if (widths != 2 && widths != 4 && widths != 8) return false; // (a sum of several is none of them)
+    if (longest <= 1u << 14) return widths > 2 || columns <= 8 || columns > 128;
+    return bytes >= (widths == 8 ? 16u << 20 : 28u << 20) && bytes <= 80u << 20 && selected >= (widths == 4 ? 0.05 : 0.3);
+}
+
+// Idle warps of a writeout (idle_warps in cs_writeout.cu) for the plan's 3-pass columns of a width, by what is
+// selected of them when the plan is made.
+uint32_t idle_warps_of(const cs_column* cols, uint32_t ncols, const std::vector<uint8_t>& one_pass,
+                       const std::vector<double>& sel, uint32_t width)
+{
+    double elems = 0.0, selected = 0.0;
+    for (uint32_t i = 0; i < ncols; ++i) {
+        if (one_pass[i] || cols[i].elem_bytes != width) continue;
+        elems += static_cast<double>(cols[i].n);
+        selected += sel[i] * static_cast<double>(cols[i].n);
+    }
+    const double share = elems > 0.0 ? selected / elems : 0.0;
+    if (width == 8) return share >= 0.75 ? 2u : 0u;
+    return share >= 0.85 && share < 0.97 ? 1u : 0u;
+}
+
 inline int to_status(cudaError_t e)
 {
     if (e == cudaSuccess) return CS_SUCCESS;
@@ -63,7 +95,7 @@ int run_direct(cs_batch* b, cudaStream_t s)
         cudaError_t e = cudaMemsetAsync(c, 0, sizeof(uint64_t), s);
         if (e != cudaSuccess) return to_status(e);
     }
-    return plan_launch(b->dev, b->counts, b->sms, b->timeout_ns, s, b->grid1);
+    return plan_launch(b->dev, b->counts, b->sms, b->timeout_ns, s, b->grid1, 0, b->idle);
 }
 
 // Selected fraction of every column, from one reduce-then-scan popcount pass over the masks
@@ -163,19 +195,34 @@ int cs_batch_create(cs_batch** out, const cs_column* cols, uint32_t ncols, const
         }
         for (uint32_t i = 0; i < ncols; ++i)
             one_pass[i] = cols[i].n && tune_batch_lookup(cols[i].n, cols[i].elem_bytes, sel[i]) == CS_ALGO_1PASS;
-        // A plan of both forms runs both chains of launches, one after the other (about 30 us on B200). So
-        // small plans, by what the 3-pass columns hold, and large ones take one form: the 3-pass form unless
-        // the columns that the table names 1-pass hold a quarter of the payload (3-pass / 1-pass, us, any
-        // selectivity: 28 columns of 9 MB 16 / 26, 101 of 40 MB 28 / 33, 256 of 2.2 GB 577 / 615).
-        uint64_t bytes3 = 0, bytes1 = 0;
-        for (uint32_t i = 0; i < ncols; ++i)
-            (one_pass[i] ? bytes1 : bytes3) += cols[i].n * static_cast<uint64_t>(cols[i].elem_bytes);
+        // A plan of both forms runs both chains of launches, one after the other (about 30 us on B200), so it takes
+        // one form where it can: the 3-pass form if the columns that the table names 1-pass hold less than a
+        // quarter of the payload, otherwise the 1-pass form if the 3-pass columns hold less than
+        // PLAN_3PASS_MIN_BYTES (3-pass / 1-pass, us: 28 columns of 9 MB 16 / 26, 101 of 40 MB 28 / 33, 256 of 2.2 GB
+        // 577 / 615). Larger plans with a quarter or more named 1-pass keep both, as the table says (both /
+        // 3-pass, us: 40 columns of 369 MB 117 / 112, 128 of 940 MB 265 / 255), and so do those between the two
+        // lines (17 columns of 273 MB 90 / 82, 66 of 277 MB 115 / 101).
+        uint64_t bytes3 = 0, bytes1 = 0, longest = 0;
+        double selected = 0.0; // bytes
+        uint32_t widths = 0, filled = 0;
+        for (uint32_t i = 0; i < ncols; ++i) {
+            const uint64_t bytes = cols[i].n * static_cast<uint64_t>(cols[i].elem_bytes);
+            (one_pass[i] ? bytes1 : bytes3) += bytes;
+            selected += sel[i] * static_cast<double>(bytes);
+            if (!cols[i].n) continue;
+            longest = std::max(longest, cols[i].n);
+            widths |= cols[i].elem_bytes;
+            ++filled;
+        }
         const bool small = bytes3 < PLAN_3PASS_MIN_BYTES;
         if (bytes1 && (small || bytes1 + bytes3 >= PLAN_LARGE_BYTES)) {
             if (bytes1 < (bytes1 + bytes3) / 4) one_pass.assign(ncols, 0);
             else if (small)
                 for (uint32_t i = 0; i < ncols; ++i) one_pass[i] = cols[i].n ? 1 : 0;
         }
+        if (!bytes1 && plan_one_launch(widths, filled, longest, bytes3, bytes3 ? selected / static_cast<double>(bytes3) : 0.0))
+            for (uint32_t i = 0; i < ncols; ++i) one_pass[i] = cols[i].n ? 1 : 0;
+        for (int wi = 2; wi < 4; ++wi) b->idle[wi] = idle_warps_of(cols, ncols, one_pass, sel, 1u << wi);
     }
     for (uint32_t i = 0; i < ncols; ++i) b->one_pass_cols += one_pass[i] && cols[i].n ? 1u : 0u;
 

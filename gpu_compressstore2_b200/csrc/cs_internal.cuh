@@ -752,7 +752,7 @@ struct WriteoutParams {
     const uint32_t* item_flags; // items pass 1 marked with its epoch (the sparse ones); null: test every item
     ws_header* hdr;
     uint32_t chunk_log2;      // at most 12
-    uint32_t throttle;        // 1: a long column, some warps stay idle when most of it is selected (set at launch)
+    uint32_t throttle;        // long columns: warps per CTA that stay idle (batch), or 1: by the selected share
 };
 
 // ---------------------------------------------------------------------------------

@@ -225,15 +225,12 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS<T, SHIFT>) k_writeout_warp(co
     const uint32_t stage_a = smem_u32(stage);
     const uint32_t lut = sizeof(T) == 1 ? smem_u32(s_lut) + lane * 4 : 0u;
     const uint32_t num_items = static_cast<uint32_t>(p.num_units) * IPU; // below 2^32 for every column the library takes
-    // a long column of mostly selected elements runs better with fewer warps (plans: throttle is 0, but as a
-    // constant the number costs their 8-byte form 32 bytes of spills)
+    // a long column of mostly selected elements runs better with fewer warps
     uint32_t active = MULTI ? WARPS - p.throttle : WARPS;
     if constexpr (!MULTI && sizeof(T) >= 4) {
-        if (p.throttle != 0u) {
-            active -= idle_warps<T>(*p.col0.d_count * 1000 / p.col0.n);
-            if (warp >= active) return;
-        }
+        if (p.throttle != 0u) active -= idle_warps<T>(*p.col0.d_count * 1000 / p.col0.n);
     }
+    if (sizeof(T) >= 4 && warp >= active) return;
     const uint32_t warp_global = blockIdx.x * active + warp;
     const uint32_t total_warps = gridDim.x * active;
 
@@ -406,7 +403,8 @@ cudaError_t launch_t(const WriteoutParams& p, uint32_t requested, int num_sms, c
     if (blocks > cap) blocks = cap;
     if (blocks == 0) blocks = 1;
     WriteoutParams pp = p;
-    pp.throttle = sizeof(T) >= 4 && !p.cols && p.col0.d_count && items >= 8 * blocks * WARPS ? 1u : 0u;
+    const bool idle = sizeof(T) >= 4 && items >= 8 * blocks * WARPS;
+    pp.throttle = !idle ? 0u : p.cols ? p.throttle : p.col0.d_count ? 1u : 0u;
     const dim3 g(static_cast<unsigned>(blocks)), b(WARPS * 32);
     cudaError_t e;
     const bool inside = (1u << p.chunk_log2) > ITEM_BYTES / sizeof(T); // items that start inside a chunk
