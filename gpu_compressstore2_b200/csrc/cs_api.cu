@@ -28,19 +28,28 @@ void note_launch(uint64_t k)
 namespace {
 
 constexpr uint64_t MAX_N = (1ull << 40) - 1; // status words carry 40-bit offsets
-// The 1-pass kernel takes one-tile units for a column with fewer full units than SMs and at
-// most this many one-tile units (the workspace reserves statuses for that many).
+// The TMA 1-pass kernel takes one-tile units for a column with fewer full units than SMs and at most this many
+// one-tile units (the workspace reserves statuses for that many). Such columns run in slices unless skip = 2
+// asks for whole tiles.
 constexpr uint64_t SHORT_UNITS_MAX = 1024;
 // ... and the deeper payload ring (mode 2) for 4- and 8-byte columns of at least this many
 // full units per SM.
 constexpr uint64_t DEEP_UNITS_PER_SM = 16;
 // Most slices per SM for which a 1-pass call of 4- and 8-byte elements runs in slices (cs_slices.cu)
 // rather than through the TMA kernel; 1- and 2-byte columns of any length do. Per call on B200, inputs
-// from HBM, TMA / slices, us: u32 p = 0.5 2^20 8.5 / 5.4, 2^22 14.3 / 11.4, 2^23 (7 per SM) 20.1 / 15.8,
-// 1.5 x 2^23 (10) 22.9 / 20.5, 2^24 (14) 25.7 / 25.4, 1.25 x 2^24 (17) 30.7 / 29.2, 2^28 282 / 303;
-// p = 0.1 2^23 16.6 / 13.6, 1.5 x 2^23 19.9 / 17.6, 2^24 21.2 / 21.3, 2^25 (28) 35.1 / 35.5; u64 2^22 (7)
-// p = 0.5 18.8 / 15.1, 2^23 (14) p = 0.1 20.1 / 22.6; u8 2^24 17.3 / 13.5, 2^28 133 / 103; u16 2^24
-// 23.2 / 18.7, 2^26 50.9 / 47.4.
+// from HBM, TMA / slices, us: u32 2^20 8.7 / 5.3, 2^22 13.7 / 9.1; by slices per SM
+//   u32       8            12           13           13.8         15           16           18           24
+//   p = 0.01  16.2 / 10.6  19.4 / 14.2  19.7 / 14.5  20.0 / 15.4  22.3 / 17.0  22.7 / 17.5  24.3 / 20.1  29.2 / 26.3
+//   p = 0.1   16.9 / 14.9  20.4 / 19.3  20.8 / 19.6  21.1 / 21.7  23.5 / 22.6  23.8 / 22.8  25.9 / 26.1  30.8 / 32.9
+//   p = 0.5   18.6 / 17.6  24.4 / 22.5  24.7 / 23.2  24.9 / 25.5  28.2 / 26.7  29.0 / 27.1  32.4 / 30.7  39.2 / 38.1
+//   p = 0.9   21.3 / 20.4  28.0 / 25.8  28.6 / 27.1  29.2 / 29.2  33.5 / 30.6  34.3 / 31.4  38.2 / 35.3  49.3 / 44.5
+//   u64       6            7            8            9            10           12           14
+//   p = 0.1   14.0 / 11.4  16.4 / 15.4  16.0 / 16.8  16.4 / 17.7  16.8 / 18.3  19.4 / 19.7  19.9 / 22.7
+//   p = 0.5   15.3 / 13.3  18.0 / 15.6  17.6 / 16.8  18.6 / 17.6  19.6 / 19.2  23.7 / 21.7  24.6 / 24.8
+// Both kernels step, the slices where an SM's last turn takes a second CTA, the TMA kernel by half units, and where
+// the call's status words fall in memory moves either by several per cent: 13.8 per SM at 0.1 over 24 places TMA
+// 20.7 .. 25.2, mean 21.4, slices 21.2 .. 22.2, mean 21.65; at 0.5 25.4 and 25.5. u8 2^24 16.5 / 11.3, 2^28 135 / 103;
+// u16 2^24 21.6 / 18.3, 2^26 51.6 / 48.
 constexpr uint64_t slices_per_sm(uint32_t elem_bytes)
 {
     return elem_bytes == 4 ? 18 : 8;

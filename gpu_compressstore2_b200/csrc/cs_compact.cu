@@ -1,6 +1,6 @@
 // cs_compact.cu — the TMA-staged, warp-specialised persistent compaction kernel: the 1-pass
-// form, and the 3-pass writeout for chunks longer than 4096 elements (cs_writeout.cu has the
-// others).
+// form of long 4- and 8-byte columns and of a plan's 1-pass columns (cs_slices.cu has the others), the 3-pass
+// writeout for chunks longer than 4096 elements (cs_writeout.cu has the others), and both for skip = 2.
 //
 // Work is split into UNITS of U consecutive tiles; a tile is TILE_BYTES of payload
 // (TILE_BYTES/w elements). One CTA per SM takes units one after another (an atomic ticket

@@ -484,15 +484,6 @@ __device__ __forceinline__ void lookback_kernel_epilogue(ws_header* hdr, uint32_
         epilogue_last(hdr, tile_counter, done_counter, is_scan, keep_begin, keep_end, popc_flags);
 }
 
-// True when pass 1 of this call saw a block sparse enough for the gather kernel (recorded
-// by the scan that followed it, which advanced the epoch).
-__device__ __forceinline__ bool last_popc_saw_sparse(const ws_header* hdr)
-{
-    if (!hdr) return true;
-    const volatile ws_header* vh = hdr;
-    return vh->sparse_epoch == prev_epoch(vh->epoch);
-}
-
 // Header flags a kernel needs, read ONCE per CTA by thread 0 with plain loads (they were
 // written by earlier kernels) and shared through shared memory: thousands of threads
 // re-reading one line with volatile loads serialise in L2. bit 0: the last scan completed
@@ -509,15 +500,6 @@ __device__ __forceinline__ uint32_t cta_header_flags(const ws_header* hdr, uint3
     }
     __syncthreads();
     return *smem_slot;
-}
-
-// True when the look-back scan that ran last on this workspace (stream-ordered before the
-// caller) completed with every tile's prefix valid.
-__device__ __forceinline__ bool last_scan_ok(const ws_header* hdr)
-{
-    if (!hdr) return true;
-    const volatile ws_header* vh = hdr;
-    return vh->scan_ok_epoch == prev_epoch(vh->epoch);
 }
 
 // ---------------------------------------------------------------------------------
@@ -614,8 +596,9 @@ struct BlockScanParams {
     uint64_t keep_end;        // preserved by the epoch-wrap clear
 };
 
-// Predicate compaction and the 1-pass form of the plain call (cs_slices.cu). lo, hi: bit patterns of the element type in their low
-// bytes; whole numbers: the lower bound and the distance to the upper one, modulo the width.
+// Predicate compaction and the 1-pass form of the plain call (cs_slices.cu). lo, hi: bit patterns of the
+// element type in their low bytes; whole numbers: the lower bound and the distance to the upper one, modulo
+// the width.
 struct SliceParams {
     const uint8_t* in;
     uint8_t* out;

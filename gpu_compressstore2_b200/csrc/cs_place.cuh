@@ -1,6 +1,6 @@
 // cs_place.cuh — a warp's item: 4 KB of payload held in registers, its selected elements put in
 // order into a stage of the warp in shared memory, and the stage written out. Used by the 3-pass
-// writeout (cs_writeout.cu) and the pattern compaction (cs_pattern.cu).
+// writeout (cs_writeout.cu), the slices (cs_slices.cu) and the pattern compaction (cs_pattern.cu).
 #pragma once
 #include <cstdint>
 

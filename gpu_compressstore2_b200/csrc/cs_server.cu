@@ -285,9 +285,11 @@ void admit_locked(cs_server* s)
 }
 
 // CTAs per SM of a batch's writeouts, of the three that fit: with all three, the next batch's counting pass
-// found no room beside them and the GPU waited for it between the batches. At 6000 GB/s offered (2000
-// requests, 3 slots), three / two: 5280 .. 5616 / 5601 .. 5627 GB/s, p99 1.5 .. 2.5 / 1.7 ms; at 3000
-// p50 0.10 / 0.083 ms. One per SM: 4900 .. 5060 GB/s.
+// found no room beside them and the GPU waited for it between the batches. GB/s at 6000 offered (2000 requests, 3
+// slots), two / three / the TMA writeout before (one CTA of 200 KB per SM): 5430 .. 5816, mean 5625 / 5321 .. 5722,
+// mean 5490 / 5544 .. 5747, mean 5660, p99 1.4 .. 2.3 / 1.3 .. 2.7 / 1.1 .. 2.0 ms; at 3000 p50 0.075 / 0.083 / 0.107 ms,
+// at 1000 0.043 / 0.044 / 0.055. One per SM: 4900 .. 5060 GB/s. Tried: shorter CTAs (4, 6 and 12 per SM: 5410 .. 5560),
+// the counting pass on a stream of higher priority (5270 .. 5400), the writeouts one after another (2 per SM 4590, 3 5500).
 constexpr uint32_t WRITEOUT_CTAS_PER_SM = 2;
 
 // Enqueue one batch on a slot (no lock held; the requests are RUNNING and stay put).

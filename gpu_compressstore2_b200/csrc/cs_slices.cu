@@ -17,8 +17,8 @@
 // closes as soon as the last CTA has summed up for the last time, so nothing follows the writes (2^20
 // u32: 7.1 -> 5.4 us).
 //
-// What bounds the predicate is instructions: the evaluation and the placing together take about as long as
-// 16 warps' issue of an SM allows while the payload streams at 4 to 5 TB/s. Per call on B200
+// What bounds the predicate is the evaluation and the placing together, with a barrier per slice: half of the
+// issue slots and half of DRAM at 24 warps per SM, the payload streaming at 4 to 5 TB/s. Per call on B200
 // against a mask pass, pass 1 + 2 and the writeout, which read the payload from HBM twice, before ->
 // now: 2^28 f32 x > c with 0.5 selected 459 -> 328 us, 0.01 259 -> 227, 0.1 414 -> 274, 0.9 556 -> 410;
 // 2^27 f64 463 -> 313, 2^28 i16 289 -> 217, 2^28 u8 225 -> 179, 2^24 f32 41 -> 25, 2^20 18 -> 7.
@@ -172,7 +172,6 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS) k_if(const SliceParams p)
             for (uint32_t r = 0; r < ROWS; ++r) load_ragged(e0, r, x[r]);
         }
     };
-    // evaluates it into b; the last warp to do so publishes the slice's total
     // the mask bits of this warp's part of a slice
     auto load_bits = [&](uint32_t slice, uint32_t (&m)[ROWS]) {
         const uint64_t e0 = item_elem(slice);
@@ -189,6 +188,7 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS) k_if(const SliceParams p)
             m[r] = v;
         }
     };
+    // evaluates this warp's part of a slice into b; the last warp to do so publishes the slice's total
     auto evaluate = [&](uint32_t slice, const uint32_t (&m)[ROWS], const uint32_t (&x)[ROWS][8], uint32_t (&b)[PK], uint32_t turn) {
         const uint64_t e0 = item_elem(slice);
         const bool whole = e0 + ITEM <= n;

@@ -29,7 +29,7 @@
 // part skips exactly these units (same count test); it looks at 32 of its items at a time.
 //
 // What bounds the dense part is HBM at half the rows and above for 4 and 8 bytes (2^26 u32
-// p = 0.5: 63.4 us, 410 MB: 6470 GB/s) and, for 1 byte, the integer pipe (packing). Per 3-pass call
+// p = 0.5: 63.4 us, 410 MB: 6470 GB/s) and, for 1 byte, the packing (61 % of the issue slots used). Per 3-pass call
 // on B200 against the TMA-staged writeout it replaces (persistent CTAs, payload tiles and masks
 // through shared-memory rings, 16 compute warps in step): 2^29 u8 p = 0.5 268 -> 195 us, p = 0.9
 // 332 -> 213, 2^28 u16 p = 0.5 179 -> 158, 2^28 f32 p = 0.1 247 -> 212, p = 0.5 304 -> 268, p = 0.9

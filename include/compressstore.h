@@ -65,7 +65,8 @@ typedef enum cs_status {
 /* Algorithm selection. */
 typedef enum cs_algo {
     CS_ALGO_AUTO = 0,   /* autotuner table (size x width bucket) */
-    CS_ALGO_1PASS = 1,  /* single-pass decoupled look-back, TMA-staged persistent kernel */
+    CS_ALGO_1PASS = 1,  /* one kernel, the mask read once: slices that carry a running sum, or
+                           (long 4- and 8-byte columns) TMA-staged units with look-back */
     CS_ALGO_3PASS = 2,  /* chunk popcount -> chunk prefix sum -> writeout */
     CS_ALGO_NAIVE = 3   /* chunk popcount -> prefix sum -> warp-per-word writeout, no
                            alignment requirement beyond elem_bytes */
@@ -79,8 +80,9 @@ typedef struct cs_config {
                                 0 -> 1024 */
     uint32_t grid_dim;       /* CTAs of the writeout/persistent kernel; 0 -> one wave of
                                 resident CTAs (SM count x occupancy) */
-    uint32_t skip;           /* 0 -> default (on), 1 -> skip payload loads of empty
-                                segments, 2 -> always load whole tiles */
+    uint32_t skip;           /* 0 -> default (on), 1 -> payload without a selected element is
+                                not loaded, 2 -> always load whole tiles (1-pass and 3-pass
+                                forms with 16-byte aligned pointers; others skip) */
     uint64_t timeout_ns;     /* bound on every device-side wait; 0 -> 2 s */
     float selectivity;       /* fraction of elements the caller expects selected, in (0, 1]
                                 (a query planner's estimate, say); 0 -> unknown. Under
@@ -101,8 +103,10 @@ typedef struct cs_config {
  * (src/benchmarks.cuh:384-394: cub::DeviceSelect::Flagged) as one entry point.
  * Scratch comes from a per-(device, stream) cache owned by the library, grown with
  * stream-ordered allocations (the role of intermediate_data, src/benchmarks.cuh:53-108).
- * Requires d_in, d_out 16-byte aligned and d_mask 16-byte aligned for the TMA path; other
- * element-aligned pointers are routed to CS_ALGO_NAIVE automatically.
+ * Pointers need element alignment (d_mask: 4 bytes). 16-byte aligned ones are the fast case;
+ * others take the 3-pass form's writeout, which shifts its loads, or, where d_in is 16-byte
+ * aligned and the 1-pass form was chosen, its slices (a caller's chunk length below 128 or
+ * above 4096 leaves CS_ALGO_NAIVE for them).
  * ---------------------------------------------------------------------------------- */
 CS_API int compressstore(const void* d_in, const void* d_mask, void* d_out, uint64_t n,
                   uint32_t elem_bytes, uint64_t* d_count, cs_stream_t stream);
@@ -214,8 +218,8 @@ CS_API int cs_writeout(const void* d_in, const uint32_t* d_mask, void* d_out, ui
  * of a mask in memory. Element i is selected when bit (i % pattern_length) of `pattern` is
  * set (LSB-first, like the mask words; bits >= pattern_length are ignored). No mask is read
  * and no scan runs: the count is (n / L) * popc + popc of the partial period, and every
- * output's source index has a closed form. Pointers need only element alignment (a 16-byte
- * aligned d_out gets 16-byte stores). A zero pattern writes count 0 and nothing else.
+ * output's source index has a closed form. Pointers need only element alignment (long columns of
+ * dense patterns run faster from a 16-byte aligned d_in, full ones between two). A zero pattern writes count 0 and nothing else.
  * Replaces bench9_pattern (src/benchmarks.cuh:397-416) / launch_pattern_proc
  * (src/kernels/kernel_pattern.cuh:83-131), whose pattern starts at the most significant bit
  * (element i <-> bit 31 - i % L): pass the bit-reversed word (__brev / rev32) of such a pattern.
@@ -229,8 +233,8 @@ CS_API int compressstore_pattern(const void* d_in, void* d_out, uint64_t n, uint
  * device, so no mask has to be built on the host and copied in. Element i is selected when
  * pred(d_in[i]) holds, with the elements compared as `type` (which also fixes the width).
  * The mask of the selection (LSB-first words) is written to d_mask_out when it is not NULL
- * (ceil(n/32) words, 16-byte aligned) and to library-owned scratch otherwise; the selected
- * elements are then compacted by the 3-pass writeout. Comparisons follow C++ semantics:
+ * (ceil(n/32) words, 16-byte aligned). One kernel reads the payload from memory once, for the
+ * comparison and the selected elements. Comparisons follow C++ semantics:
  * with floats, every ordered comparison with a NaN is false and NE is true.
  * d_in and d_out must be 16-byte aligned. Errors are reported as for compressstore
  * (compressstore_check on the stream). Reference: the reference evaluates its predicate on
@@ -304,8 +308,8 @@ CS_API int cs_gen_mask_pattern(uint32_t* d_mask, uint64_t n, uint32_t pattern, u
  * Each column takes the 3-pass hybrid or the 1-pass form, and each
  * pass runs ONCE for all the columns that take it: one reduce-then-scan popcount + prefix
  * launch over the 3-pass columns' blocks, one writeout launch per element width over their
- * units and sparse items (a work list spread over every SM), and one 1-pass launch per element width over the 1-pass columns'
- * units (decoupled look-back confined to each column). The plan is built once
+ * units and sparse items (a work list spread over every SM), and one 1-pass launch per element
+ * width over the 1-pass columns' units (decoupled look-back confined to each column). The plan is built once
  * (descriptors, work-to-column maps and scratch live in one device allocation made by
  * cs_batch_create); cs_batch_graph captures the launches in a CUDA graph that later
  * cs_batch_run calls replay. Column pointers are fixed by the plan; their contents may
@@ -314,7 +318,8 @@ CS_API int cs_gen_mask_pattern(uint32_t* d_mask, uint64_t n, uint32_t pattern, u
  * CS_ALGO_AUTO (or cfg NULL) takes the batch table's choice for the column's (width, size,
  * selectivity) bucket (cs_tune_batch_set). When that table holds a 1-pass entry,
  * cs_batch_create measures each column's selectivity with one popcount pass over the masks
- * as they are at that moment (into plan-owned memory); the choice affects speed only.
+ * as they are at that moment (into plan-owned memory), and a plan of few, short or like columns
+ * takes one form throughout; the choice affects speed only.
  * Reference: the reference's only multi-segment form is the 2-stream split with offset
  * stitching of bench3_3pass_streaming (src/benchmarks.cuh:195-293,
  * src/kernels/kernel_streaming_add.cuh:8-16).
@@ -363,8 +368,8 @@ CS_API int cs_batch_destroy(cs_batch* b);
  * order, until the arena can hold them. A scheduler thread forms a batch from every
  * admitted request not yet running (up to max_batch requests and max_batch_elems
  * elements) as soon as one of `slots` batch slots is free, and launches it as one
- * multi-column plan (the batched form's three launches: fused popcount+scan, sparse
- * gather, TMA writeout per width) on that slot's stream. Up to `slots` batches are on the
+ * multi-column plan (the batched form's popcount + prefix launch and one writeout per
+ * width) on that slot's stream. Up to `slots` batches are on the
  * GPU at once, so requests that arrive while others run are launched beside them instead
  * of waiting for them. A request's output is the same whichever batch it lands in.
  * CS_SERVE_PER_CALL runs each admitted request as its own compressstore_ex call (the
@@ -490,7 +495,8 @@ CS_API uint64_t cs_launch_count(void);
 CS_API uint32_t cs_tile_elems(uint32_t elem_bytes);
 
 /* Dynamic shared memory in bytes of one CTA of the TMA-staged persistent kernel for
- * elem_bytes and algo (CS_ALGO_1PASS or CS_ALGO_3PASS); 0 for other arguments. Diagnostic. */
+ * elem_bytes and algo (CS_ALGO_1PASS, or CS_ALGO_3PASS with chunks above 4096 elements or
+ * skip = 2); 0 for other arguments. Diagnostic. */
 CS_API uint32_t cs_compact_smem_bytes(uint32_t elem_bytes, int32_t algo);
 /* Library version as 0xMMmmpp. */
 CS_API uint32_t cs_version(void);
