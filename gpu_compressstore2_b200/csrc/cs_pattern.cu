@@ -22,6 +22,7 @@
 // kernel_pattern_proc (src/kernels/kernel_pattern.cuh:13-131), whose pattern is read from
 // the most significant bit (element i <-> bit 31 - i % L); pass __brev of such a pattern.
 #include <cstdint>
+#include <type_traits>
 
 #include <cuda_runtime.h>
 
@@ -34,7 +35,10 @@ namespace cs {
 namespace {
 
 constexpr uint32_t PATTERN_RUNS = 8;
-constexpr uint32_t PATTERN_CTAS = 8; // per SM
+// CTAs per SM. 5 or 6 are resident; 4- and 8-byte elements keep the memory busier with a second set of blocks
+// that start as the first end (8 / 16, us, output not 16-byte aligned: 2^28 u32 1 of 2 278 / 250, 2 of 3 342 / 288, 2^26
+// u64 6 of 7 172 / 161), where 2-byte ones lose (2^28 1 of 2 179 / 194) and bytes do not care (8 of 8 269 / 262, 2 of 3 6.2 / 6.2).
+template <typename T> constexpr uint32_t PATTERN_CTAS = sizeof(T) >= 4 ? 16u : 8u;
 
 // VEC_OUT: the output is aligned to a lane's bytes. APART: the selected elements lie 64 bytes and
 // more apart on average, so a load fetches 64 bytes rather than a line.
@@ -68,14 +72,18 @@ __global__ void __launch_bounds__(256) k_pattern(const T* __restrict__ in, T* __
     }
     __syncthreads();
     const uint32_t lane = threadIdx.x & 31u;
-    // (numbers of warps of a resident grid: divided in 32 bits)
-    const uint32_t s_first = ((blockIdx.x * 256u + threadIdx.x) >> 5) * U;
-    const uint32_t step = gridDim.x * 8u * U; // runs between a warp's groups
+    // Numbers of warps of a bounded grid: divided in 32 bits, which a short column notices (2^20 u64, 6 of 7, 6.1 -> 4.7 us).
+    // The loop of 2-byte elements that are stored one by one comes out better from 64 (2^28, us, 32 / 64: 1 of 2 196 /
+    // 179, 2 of 3 256 / 230, 8 of 8 372 / 328).
+    using Index = std::conditional_t<sizeof(T) == 2 && !VEC_OUT, uint64_t, uint32_t>;
+    const Index s_first = ((static_cast<Index>(blockIdx.x) * 256u + threadIdx.x) >> 5) * U;
+    const Index step = static_cast<Index>(gridDim.x) * 8u * U; // runs between a warp's groups
     const uint64_t runs = (count + RUN - 1) / RUN;
-    const uint32_t dq = step / P, dr = step % P;
+    const Index dq = step / P;
+    const uint32_t dr = static_cast<uint32_t>(step % P);
     const uint32_t period = RUN * L; // inputs of P runs
     uint64_t q = s_first / P;
-    uint32_t r = s_first % P;
+    uint32_t r = static_cast<uint32_t>(s_first % P);
     for (uint64_t s0 = s_first; s0 < runs; s0 += step) {
         T x[U][G];
         const T* src = in + q * period;
@@ -284,7 +292,7 @@ cudaError_t launch_t(const void* in, void* out, uint64_t n, uint32_t pattern, ui
 {
     constexpr uint64_t GROUP = 8 * PATTERN_RUNS * 32 * (sizeof(T) < 4 ? 4 / sizeof(T) : 1); // outputs per CTA and iteration
     uint64_t blocks = (count + GROUP - 1) / GROUP;
-    const uint64_t cap = static_cast<uint64_t>(sms) * PATTERN_CTAS;
+    const uint64_t cap = static_cast<uint64_t>(sms) * PATTERN_CTAS<T>;
     if (blocks > cap) blocks = cap;
     if (blocks == 0) blocks = 1;
     const bool vec = (reinterpret_cast<uintptr_t>(out) & 3u) == 0;

@@ -46,3 +46,13 @@ def test_everything(cuda, oracle, w):
             _check(oracle, w, n, pattern, length, 16 // w, 0)
             _check(oracle, w, n, pattern, length, 1, 0)  # inside a 16-byte group: gathered
             _check(oracle, w, n, pattern, length, 0, 1)
+
+
+@pytest.mark.parametrize("w", [1, 2, 4, 8])
+def test_gathers_of_several_rounds(cuda, oracle, w):
+    # unaligned, so gathered: a resident grid of 16 blocks per SM with 8 warps of 8 runs, once and once more
+    outputs = 148 * 16 * 8 * 8 * max(128 // w, 32)
+    for pattern, length in ((0b101, 3), (0b1110111, 7)):
+        n = outputs // bin(pattern).count("1") * length
+        for extra in (0, 1, n // 2 + 13):
+            _check(oracle, w, n + extra, pattern, length, 1, 1)
