@@ -34,7 +34,7 @@ struct cs_batch {
     PlanDevice dev;
     PlanCounts counts;
     uint32_t grid1[4] = {0, 0, 0, 0};
-    uint32_t idle[4] = {0, 0, 0, 0}; // warps per CTA of each width's writeout
+    uint32_t idle8 = 0; // idle warps per CTA of the 8-byte columns' writeout
     uint32_t one_pass_cols = 0;
     std::vector<cs_column> cols; // for the per-call loop
     uint64_t timeout_ns = 2000000000ull;
@@ -66,20 +66,22 @@ bool plan_one_launch(uint32_t widths, uint32_t columns, uint64_t longest, uint64
     return bytes >= (widths == 8 ? 16u << 20 : 28u << 20) && bytes <= 80u << 20 && selected >= (widths == 4 ? 0.05 : 0.3);
 }
 
-// Idle warps of a writeout (idle_warps in cs_writeout.cu) for the plan's 3-pass columns of a width, by what is
-// selected of them when the plan is made.
-uint32_t idle_warps_of(const cs_column* cols, uint32_t ncols, const std::vector<uint8_t>& one_pass,
-                       const std::vector<double>& sel, uint32_t width)
+// Idle warps of the writeout (idle_warps in cs_writeout.cu) for the plan's 3-pass columns of 8 bytes, by what is
+// selected of them when the plan is made: for 512 MB and more of them in columns of 11 MB and more on average. us with
+// all warps / with idle ones, 0.85 to 0.95 selected: 16 columns 250 MB 87.5 / 89.9, 400 MB 139.7 / 134.1, 1.5 GB 502 / 457;
+// 64 columns 550 MB 178.9 / 182.3, 750 MB 246.9 / 241.1, 1.5 GB 504 / 462; 128 columns 750 MB 239.8 / 244.8, 1.5 GB 496 /
+// 467; 256 columns 400 MB 137 / 144, 1 GB 313 / 328. Plans of 4-byte columns lose (64 columns, 750 MB 252 / 259).
+uint32_t idle_warps_of(const cs_column* cols, uint32_t ncols, const std::vector<uint8_t>& one_pass, const std::vector<double>& sel)
 {
-    double elems = 0.0, selected = 0.0;
+    double elems = 0.0, selected = 0.0, columns = 0.0;
     for (uint32_t i = 0; i < ncols; ++i) {
-        if (one_pass[i] || cols[i].elem_bytes != width) continue;
+        if (one_pass[i] || cols[i].elem_bytes != 8 || !cols[i].n) continue;
+        columns += 1.0;
         elems += static_cast<double>(cols[i].n);
         selected += sel[i] * static_cast<double>(cols[i].n);
     }
-    const double share = elems > 0.0 ? selected / elems : 0.0;
-    if (width == 8) return share >= 0.75 ? 2u : 0u;
-    return share >= 0.85 && share < 0.97 ? 1u : 0u;
+    const double bytes = elems * 8;
+    return bytes >= 512.0 * (1 << 20) && bytes >= columns * 11.0 * (1 << 20) && selected >= 0.75 * elems ? 2u : 0u;
 }
 
 inline int to_status(cudaError_t e)
@@ -95,7 +97,7 @@ int run_direct(cs_batch* b, cudaStream_t s)
         cudaError_t e = cudaMemsetAsync(c, 0, sizeof(uint64_t), s);
         if (e != cudaSuccess) return to_status(e);
     }
-    return plan_launch(b->dev, b->counts, b->sms, b->timeout_ns, s, b->grid1, 0, b->idle);
+    return plan_launch(b->dev, b->counts, b->sms, b->timeout_ns, s, b->grid1, 0, b->idle8);
 }
 
 // Selected fraction of every column, from one reduce-then-scan popcount pass over the masks
@@ -222,7 +224,7 @@ int cs_batch_create(cs_batch** out, const cs_column* cols, uint32_t ncols, const
         }
         if (!bytes1 && plan_one_launch(widths, filled, longest, bytes3, bytes3 ? selected / static_cast<double>(bytes3) : 0.0))
             for (uint32_t i = 0; i < ncols; ++i) one_pass[i] = cols[i].n ? 1 : 0;
-        for (int wi = 2; wi < 4; ++wi) b->idle[wi] = idle_warps_of(cols, ncols, one_pass, sel, 1u << wi);
+        b->idle8 = idle_warps_of(cols, ncols, one_pass, sel);
     }
     for (uint32_t i = 0; i < ncols; ++i) b->one_pass_cols += one_pass[i] && cols[i].n ? 1u : 0u;
 

@@ -249,7 +249,7 @@ uint32_t plan_kernels(const PlanCounts& c)
 }
 
 int plan_launch(const PlanDevice& d, const PlanCounts& c, int sms, uint64_t timeout_ns, cudaStream_t s,
-                const uint32_t* grid1, uint32_t writeout_ctas, const uint32_t* idle)
+                const uint32_t* grid1, uint32_t writeout_ctas, uint32_t idle8)
 {
     if (c.tiles) {
         BlockScanParams bp{};
@@ -282,7 +282,7 @@ int plan_launch(const PlanDevice& d, const PlanCounts& c, int sms, uint64_t time
         first_item += c.width_items[wi];
         p.hdr = d.hdr;
         p.chunk_log2 = PLAN_CHUNK_LOG2;
-        p.throttle = idle ? idle[wi] : 0u;
+        p.throttle = w == 8 ? idle8 : 0u;
         cudaError_t e = launch_writeout_warp(p, w, writeout_ctas, sms, s);
         if (e != cudaSuccess) return to_status(e);
     }

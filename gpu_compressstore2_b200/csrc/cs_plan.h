@@ -117,9 +117,9 @@ uint32_t plan_kernels(const PlanCounts& c);
 // sparse units); then one
 // 1-pass TMA kernel per width with 1-pass columns (grid1, may be null when there are none).
 // The 1-pass kernels come last: each advances the workspace epoch, which the 3-pass writeouts
-// read to validate the pass-2 results. writeout_ctas: CTAs of a writeout (0: one resident wave); idle: of
-// each width, warps per CTA that a long writeout leaves idle (null: none). Returns a cs_status.
+// read to validate the pass-2 results. writeout_ctas: CTAs of a writeout (0: one resident wave); idle8: warps
+// per CTA that the writeout of 8-byte columns leaves idle where it is long. Returns a cs_status.
 int plan_launch(const PlanDevice& d, const PlanCounts& c, int sms, uint64_t timeout_ns, cudaStream_t s,
-                const uint32_t* grid1 = nullptr, uint32_t writeout_ctas = 0, const uint32_t* idle = nullptr);
+                const uint32_t* grid1 = nullptr, uint32_t writeout_ctas = 0, uint32_t idle8 = 0);
 
 } // namespace cs

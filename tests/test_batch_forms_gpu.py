@@ -81,3 +81,10 @@ def test_long_plans_mostly_selected(cuda, w, share):
     """More than 8 items of 4 KB for every warp, in columns of odd lengths."""
     n = 148 * 3 * 8 * 8 * 4096 // w // 3 + 1001
     _check([(n + i, w, share) for i in range(4)] + [(5000, w, 0.01)], 2)
+
+
+@pytest.mark.parametrize("share", [0.74, 0.76, 1])
+def test_idle_warps_of_plans(cuda, share):
+    """512 MB and more of 8-byte columns, and a narrower and a short one beside them."""
+    _check([((64 << 20) // 3 + 1001 + i, 8, share) for i in range(3)] + [(5000, 8, 0.01)], 2)
+    _check([((64 << 20) // 3 + 1001 + i, 8, share) for i in range(3)] + [(70001, 4, 0.9)], 3)
